@@ -28,6 +28,7 @@
 #include "cvl_internal.h"
 #include "cvl_pinned.h"
 #include "cvl_contours.cuh"
+#include "cvl_curvelets.cuh"
 #include "cvl_path.cuh"
 #include "cvl_polyarcs.cuh"
 #include "cvl_scan.cuh"
@@ -172,6 +173,8 @@ struct cvl_engine {
     bool persist_on = std::getenv("CVL_NO_PERSIST") == nullptr;
     // the transport's k_dx quotient pairs on one reciprocal (CVL_NO_SHARED_QUOTIENTS: divisions)
     bool shared_quot_on = std::getenv("CVL_NO_SHARED_QUOTIENTS") == nullptr;
+    // decisions on single-precision enclosures (CVL_NO_ENCLOSURES: every bundle in FP64)
+    bool enclosures_on = std::getenv("CVL_NO_ENCLOSURES") == nullptr;
     uint64_t ws_epoch = 0;                         // workspace (re)allocations so far
     uint64_t graph_replays = 0, graph_fallbacks = 0, graph_captures = 0, graph_clock = 0;
     DBuf gdims, gchunks, gread;
@@ -640,6 +643,168 @@ inline bool persistent_chunks(const cvl_engine *e, long long n) {
 // the record arena's chunk tails in the workspace formula
 constexpr unsigned long long PERSIST_GROWTH_WARPS_MAX = 160ull * 4 * 8;
 
+// ---- the fused path (cvl_curvelets.cuh) -------------------------------------------
+// The edges as k_curvelets gathers them live in the anchor trig rows' buffer, which the
+// path does not use otherwise: 48 bytes per edge of its 16 (Q + 1), Q >= 3.
+inline FastBinned fast_binned(const cvl_engine *e, size_t n) {
+    return FastBinned{(FastEdge *)e->atrig.p, (double2 *)((FastEdge *)e->atrig.p + n)};
+}
+
+// k_curvelets over the anchors, then k_curvelets_exact over those it left.
+int launch_curvelets(cvl_engine *e, const FastArgs &a, int blocks, int exact_blocks) {
+    cudaStream_t s = e->stream;
+    constexpr size_t smem = fast_smem_bytes<FastSmem<FAST_CAP, FAST_SLOTS>>(), wide = fast_smem_bytes<FastWideSmem>();
+    if (a.queue) {
+        CVL_CUDA(cudaFuncSetAttribute(k_curvelets<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_curvelets<true><<<blocks, FAST_WARPS * 32, smem, s>>>(a);
+    } else {
+        CVL_CUDA(cudaFuncSetAttribute(k_curvelets<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_curvelets<false><<<blocks, FAST_WARPS * 32, smem, s>>>(a);
+    }
+    CVL_TRY(check_launch("k_curvelets"));
+    CVL_CUDA(cudaFuncSetAttribute(k_curvelets_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide));
+    k_curvelets_exact<<<exact_blocks, FAST_WARPS * 32, wide, s>>>(a);
+    return check_launch("k_curvelets_exact");
+}
+
+FinalArgs final_args(const cvl_engine *e, const Model &md, const BinnedT<double> &B, const FastBinned &F, int n, int M,
+                     const int *d_map_off, unsigned long long out_cap) {
+    FinalArgs f{};
+    f.md = md;
+    f.B = B;
+    f.cs2 = F.cs2;
+    f.pos_of = (const int *)e->pos_of.p;
+    f.N = n;
+    f.M = M;
+    f.map_off = d_map_off;
+    f.rec_ids = (const unsigned *)e->rec_ids.p;
+    f.rec_meta = (const unsigned *)e->rec_meta.p;
+    f.rec_base = (const unsigned *)e->rec_base.p;
+    f.run_cnt = (const unsigned *)e->run_cnt.p;
+    f.out_off = (const unsigned long long *)e->out_off.p;
+    f.out_cap = out_cap;
+    f.cell_rank = (const unsigned short *)e->crank.p;
+    f.chains = (unsigned *)e->chains.p;
+    f.info = (double *)e->info.p;
+    return f;
+}
+
+// (c) + (d) + (e) of a direct run by k_curvelets and k_finalize_exact; a run with a yield
+// hook goes chunk by chunk (anchors [cstart[c], cstart[c + 1])), on short blocks.
+int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, const BinnedT<double> &B, const Model &md,
+                    int n, int M, const int *d_map_off, const std::vector<int32_t> &map_off_host, int mode,
+                    const cvl_tuning &tn, const std::vector<int> &cstart, int nchunks, RunOut &ro) {
+    cudaStream_t s = e->stream;
+    const int sms = e->prop.multiProcessorCount;
+    const bool persist = persistent_chunks(e, n);
+    const int blocks = sms * FAST_BLOCKS;
+    unsigned long long *work = (unsigned long long *)e->work.p;
+    unsigned *queues = (unsigned *)(work + 3);  // anchors taken, anchors pushed to the wide variant
+    unsigned *err = (unsigned *)e->err.p;
+    MapStats *stats = (MapStats *)e->stats.p;
+    const int launches = e->yield_fn ? nchunks : 1;
+    CVL_TRY(e->alloc(e->crank, sizeof(unsigned short) * CELLS_MAX));
+    k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
+    CVL_TRY(check_launch("k_cell_ranks"));
+    for (int attempt = 0;; ++attempt) {
+        // the chunk tails the warps leave unused: one record per anchor, or a chunk per
+        // persistent warp and launch
+        unsigned long long cap = std::max<unsigned long long>(e->arena_hint, 4ull * (unsigned long long)n + 4096ull) +
+                                 (unsigned long long)n + (unsigned long long)GROWTH_ARENA_CHUNK * (nchunks + 1) +
+                                 (persist ? (unsigned long long)GROWTH_ARENA_CHUNK * blocks * FAST_WARPS : 0ull);
+        if (mode == 0) {
+            CVL_TRY(e->alloc(e->rec_ids, sizeof(unsigned) * cap * md.gms));
+            CVL_TRY(e->alloc(e->rec_meta, sizeof(unsigned) * cap));
+        } else {
+            cap = 0;
+        }
+        cap = std::min<unsigned long long>(cap, 0xffffffffull);  // record indices are 32-bit
+        for (int c = 0; c < launches; ++c) {
+            const int a0 = launches == 1 ? 0 : cstart[c], a1 = launches == 1 ? n : cstart[c + 1];
+            if (a1 <= a0) continue;
+            if (e->yield_fn && c > 0) {
+                // let the previous chunk finish, then give the hook the chance to hold
+                // this stream back while others' work goes first
+                if (!e->chunk_done) CVL_CUDA(cudaEventCreateWithFlags(&e->chunk_done, cudaEventDisableTiming));
+                CVL_CUDA(cudaEventRecord(e->chunk_done, s));
+                CVL_CUDA(cudaEventSynchronize(e->chunk_done));
+                e->yield_fn(e->yield_ctx);
+            }
+            CVL_CUDA(cudaMemsetAsync(queues, 0, 2 * sizeof(unsigned), s));
+            FastArgs fa{};
+            fa.md = md;
+            fa.fm = fm;
+            fa.B = B;
+            fa.F = F;
+            fa.a_begin = a0;
+            fa.a_end = a1;
+            fa.pair_off = (const unsigned long long *)e->pair_off.p;
+            fa.csr_ids = (const int *)e->csr_ids.p;
+            fa.pcls = (const unsigned char *)e->pcls.p;
+            fa.rec_ids = (unsigned *)e->rec_ids.p;
+            fa.rec_meta = (unsigned *)e->rec_meta.p;
+            fa.arena_cap = cap;
+            fa.arena_ctr = work;
+            fa.rec_base = (unsigned *)e->rec_base.p;
+            fa.run_cnt = (unsigned *)e->run_cnt.p;
+            fa.count = (unsigned *)e->count.p;
+            fa.stats = stats;
+            fa.count_only = (mode == 1) ? 1 : 0;
+            fa.err = err;
+            fa.cell_rank = (const unsigned short *)e->crank.p;
+            fa.arena_chunk = persist ? GROWTH_ARENA_CHUNK : 1;
+            fa.tile = persist ? FAST_TILE : 1;
+            fa.queue = persist ? queues : nullptr;
+            fa.over_cnt = queues + 1;
+            fa.over_list = (int *)e->deg.p;  // (its scan is done)
+            const int grid = persist ? blocks : short_grid(a1 - a0, (long long)FAST_WARPS * tn.anchors_per_warp);
+            CVL_TRY(launch_curvelets(e, fa, grid, sms * FAST_EXACT_BLOCKS));
+            e->mark("curvelets");
+        }
+        if (mode == 1) {
+            unsigned h_err = 0;
+            CVL_CUDA(cudaMemcpyAsync(ro.stats.data(), stats, sizeof(MapStats) * M, cudaMemcpyDeviceToHost, s));
+            CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+            e->mark("end");
+            CVL_CUDA(cudaStreamSynchronize(s));
+            if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
+            return CVL_OK;
+        }
+        // ---- output positions (anchor-major, compact_curvelet_output)
+        CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->count.p, n,
+                                                    (unsigned long long *)e->out_off.p)));
+        ro.cv_off.assign(M + 1, 0);
+        for (int m = 0; m <= M; ++m)
+            CVL_CUDA(cudaMemcpyAsync(&ro.cv_off[m], (unsigned long long *)e->out_off.p + map_off_host[m],
+                                     sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        unsigned long long used = 0;
+        unsigned h_err = 0;
+        CVL_CUDA(cudaMemcpyAsync(ro.stats.data(), stats, sizeof(MapStats) * M, cudaMemcpyDeviceToHost, s));
+        CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+        CVL_CUDA(cudaMemcpyAsync(&used, work, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        CVL_CUDA(cudaStreamSynchronize(s));
+        if ((h_err & ERR_ARENA) && attempt == 0) {
+            // the record arena was too small: size it to what this input needs and grow the
+            // chains again (valid and close pairs are recounted from zero)
+            e->arena_hint = used + used / 8 + 4096;
+            for (MapStats &st : ro.stats) st.valid_pairs = st.close_pairs = 0;
+            CVL_CUDA(cudaMemcpyAsync(stats, ro.stats.data(), sizeof(MapStats) * M, cudaMemcpyHostToDevice, s));
+            CVL_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(unsigned) * 4, s));
+            CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 2, s));
+            continue;
+        }
+        if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
+        const unsigned long long C = ro.cv_off[M];
+        ro.total_curvelets = C;
+        CVL_TRY(e->alloc(e->chains, sizeof(unsigned) * C * (md.gms + 1)));
+        CVL_TRY(e->alloc(e->info, sizeof(double) * C * 10));
+        k_finalize_exact<<<short_grid(n, 256), 256, 0, s>>>(final_args(e, md, B, F, n, M, d_map_off, C));
+        CVL_TRY(check_launch("k_finalize_exact"));
+        e->mark("finalize");
+        return CVL_OK;
+    }
+}
+
 // mode: 0 = full run, 1 = count valid pairs only, 2 = neighbour graph only
 template <typename R>
 int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const int *d_map_off,
@@ -704,6 +869,17 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     MapStats *stats = (MapStats *)e->stats.p;
     unsigned long long *arena_ctr = (unsigned long long *)e->work.p;
 
+    const bool path = (mode != 2);
+    FastModel fm{};
+    FastBinned F{};
+    if constexpr (std::is_same<R, double>::value) {
+        if (path && e->enclosures_on) fm = make_fast(md);
+        if (fm.ok) {
+            CVL_TRY(e->alloc(e->atrig, sizeof(R) * (size_t)n * (2 * md.Q + 2)));
+            F = fast_binned(e, (size_t)n);
+        }
+    }
+
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->bfill.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * M, s));
@@ -719,7 +895,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B, (int *)e->pos_of.p,
-                                     nullptr);
+                                     F.e, F.cs2, nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
 
@@ -763,6 +939,8 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
                              cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(ro.stats.data(), stats, sizeof(MapStats) * M, cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    unsigned h_uncertified = 0;
+    CVL_CUDA(cudaMemcpyAsync(&h_uncertified, uncertified, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(cstart.data(), e->chunk_start.p, sizeof(int) * (max_chunks + 1), cudaMemcpyDeviceToHost,
                              s));
     CVL_CUDA(cudaStreamSynchronize(s));
@@ -779,9 +957,9 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     // ---- (b) neighbour fill: CSR, pair classes, pair -> anchor, anchor trig
     CVL_TRY(e->alloc(e->csr_ids, sizeof(int) * P));
     if (want_d2) CVL_TRY(e->alloc(e->csr_d2, sizeof(R) * P));
-    const bool path = (mode != 2);
-    if (path) {
-        CVL_TRY(e->alloc(e->pcls, P));
+    const bool fast = fm.ok && !(h_uncertified & UNCERT_ANGLE);
+    if (path) CVL_TRY(e->alloc(e->pcls, P));
+    if (path && !fast) {
         CVL_TRY(e->alloc(e->pflag, P));
         CVL_TRY(e->alloc(e->pair_anchor, sizeof(int) * P));
         CVL_TRY(e->alloc(e->atrig, sizeof(R) * (size_t)n * (2 * md.Q + 2)));
@@ -789,8 +967,9 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     na.csr_ids = (int *)e->csr_ids.p;
     na.csr_d2 = want_d2 ? (R *)e->csr_d2.p : nullptr;
     na.pcls = path ? (unsigned char *)e->pcls.p : nullptr;
-    na.pair_anchor = path ? (int *)e->pair_anchor.p : nullptr;
-    na.atrig = path ? (R *)e->atrig.p : nullptr;
+    na.pair_anchor = path && !fast ? (int *)e->pair_anchor.p : nullptr;
+    na.atrig = path && !fast ? (R *)e->atrig.p : nullptr;
+    na.cs2 = fast ? F.cs2 : nullptr;
     na.uncertified = uncertified;
     k_nb<R, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
     CVL_TRY(check_launch("k_nb<FILL>"));
@@ -798,6 +977,11 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     if (mode == 2) {
         e->mark("end");
         return CVL_OK;
+    }
+
+    if constexpr (std::is_same<R, double>::value) {
+        if (fast)
+            return run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, cstart, nchunks, ro);
     }
 
     // ---- (c) + (d) per chunk
@@ -845,7 +1029,6 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         for (int c = 0; c <= nchunks; ++c)
             CVL_CUDA(cudaMemcpyAsync(&h_poff[c], (unsigned long long *)e->pair_off.p + cstart[c],
                                      sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-        unsigned h_uncertified = 0;
         CVL_CUDA(cudaMemcpyAsync(&h_uncertified, uncertified, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaStreamSynchronize(s));
         const int shared_quot = (md.shared_quot && !h_uncertified) ? 1 : 0;
@@ -1086,8 +1269,13 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     sh.edge_data_sz = sz;
     // (the input rows and map offsets are the caller's, already in place: they are
     // not reallocated here)
+    const FastModel fm = e->enclosures_on ? make_fast(md) : FastModel{};
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
         if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off) continue;
+        // k_curvelets keeps no bundles, pair flags or numbers in memory
+        if (fm.ok && (w.buf == &cvl_engine::bund || w.buf == &cvl_engine::pflag || w.buf == &cvl_engine::pair_anchor ||
+                      w.buf == &cvl_engine::rec_k))
+            continue;
         CVL_TRY(e->alloc(e->*(w.buf), w.bytes));
     }
     CVL_TRY(e->alloc(e->gdims, sizeof(RunDims)));
@@ -1116,7 +1304,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     const void *ptrs[] = {d_edges, d_map_off, e->chains.p, e->info.p};
     key.append((const char *)ptrs, sizeof(ptrs));
     const unsigned long long nums[] = {(unsigned long long)b, (unsigned long long)sz, (unsigned long long)cpl,
-                                       e->ws_epoch, arena_cap, per_chunk};
+                                       e->ws_epoch, arena_cap, per_chunk, (unsigned long long)fm.ok};
     key.append((const char *)nums, sizeof(nums));
     key.append((const char *)&tn, sizeof(tn));
     cvl_engine::GraphSlot *slot = nullptr;
@@ -1153,6 +1341,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
         ChunkDims *cdp = (ChunkDims *)e->gchunks.p;
         const int sms = e->prop.multiProcessorCount;
         const int N = cap.N;
+        const FastBinned F = fm.ok ? fast_binned(e, (size_t)N) : FastBinned{};
         CVL_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         auto enqueue = [&]() -> int {
             CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
@@ -1170,7 +1359,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B,
-                                             (int *)e->pos_of.p, dd);
+                                             (int *)e->pos_of.p, F.e, F.cs2, dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;
@@ -1191,17 +1380,20 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY(check_launch("k_deg_from_ncand"));
             CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->deg.p, N,
                                                         (unsigned long long *)e->pair_off.p)));
-            k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
-                                             (int *)e->chunk_start.p, dd);
-            CVL_TRY(check_launch("k_chunk_starts"));
-            k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p, (const int *)e->chunk_start.p,
-                                          per_chunk, cap.K, cdp, err);
-            CVL_TRY(check_launch("k_chunk_dims"));
+            if (!fm.ok) {
+                k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
+                                                 (int *)e->chunk_start.p, dd);
+                CVL_TRY(check_launch("k_chunk_starts"));
+                k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
+                                              (const int *)e->chunk_start.p, per_chunk, cap.K, cdp, err);
+                CVL_TRY(check_launch("k_chunk_dims"));
+            }
             na.csr_ids = (int *)e->csr_ids.p;
             na.csr_d2 = nullptr;
             na.pcls = (unsigned char *)e->pcls.p;
-            na.pair_anchor = (int *)e->pair_anchor.p;
-            na.atrig = (double *)e->atrig.p;
+            na.pair_anchor = fm.ok ? nullptr : (int *)e->pair_anchor.p;
+            na.atrig = fm.ok ? nullptr : (double *)e->atrig.p;
+            na.cs2 = F.cs2;
             na.uncertified = uncertified;
             k_nb<double, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
             CVL_TRY(check_launch("k_nb<FILL>"));
@@ -1213,7 +1405,38 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             rec.meta = (unsigned *)e->rec_meta.p;
             // the chunks' work queues (bundle pair tiles, growth anchors)
             unsigned *queues = (unsigned *)((unsigned long long *)e->work.p + 3);
-            for (int c = 0; c < cap.K; ++c) {
+            if (fm.ok) {
+                FastArgs fa{};
+                fa.md = md;
+                fa.fm = fm;
+                fa.B = B;
+                fa.F = F;
+                fa.pair_off = (const unsigned long long *)e->pair_off.p;
+                fa.csr_ids = (const int *)e->csr_ids.p;
+                fa.pcls = (const unsigned char *)e->pcls.p;
+                fa.rec_ids = rec.ids;
+                fa.rec_meta = rec.meta;
+                fa.arena_cap = arena_cap;
+                fa.arena_ctr = arena_ctr;
+                fa.rec_base = (unsigned *)e->rec_base.p;
+                fa.run_cnt = (unsigned *)e->run_cnt.p;
+                fa.count = (unsigned *)e->count.p;
+                fa.stats = stats;
+                fa.err = err;
+                fa.cell_rank = (const unsigned short *)e->crank.p;
+                fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
+                fa.dims = dd;
+                fa.tile = b == 1 ? FAST_TILE : 1;
+                fa.pair_cap = (unsigned long long)sh.num_pairs;
+                // bucket 1 pulls anchors from the queue; bucket 0's runs are too small for
+                // the atomics to pay
+                fa.queue = b == 1 ? queues : nullptr;
+                fa.over_cnt = queues + 1;
+                fa.over_list = (int *)e->deg.p;
+                fa.uncertified = uncertified;  // a run outside the certified angles goes kernel by kernel
+                CVL_TRY(launch_curvelets(e, fa, sms * FAST_BLOCKS, sms * FAST_EXACT_BLOCKS));
+            }
+            for (int c = 0; c < (fm.ok ? 0 : cap.K); ++c) {
                 CVL_CUDA(cudaMemsetAsync(queues, 0, 2 * sizeof(unsigned), s));
                 BundleArgsT<double> ba{};
                 ba.md = md;
@@ -1265,11 +1488,18 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             }
             CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->count.p, N,
                                                         (unsigned long long *)e->out_off.p)));
-            k_finalize<double><<<gb, 256, 0, s>>>(md, d_edges, sz, N, d_map_off, cap.M, rec,
-                                                  (const unsigned *)e->rec_base.p, (const unsigned *)e->run_cnt.p,
-                                                  (const unsigned long long *)e->out_off.p, C_cap,
-                                                  (unsigned *)e->chains.p, (double *)e->info.p, dd);
-            CVL_TRY(check_launch("k_finalize"));
+            if (fm.ok) {
+                FinalArgs f = final_args(e, md, B, F, N, cap.M, d_map_off, C_cap);
+                f.dims = dd;
+                k_finalize_exact<<<gb, 256, 0, s>>>(f);
+                CVL_TRY(check_launch("k_finalize_exact"));
+            } else {
+                k_finalize<double><<<gb, 256, 0, s>>>(md, d_edges, sz, N, d_map_off, cap.M, rec,
+                                                      (const unsigned *)e->rec_base.p, (const unsigned *)e->run_cnt.p,
+                                                      (const unsigned long long *)e->out_off.p, C_cap,
+                                                      (unsigned *)e->chains.p, (double *)e->info.p, dd);
+                CVL_TRY(check_launch("k_finalize"));
+            }
             k_graph_readback<<<(cap.M + 1 + 255) / 256, 256, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
                                                                      (const unsigned long long *)e->out_off.p,
                                                                      d_map_off, (unsigned long long *)e->gread.p);

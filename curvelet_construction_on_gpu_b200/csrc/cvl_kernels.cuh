@@ -34,6 +34,9 @@ constexpr int MAPS_SMEM = 256;  // per-block map statistics kept in shared memor
 constexpr double CVL_PI = 3.14159265358979323846;  // curvelet_utils.hpp:10
 
 // Error bits raised by kernels (checked by the host after a run).
+// a run's certification flag: bit 0, an operand outside certify_*'s ranges; bit 1, an
+// orientation beyond +-1024 rad, where the enclosures of cvl_curvelets.cuh do not hold
+constexpr unsigned UNCERT_ANGLE = 2u;
 constexpr unsigned ERR_NONFINITE = 1u;   // non-finite or out-of-range coordinate
 constexpr unsigned ERR_CAPACITY = 2u;    // a device capacity was exceeded
 constexpr unsigned ERR_INTERNAL = 4u;    // an internal invariant failed (bounds check)
@@ -92,6 +95,13 @@ struct BinnedT {
     int2 *cell;                 // pixel cell (lrint(x), lrint(y))
     int *orig;                  // global input index
     int *map;                   // map of the edge
+};
+
+// One edge as k_curvelets gathers it (cvl_curvelets.cuh): FP64 position, sin/cos(T0 -+ dt)
+// in single precision. One 32-byte sector per neighbour.
+struct __align__(16) FastEdge {
+    double x, y;
+    float cm, sm, cp, sp;
 };
 
 // The sizes of a run that a captured graph replays (one graph per size bucket
@@ -266,7 +276,10 @@ __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int
             atomicAdd(&bcount[0], 1u);
             continue;
         }
-        if (uncertified && !(certify_coord(x) && certify_coord(y))) atomicOr(uncertified, 1u);
+        if (uncertified) {
+            const unsigned un = (certify_coord(x) && certify_coord(y) ? 0u : 1u) | (fabs(th) <= T(1024) ? 0u : UNCERT_ANGLE);
+            if (un) atomicOr(uncertified, un);
+        }
         const int m = map_of(map_off, M, e);
         const int cx = lrint_dev(x);  // lrint, round half to even (preprocess.hpp:85-86)
         const int cy = lrint_dev(y);
@@ -280,7 +293,8 @@ template <typename T>
 __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const int *__restrict__ map_off,
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bfill, BinnedT<T> B,
-                              int *__restrict__ pos_of, const RunDims *__restrict__ dims) {
+                              int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
+                              const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
         M = dims->M;
@@ -297,10 +311,20 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
         // T0 +- dt and their sin/cos (cpu_curvelet.hpp:655-656, 730-733), once per edge
         const T t_p = th + md.dt;
         const T t_m = th - md.dt;
-        B.sp[pos] = sin(t_p);
-        B.cp[pos] = cos(t_p);
-        B.sm[pos] = sin(t_m);
-        B.cm[pos] = cos(t_m);
+        // (sincos gives the values of sin and cos: tests/probes/sincos_identity.cu)
+        T sp, cp, sm, cm;
+        sincos(t_p, &sp, &cp);
+        sincos(t_m, &sm, &cm);
+        B.sp[pos] = sp;
+        B.cp[pos] = cp;
+        B.sm[pos] = sm;
+        B.cm[pos] = cm;
+        if (fe) {
+            fe[pos] = FastEdge{(double)x, (double)y, (float)cm, (float)sm, (float)cp, (float)sp};
+            double s2, c2;
+            sincos((double)th, &s2, &c2);
+            cs2[pos] = make_double2(c2, s2);
+        }
         B.cell[pos] = make_int2(lrint_dev(x), lrint_dev(y));
         B.orig[pos] = e;
         B.map[pos] = map_of(map_off, M, e);
@@ -477,8 +501,9 @@ struct NbArgsT {
     const unsigned long long *pair_off;  // FILL: [N+1] internal order
     int *csr_ids;                        // FILL: internal neighbour indices, by pair
     T *csr_d2;                           // FILL (optional): squared distances
-    unsigned char *pcls;                 // FILL (optional): run | close << 2 per pair
+    unsigned char *pcls;                 // FILL (optional): run | close << 2 | branch1 << 3 per pair
     int *pair_anchor;                    // FILL (optional): internal anchor of each pair
+    const double2 *cs2;                  // FILL (optional): cos/sin(T2) of each edge, in place of its own sincos
     T *atrig;                            // FILL (optional): [N][2Q + 2] sin/cos(T2 + delta_t2_j), cos/sin(T2)
     unsigned *err;
     unsigned *uncertified;               // FILL (optional): set when a trig value fails certify_trig
@@ -598,7 +623,11 @@ __global__ void __launch_bounds__(256, MODE == NB_COUNT ? 8 : 6) k_nb(const __gr
         // (tests/probes/sincos_identity.cu compares them on the device, double and float).
         const T T2 = a.B.th[i];
         T cosT2 = T(0), sinT2 = T(0);
-        if (a.pcls || a.atrig) {
+        if (a.cs2) {  // (no trig row is asked for then)
+            const double2 v = a.cs2[i];
+            cosT2 = T(v.x);
+            sinT2 = T(v.y);
+        } else if (a.pcls || a.atrig) {
             T sT2 = T(0), cT2 = T(0);
             T *row = a.atrig ? a.atrig + (size_t)i * (2 * md.Q + 2) : nullptr;
             for (int j = lane; j <= md.Q; j += 32) {
@@ -642,7 +671,8 @@ __global__ void __launch_bounds__(256, MODE == NB_COUNT ? 8 : 6) k_nb(const __gr
                 const unsigned run = direction_class(ax, ay, lx, ly, cosT2, sinT2);
                 const T DX = ax - lx, DY = ay - ly;
                 const bool close = (DX * DX + DY * DY < md.four_dx_dx);
-                a.pcls[off + rk] = (unsigned char)(run | (close ? 4u : 0u));
+                const bool branch1 = (DX * cosT2 + DY * sinT2) < 0;  // :690
+                a.pcls[off + rk] = (unsigned char)(run | (close ? 4u : 0u) | (branch1 ? 8u : 0u));
             }
         }
         __syncwarp();

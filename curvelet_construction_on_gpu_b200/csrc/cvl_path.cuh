@@ -145,58 +145,85 @@ __device__ __forceinline__ bool markstein_numerator(double a) {
 //   QUOT_CHECKED the same, with every operand's range tested in each cell.
 // All three give the same bits. A cell whose e1 is zero, or whose significand is
 // among the largest (high_significand), divides.
+//
+// A column's operands: the k_dt bounds' triples chosen once (branch 1 takes its lower
+// one from s_m and its upper one from s_p, branch 2 the other way round, :731-744,
+// :787-800; the branch is the pair's).
+struct TransportColumn {
+    double DX2, DY2, tt, tt2, dx_2;
+    double s_lo, s_hi, c_lo, c_hi, n_lo, n_hi;
+    bool branch1;
+};
+
+__device__ __forceinline__ TransportColumn transport_column(const Model &md, const PairGeom &g2, double tt, double s_m,
+                                                            double s_p) {
+    TransportColumn t;
+    t.DX2 = g2.DX2;
+    t.DY2 = g2.DY2;
+    t.tt = tt;
+    t.tt2 = 2.0 * tt;
+    t.dx_2 = 2.0 * md.dx;
+    t.s_lo = g2.branch1 ? s_m : s_p;
+    t.s_hi = g2.branch1 ? s_p : s_m;
+    t.c_lo = g2.branch1 ? g2.cos_m_DX : g2.cos_p_DX;
+    t.c_hi = g2.branch1 ? g2.cos_p_DX : g2.cos_m_DX;
+    t.n_lo = g2.branch1 ? g2.sin_m_DY : g2.sin_p_DY;
+    t.n_hi = g2.branch1 ? g2.sin_p_DY : g2.sin_m_DY;
+    t.branch1 = g2.branch1;
+    return t;
+}
+
+// One cell of a column: delta_x2 and its multiples d2_2 = 2 delta_x2, dsq = delta_x2^2.
+template <int QUOT>
+__device__ __forceinline__ void bundle_cell_fp64(const Model &md, double delta_x2, double d2_2, double dsq,
+                                                 const TransportColumn &t, double &bmin, double &bmax) {
+    const double ttmdx2_2 = t.tt2 - d2_2;                            // 2 ttmdx2
+    const double lo2 = ttmdx2_2 - t.dx_2, hi2 = ttmdx2_2 + t.dx_2;  // 2 (ttmdx2 -+ dx)
+    const double e1 = (((t.DX2 - d2_2 * t.tt) + t.DY2) - md.dx2) + dsq;
+    double k_dx_min, k_dx_max;
+    // The one value where branch 2's eq is not e1 * 0.5: when e1 cancels to
+    // +0, branch 2's sum cancels to +0 as well and its eq is -(+0) / 2 = -0,
+    // so its k_dx are the infinities of the other sign (0 / 0 stays NaN).
+    auto divide = [&] {
+        k_dx_min = lo2 / e1;
+        k_dx_max = hi2 / e1;
+        if (e1 == 0.0 && !t.branch1) {
+            k_dx_min = -k_dx_min;
+            k_dx_max = -k_dx_max;
+        }
+    };
+    if constexpr (QUOT != QUOT_DIVIDE) {
+        const double y = __drcp_rn(e1);
+        k_dx_min = markstein_quotient(lo2, e1, y);
+        k_dx_max = markstein_quotient(hi2, e1, y);
+        bool by_division = e1 == 0.0 || high_significand(e1);
+        if constexpr (QUOT == QUOT_CHECKED)
+            by_division = by_division || !markstein_range(e1) || !markstein_numerator(lo2) ||
+                          !markstein_numerator(hi2);
+        if (by_division) divide();
+    } else {
+        divide();
+    }
+    bmin = -md.max_k;
+    bmax = md.max_k;
+    if (bmin < k_dx_min) bmin = k_dx_min;
+    if (bmax > k_dx_max) bmax = k_dx_max;
+    const double k2min = t.s_lo / (-t.s_lo * delta_x2 + t.c_lo + t.n_lo);
+    const double k2max = t.s_hi / (-t.s_hi * delta_x2 + t.c_hi + t.n_hi);
+    if (bmin < k2min) bmin = k2min;
+    if (bmax > k2max) bmax = k2max;
+}
+
 template <int QUOT, class Store>
 __device__ __forceinline__ bool bundle_column_fp64(const Model &md, const double *dx2, const double *dx2_2,
                                                    const double *dx2sq, const PairGeom &g2, double tt, double s_m,
                                                    double s_p, Store &&store) {
-    const double dx_2 = 2.0 * md.dx;
-    const double tt2 = 2.0 * tt;
-    // The k_dt bounds: branch 1 takes its lower one from s_m and its upper one from
-    // s_p, branch 2 the other way round (:731-744, :787-800). The branch is the
-    // pair's, so the operand triples are chosen once here.
-    const double s_lo = g2.branch1 ? s_m : s_p, s_hi = g2.branch1 ? s_p : s_m;
-    const double c_lo = g2.branch1 ? g2.cos_m_DX : g2.cos_p_DX;
-    const double c_hi = g2.branch1 ? g2.cos_p_DX : g2.cos_m_DX;
-    const double n_lo = g2.branch1 ? g2.sin_m_DY : g2.sin_p_DY;
-    const double n_hi = g2.branch1 ? g2.sin_p_DY : g2.sin_m_DY;
+    const TransportColumn t = transport_column(md, g2, tt, s_m, s_p);
     bool open = false;
 #pragma unroll 1  // (measured: unrolling by 2 or 3 is 1-2% slower, with or without a larger register budget)
     for (int i = 0; i < md.P; ++i) {
-        const double delta_x2 = dx2[i], d2_2 = dx2_2[i];
-        const double ttmdx2_2 = tt2 - d2_2;                          // 2 ttmdx2
-        const double lo2 = ttmdx2_2 - dx_2, hi2 = ttmdx2_2 + dx_2;  // 2 (ttmdx2 -+ dx)
-        const double e1 = (((g2.DX2 - d2_2 * tt) + g2.DY2) - md.dx2) + dx2sq[i];
-        double k_dx_min, k_dx_max;
-        // The one value where branch 2's eq is not e1 * 0.5: when e1 cancels to
-        // +0, branch 2's sum cancels to +0 as well and its eq is -(+0) / 2 = -0,
-        // so its k_dx are the infinities of the other sign (0 / 0 stays NaN).
-        auto divide = [&] {
-            k_dx_min = lo2 / e1;
-            k_dx_max = hi2 / e1;
-            if (e1 == 0.0 && !g2.branch1) {
-                k_dx_min = -k_dx_min;
-                k_dx_max = -k_dx_max;
-            }
-        };
-        if constexpr (QUOT != QUOT_DIVIDE) {
-            const double y = __drcp_rn(e1);
-            k_dx_min = markstein_quotient(lo2, e1, y);
-            k_dx_max = markstein_quotient(hi2, e1, y);
-            bool by_division = e1 == 0.0 || high_significand(e1);
-            if constexpr (QUOT == QUOT_CHECKED)
-                by_division = by_division || !markstein_range(e1) || !markstein_numerator(lo2) ||
-                              !markstein_numerator(hi2);
-            if (by_division) divide();
-        } else {
-            divide();
-        }
-        double bmin = -md.max_k, bmax = md.max_k;
-        if (bmin < k_dx_min) bmin = k_dx_min;
-        if (bmax > k_dx_max) bmax = k_dx_max;
-        const double k2min = s_lo / (-s_lo * delta_x2 + c_lo + n_lo);
-        const double k2max = s_hi / (-s_hi * delta_x2 + c_hi + n_hi);
-        if (bmin < k2min) bmin = k2min;
-        if (bmax > k2max) bmax = k2max;
+        double bmin, bmax;
+        bundle_cell_fp64<QUOT>(md, dx2[i], dx2_2[i], dx2sq[i], t, bmin, bmax);
         open = open || (bmax > bmin);
         store(i, bmin, bmax);
     }
