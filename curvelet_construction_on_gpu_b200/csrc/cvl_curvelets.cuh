@@ -58,6 +58,7 @@
 #pragma once
 
 #include "cvl_path.cuh"
+#include "cvl_search.cuh"
 
 namespace cvl {
 
@@ -132,6 +133,7 @@ inline FastModel make_fast(const Model &md) {
 struct FastBinned {
     FastEdge *e;     // [N], bucket order
     double2 *cs2;    // [N] cos(theta), sin(theta)
+    int4 *at;        // [N] pixel cell, input index, map
 };
 
 // Records of k_curvelets: ids[slot][gms] internal edge indices, the seed's first (its
@@ -143,7 +145,7 @@ struct FastArgs {
     BinnedT<double> B;
     FastBinned F;
     int a_begin, a_end;
-    const unsigned long long *pair_off;
+    const unsigned long long *row;      // [N] the anchors' rows (pack_row)
     const int *csr_ids;
     const unsigned char *pcls;          // run | close << 2 | branch1 << 3
     unsigned *rec_ids, *rec_meta;
@@ -161,7 +163,6 @@ struct FastArgs {
     unsigned *over_cnt;                 // anchors k_curvelets leaves to k_curvelets_exact
     int *over_list;
     const unsigned *uncertified;        // bit 1: an orientation is outside the certified range
-    unsigned long long pair_cap;        // graph runs: pairs the CSR holds (0: sized to the run)
 };
 
 constexpr unsigned L_KMASK = 0x3ffu, L_NOSEED = 0x2000u, L_CLOSE = 0x4000u, L_BRANCH1 = 0x8000u;
@@ -538,10 +539,10 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
     };
     for (int t = QUEUE ? next_tile(0) : (int)blockIdx.x * FAST_WARPS + wib; t < tiles; t = next_tile(t))
     for (int i = a.a_begin + t * a.tile, i_end = min(i + a.tile, a_end); i < i_end; ++i) {
-        const unsigned long long off = a.pair_off[i];
-        const int deg = (int)(a.pair_off[i + 1] - off);
-        // a graph run beyond its pair buffers has no rows there (k_nb raised ERR_CAPACITY)
-        if (a.pair_cap && off + (unsigned long long)deg > a.pair_cap) continue;
+        const unsigned long long row = a.row[i];
+        if (row == NO_ROW) continue;  // (ERR_CAPACITY is raised: the run is run again)
+        const unsigned long long off = row & ((1ull << 48) - 1ull);
+        const int deg = (int)(row >> 48);
         const bool joint = deg <= FAST_CAP;  // both runs' pairs in one pass
         __syncwarp();
         fast_trig(T, a.F.cs2[i], Q, lane, S.trig);
@@ -845,8 +846,9 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
     FastCounts counts;
     for (int it = (int)blockIdx.x * FAST_WARPS + wib; it < n_over; it += (int)gridDim.x * FAST_WARPS) {
         const int i = a.over_list[it];
-        const unsigned long long off = a.pair_off[i];
-        const int deg = (int)(a.pair_off[i + 1] - off);
+        const unsigned long long row = a.row[i];
+        const unsigned long long off = row & ((1ull << 48) - 1ull);
+        const int deg = (int)(row >> 48);
         __syncwarp();
         int cnt0, cnt1;
         unsigned close_cnt;

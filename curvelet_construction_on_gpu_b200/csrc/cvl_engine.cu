@@ -645,9 +645,54 @@ constexpr unsigned long long PERSIST_GROWTH_WARPS_MAX = 160ull * 4 * 8;
 
 // ---- the fused path (cvl_curvelets.cuh) -------------------------------------------
 // The edges as k_curvelets gathers them live in the anchor trig rows' buffer, which the
-// path does not use otherwise: 48 bytes per edge of its 16 (Q + 1), Q >= 3.
+// path does not use otherwise: 64 bytes per edge of its 16 (Q + 1), Q >= 3.
 inline FastBinned fast_binned(const cvl_engine *e, size_t n) {
-    return FastBinned{(FastEdge *)e->atrig.p, (double2 *)((FastEdge *)e->atrig.p + n)};
+    FastBinned F;
+    F.e = (FastEdge *)e->atrig.p;
+    F.cs2 = (double2 *)(F.e + n);
+    F.at = (int4 *)(F.cs2 + n);
+    return F;
+}
+// The one-pass search: pairs into csr_ids / pcls (pair_cap of them), rows into fast_rows.
+SearchArgs search_args(const cvl_engine *e, const Model &md, const BinnedT<double> &B, const FastBinned &F, int n, int M,
+                       unsigned long long pair_cap) {
+    SearchArgs a{};
+    unsigned long long *work = (unsigned long long *)e->work.p;
+    a.md = md;
+    a.B = B;
+    a.e = F.e;
+    a.cs2 = F.cs2;
+    a.at = F.at;
+    a.bstart = (const unsigned *)e->bstart.p;
+    a.N = n;
+    a.M = M;
+    a.row = (unsigned long long *)e->pair_off.p;
+    a.pair_ctr = work + 1;
+    a.pair_cap = pair_cap;
+    a.csr_ids = (int *)e->csr_ids.p;
+    a.pcls = (unsigned char *)e->pcls.p;
+    a.stats = (MapStats *)e->stats.p;
+    a.err = (unsigned *)e->err.p;
+    a.wide_cnt = (unsigned *)(work + 2) + 1;
+    a.wide_list = (int *)e->ncand.p;
+    return a;
+}
+// A window within the 3 x 3 hash blocks around its anchor's.
+template <typename T>
+inline bool search_serves(const ModelT<T> &md) {
+    return md.w <= (1 << SEARCH_SBITS) && md.max_cand > 1;
+}
+
+int launch_search(cvl_engine *e, const SearchArgs &a, int blocks, int wide_blocks) {
+    cudaStream_t s = e->stream;
+    constexpr size_t smem = SEARCH_WARPS * sizeof(SearchSmem);
+    const size_t wide = 8 * nbr_smem_per_warp(a.md.max_cand);
+    CVL_CUDA(cudaFuncSetAttribute(k_search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CVL_CUDA(cudaFuncSetAttribute(k_search_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wide));
+    k_search<<<blocks, SEARCH_WARPS * 32, smem, s>>>(a);
+    CVL_TRY(check_launch("k_search"));
+    k_search_wide<<<wide_blocks, 256, wide, s>>>(a);
+    return check_launch("k_search_wide");
 }
 
 // k_curvelets over the anchors, then k_curvelets_exact over those it left.
@@ -689,11 +734,28 @@ FinalArgs final_args(const cvl_engine *e, const Model &md, const BinnedT<double>
     return f;
 }
 
+// A run's error bits: CVL_EAGAIN where the two-pass search, or the two-kernel path, is to run.
+int fast_status(unsigned h_err) {
+    if (h_err & ERR_NONFINITE) return fail(CVL_EINVAL, "non-finite or out-of-range (|v| >= 1e9) edge coordinate");
+    if (h_err & ERR_CAPACITY) return CVL_EAGAIN;
+    if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
+    return CVL_OK;
+}
+void fast_totals(RunOut &ro) {
+    ro.max_deg = 0;
+    ro.total_pairs = 0;
+    for (const MapStats &st : ro.stats) {
+        ro.max_deg = std::max(ro.max_deg, st.max_deg);
+        ro.total_pairs += st.pairs;
+    }
+}
+
 // (c) + (d) + (e) of a direct run by k_curvelets and k_finalize_exact; a run with a yield
-// hook goes chunk by chunk (anchors [cstart[c], cstart[c + 1])), on short blocks.
+// hook goes chunk by chunk of anchors (about chunk_pairs pairs at 16 per edge), on short blocks.
+// CVL_EAGAIN: the pairs did not fit, or an orientation is outside the enclosures' range.
 int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, const BinnedT<double> &B, const Model &md,
                     int n, int M, const int *d_map_off, const std::vector<int32_t> &map_off_host, int mode,
-                    const cvl_tuning &tn, const std::vector<int> &cstart, int nchunks, RunOut &ro) {
+                    const cvl_tuning &tn, bool two_pass, RunOut &ro) {
     cudaStream_t s = e->stream;
     const int sms = e->prop.multiProcessorCount;
     const bool persist = persistent_chunks(e, n);
@@ -702,15 +764,23 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
     unsigned *queues = (unsigned *)(work + 3);  // anchors taken, anchors pushed to the wide variant
     unsigned *err = (unsigned *)e->err.p;
     MapStats *stats = (MapStats *)e->stats.p;
-    const int launches = e->yield_fn ? nchunks : 1;
+    const long long per_chunk = std::max<long long>(tn.chunk_pairs / 16, 1024);
+    const int launches = e->yield_fn ? (int)((n + per_chunk - 1) / per_chunk) : 1;
     CVL_TRY(e->alloc(e->crank, sizeof(unsigned short) * CELLS_MAX));
     k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
     CVL_TRY(check_launch("k_cell_ranks"));
+    // the rows: where the one-pass search put them, or made from the two passes' offsets in
+    // the output offsets' buffer (written after the rows' last use)
+    unsigned long long *rows = (unsigned long long *)(two_pass ? e->out_off.p : e->pair_off.p);
     for (int attempt = 0;; ++attempt) {
+        if (two_pass) {
+            k_pack_rows<<<short_grid(n, 256), 256, 0, s>>>(n, (const unsigned long long *)e->pair_off.p, rows);
+            CVL_TRY(check_launch("k_pack_rows"));
+        }
         // the chunk tails the warps leave unused: one record per anchor, or a chunk per
         // persistent warp and launch
         unsigned long long cap = std::max<unsigned long long>(e->arena_hint, 4ull * (unsigned long long)n + 4096ull) +
-                                 (unsigned long long)n + (unsigned long long)GROWTH_ARENA_CHUNK * (nchunks + 1) +
+                                 (unsigned long long)n +
                                  (persist ? (unsigned long long)GROWTH_ARENA_CHUNK * blocks * FAST_WARPS : 0ull);
         if (mode == 0) {
             CVL_TRY(e->alloc(e->rec_ids, sizeof(unsigned) * cap * md.gms));
@@ -720,8 +790,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
         }
         cap = std::min<unsigned long long>(cap, 0xffffffffull);  // record indices are 32-bit
         for (int c = 0; c < launches; ++c) {
-            const int a0 = launches == 1 ? 0 : cstart[c], a1 = launches == 1 ? n : cstart[c + 1];
-            if (a1 <= a0) continue;
+            const int a0 = (int)(c * per_chunk), a1 = launches == 1 ? n : (int)std::min<long long>(n, (c + 1) * per_chunk);
             if (e->yield_fn && c > 0) {
                 // let the previous chunk finish, then give the hook the chance to hold
                 // this stream back while others' work goes first
@@ -738,7 +807,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             fa.F = F;
             fa.a_begin = a0;
             fa.a_end = a1;
-            fa.pair_off = (const unsigned long long *)e->pair_off.p;
+            fa.row = rows;
             fa.csr_ids = (const int *)e->csr_ids.p;
             fa.pcls = (const unsigned char *)e->pcls.p;
             fa.rec_ids = (unsigned *)e->rec_ids.p;
@@ -756,7 +825,8 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             fa.tile = persist ? FAST_TILE : 1;
             fa.queue = persist ? queues : nullptr;
             fa.over_cnt = queues + 1;
-            fa.over_list = (int *)e->deg.p;  // (its scan is done)
+            fa.over_list = (int *)e->deg.p;  // (not read any more)
+            fa.uncertified = (const unsigned *)(work + 2);
             const int grid = persist ? blocks : short_grid(a1 - a0, (long long)FAST_WARPS * tn.anchors_per_warp);
             CVL_TRY(launch_curvelets(e, fa, grid, sms * FAST_EXACT_BLOCKS));
             e->mark("curvelets");
@@ -767,7 +837,8 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
             e->mark("end");
             CVL_CUDA(cudaStreamSynchronize(s));
-            if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
+            CVL_TRY(fast_status(h_err));
+            fast_totals(ro);
             return CVL_OK;
         }
         // ---- output positions (anchor-major, compact_curvelet_output)
@@ -783,6 +854,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
         CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaMemcpyAsync(&used, work, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaStreamSynchronize(s));
+        if (!(h_err & ERR_ARENA) || (h_err & ~ERR_ARENA)) CVL_TRY(fast_status(h_err));
         if ((h_err & ERR_ARENA) && attempt == 0) {
             // the record arena was too small: size it to what this input needs and grow the
             // chains again (valid and close pairs are recounted from zero)
@@ -790,10 +862,11 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             for (MapStats &st : ro.stats) st.valid_pairs = st.close_pairs = 0;
             CVL_CUDA(cudaMemcpyAsync(stats, ro.stats.data(), sizeof(MapStats) * M, cudaMemcpyHostToDevice, s));
             CVL_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(unsigned) * 4, s));
-            CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 2, s));
+            CVL_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), s));
             continue;
         }
         if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
+        fast_totals(ro);
         const unsigned long long C = ro.cv_off[M];
         ro.total_curvelets = C;
         CVL_TRY(e->alloc(e->chains, sizeof(unsigned) * C * (md.gms + 1)));
@@ -806,10 +879,11 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
 }
 
 // mode: 0 = full run, 1 = count valid pairs only, 2 = neighbour graph only
+// two_pass: count and fill the neighbour lists even where the one-pass search could serve.
 template <typename R>
 int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const int *d_map_off,
                  const std::vector<int32_t> &map_off_host, ModelT<R> md, int cpl, int mode, bool want_d2,
-                 RunOut &ro) {
+                 RunOut &ro, bool two_pass = false) {
     const int M = (int)map_off_host.size() - 1;
     cudaStream_t s = e->stream;
     // one NVTX range per run on the host timeline, a mark at each stage's end
@@ -826,6 +900,24 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     md.sbits = tn.cell_size == 2 ? 1 : (tn.cell_size == 8 ? 3 : 2);
     const unsigned T = next_pow2(std::max<unsigned long long>((unsigned long long)n, 1024ull));
     md.hash_mask = T - 1;
+    const bool path = (mode != 2);
+    FastModel fm{};
+    if constexpr (std::is_same<R, double>::value) {
+        if (path && e->enclosures_on) fm = make_fast(md);
+    }
+    // The one-pass search's pairs go to the buffers as they are, or to new ones of 32 per edge
+    // (the workloads' mean is 7 to 22; 160 bytes per edge); a run they do not hold, or that
+    // has no room for them, counts first.
+    unsigned long long pair_cap = 0;
+    if (fm.ok && !two_pass && search_serves(md)) {
+        pair_cap = std::min<unsigned long long>(e->csr_ids.bytes / sizeof(int), e->pcls.bytes);
+        if (pair_cap < 4ull * (unsigned long long)n) {
+            pair_cap = 32ull * (unsigned long long)n;
+            if (e->alloc(e->csr_ids, sizeof(int) * pair_cap) != CVL_OK || e->alloc(e->pcls, pair_cap) != CVL_OK)
+                pair_cap = 0;
+        }
+    }
+    if (pair_cap) md.sbits = SEARCH_SBITS;
 
     // ---- workspace for N-sized arrays
     CVL_TRY(e->alloc(e->ehash, sizeof(unsigned) * n));
@@ -869,15 +961,10 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     MapStats *stats = (MapStats *)e->stats.p;
     unsigned long long *arena_ctr = (unsigned long long *)e->work.p;
 
-    const bool path = (mode != 2);
-    FastModel fm{};
     FastBinned F{};
-    if constexpr (std::is_same<R, double>::value) {
-        if (path && e->enclosures_on) fm = make_fast(md);
-        if (fm.ok) {
-            CVL_TRY(e->alloc(e->atrig, sizeof(R) * (size_t)n * (2 * md.Q + 2)));
-            F = fast_binned(e, (size_t)n);
-        }
+    if (fm.ok) {
+        CVL_TRY(e->alloc(e->atrig, sizeof(R) * (size_t)n * (2 * md.Q + 2)));
+        F = fast_binned(e, (size_t)n);
     }
 
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
@@ -895,9 +982,30 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B, (int *)e->pos_of.p,
-                                     F.e, F.cs2, nullptr);
+                                     F.e, F.cs2, F.at, nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
+
+    if constexpr (std::is_same<R, double>::value) {
+        if (pair_cap) {
+            const int sms = e->prop.multiProcessorCount;
+            // a persistent grid; short blocks where others' work is to be let in
+            const SearchArgs sa = search_args(e, md, B, F, n, M, pair_cap);
+            int blocks = short_grid((long long)T, SEARCH_WARPS * 32);
+            if (!e->yield_fn) blocks = std::min(blocks, sms * SEARCH_BLOCKS);
+            CVL_TRY(launch_search(e, sa, blocks, sms * 4));
+            e->mark("neighbors");
+            ro.stats.assign(M, MapStats{});
+            const int rc = run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, false, ro);
+            if (rc != CVL_EAGAIN) return rc;
+            // the two passes, or once more with the pairs' own count of room
+            unsigned long long need = 0;
+            for (const MapStats &st : ro.stats) need += st.pairs;
+            if (need > pair_cap && e->alloc(e->csr_ids, sizeof(int) * need) == CVL_OK && e->alloc(e->pcls, need) == CVL_OK)
+                return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, false);
+            return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, true);
+        }
+    }
 
     // ---- (b) neighbour count, CSR offsets, chunk boundaries
     const int nb_wpb = 8;
@@ -981,7 +1089,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
 
     if constexpr (std::is_same<R, double>::value) {
         if (fast)
-            return run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, cstart, nchunks, ro);
+            return run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, true, ro);
     }
 
     // ---- (c) + (d) per chunk
@@ -1269,7 +1377,8 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     sh.edge_data_sz = sz;
     // (the input rows and map offsets are the caller's, already in place: they are
     // not reallocated here)
-    const FastModel fm = e->enclosures_on ? make_fast(md) : FastModel{};
+    const FastModel fm = e->enclosures_on && search_serves(md) ? make_fast(md) : FastModel{};
+    if (fm.ok) md.sbits = SEARCH_SBITS;
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
         if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off) continue;
         // k_curvelets keeps no bundles, pair flags or numbers in memory
@@ -1359,7 +1468,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B,
-                                             (int *)e->pos_of.p, F.e, F.cs2, dd);
+                                             (int *)e->pos_of.p, F.e, F.cs2, F.at, dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;
@@ -1374,29 +1483,34 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             na.dims = dd;
             na.pair_cap = (unsigned long long)sh.num_pairs;
             const int gn = std::min(short_grid(N, (long long)nb_wpb * 4), sms * 8);
-            k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
-            CVL_TRY(check_launch("k_nb<COUNT>"));
-            k_deg_from_ncand<<<gb, 256, 0, s>>>(N, md.max_cand, (const unsigned *)e->ncand.p, (unsigned *)e->deg.p, dd);
-            CVL_TRY(check_launch("k_deg_from_ncand"));
-            CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->deg.p, N,
-                                                        (unsigned long long *)e->pair_off.p)));
-            if (!fm.ok) {
-                k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
-                                                 (int *)e->chunk_start.p, dd);
-                CVL_TRY(check_launch("k_chunk_starts"));
-                k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
-                                              (const int *)e->chunk_start.p, per_chunk, cap.K, cdp, err);
-                CVL_TRY(check_launch("k_chunk_dims"));
+            if (fm.ok) {
+                SearchArgs sa = search_args(e, md, B, F, N, cap.M, (unsigned long long)sh.num_pairs);
+                sa.dims = dd;
+                CVL_TRY(launch_search(e, sa, std::min(short_grid(T, SEARCH_WARPS * 32), sms * SEARCH_BLOCKS), sms));
+            } else {
+                k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
+                CVL_TRY(check_launch("k_nb<COUNT>"));
+                k_deg_from_ncand<<<gb, 256, 0, s>>>(N, md.max_cand, (const unsigned *)e->ncand.p, (unsigned *)e->deg.p, dd);
+                CVL_TRY(check_launch("k_deg_from_ncand"));
+                CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->deg.p, N,
+                                                            (unsigned long long *)e->pair_off.p)));
+                {
+                    k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
+                                                     (int *)e->chunk_start.p, dd);
+                    CVL_TRY(check_launch("k_chunk_starts"));
+                    k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
+                                                  (const int *)e->chunk_start.p, per_chunk, cap.K, cdp, err);
+                    CVL_TRY(check_launch("k_chunk_dims"));
+                }
+                na.csr_ids = (int *)e->csr_ids.p;
+                na.csr_d2 = nullptr;
+                na.pcls = (unsigned char *)e->pcls.p;
+                na.pair_anchor = (int *)e->pair_anchor.p;
+                na.atrig = (double *)e->atrig.p;
+                na.uncertified = uncertified;
+                k_nb<double, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
+                CVL_TRY(check_launch("k_nb<FILL>"));
             }
-            na.csr_ids = (int *)e->csr_ids.p;
-            na.csr_d2 = nullptr;
-            na.pcls = (unsigned char *)e->pcls.p;
-            na.pair_anchor = fm.ok ? nullptr : (int *)e->pair_anchor.p;
-            na.atrig = fm.ok ? nullptr : (double *)e->atrig.p;
-            na.cs2 = F.cs2;
-            na.uncertified = uncertified;
-            k_nb<double, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
-            CVL_TRY(check_launch("k_nb<FILL>"));
             k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
             CVL_TRY(check_launch("k_cell_ranks"));
             Records rec;
@@ -1411,7 +1525,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 fa.fm = fm;
                 fa.B = B;
                 fa.F = F;
-                fa.pair_off = (const unsigned long long *)e->pair_off.p;
+                fa.row = (const unsigned long long *)e->pair_off.p;
                 fa.csr_ids = (const int *)e->csr_ids.p;
                 fa.pcls = (const unsigned char *)e->pcls.p;
                 fa.rec_ids = rec.ids;
@@ -1427,7 +1541,6 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
                 fa.dims = dd;
                 fa.tile = b == 1 ? FAST_TILE : 1;
-                fa.pair_cap = (unsigned long long)sh.num_pairs;
                 // bucket 1 pulls anchors from the queue; bucket 0's runs are too small for
                 // the atomics to pay
                 fa.queue = b == 1 ? queues : nullptr;
@@ -1500,7 +1613,8 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                                                       (unsigned *)e->chains.p, (double *)e->info.p, dd);
                 CVL_TRY(check_launch("k_finalize"));
             }
-            k_graph_readback<<<(cap.M + 1 + 255) / 256, 256, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
+            k_graph_readback<<<(cap.M + 1 + 255) / 256, 256, 0, s>>>(dd, fm.ok ? arena_ctr + 1 : nullptr,
+                                                                     (const unsigned long long *)e->pair_off.p,
                                                                      (const unsigned long long *)e->out_off.p,
                                                                      d_map_off, (unsigned long long *)e->gread.p);
             CVL_TRY(check_launch("k_graph_readback"));
@@ -1559,6 +1673,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     ro.max_deg = 0;
     for (const MapStats &st : ro.stats) ro.max_deg = std::max(ro.max_deg, st.max_deg);
     ro.total_pairs = P;
+    if (fm.ok) fast_totals(ro);
     ro.cv_off.assign(rb_h + 2, rb_h + 2 + M + 1);
     ro.total_curvelets = C;
     return CVL_OK;

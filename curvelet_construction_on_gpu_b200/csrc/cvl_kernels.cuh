@@ -294,7 +294,7 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bfill, BinnedT<T> B,
                               int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
-                              const RunDims *__restrict__ dims) {
+                              int4 *__restrict__ at, const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
         M = dims->M;
@@ -325,9 +325,12 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
             sincos((double)th, &s2, &c2);
             cs2[pos] = make_double2(c2, s2);
         }
-        B.cell[pos] = make_int2(lrint_dev(x), lrint_dev(y));
+        const int2 cell = make_int2(lrint_dev(x), lrint_dev(y));
+        const int m = map_of(map_off, M, e);
+        B.cell[pos] = cell;
         B.orig[pos] = e;
-        B.map[pos] = map_of(map_off, M, e);
+        B.map[pos] = m;
+        if (fe) at[pos] = make_int4(cell.x, cell.y, e, m);
         pos_of[e] = (int)pos;
     }
 }

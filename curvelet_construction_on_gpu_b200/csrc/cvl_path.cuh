@@ -1111,16 +1111,18 @@ __global__ void k_transport_cells(Model md, const double *__restrict__ ops, int 
 // Utility kernels
 // ---------------------------------------------------------------------------
 // The end of a graph run: its pair and curvelet totals and each map's curvelet
-// offset, for the host to read in one copy: out[0] = P, out[1] = C,
+// offset, for the host to read in one copy: out[0] = P (the one-pass search's counter, or
+// the two passes' last offset), out[1] = C,
 // out[2 + m] = out_off[map_off[m]] for m <= M. out_off is the scan over the
 // bucket's N, with zero counts past the run.
-__global__ void k_graph_readback(const RunDims *__restrict__ dims, const unsigned long long *__restrict__ pair_off,
+__global__ void k_graph_readback(const RunDims *__restrict__ dims, const unsigned long long *__restrict__ pair_ctr,
+                                 const unsigned long long *__restrict__ pair_off,
                                  const unsigned long long *__restrict__ out_off, const int *__restrict__ map_off,
                                  unsigned long long *__restrict__ out) {
     const int N = dims->N, M = dims->M;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m <= M; m += gridDim.x * blockDim.x) {
         if (m == 0) {
-            out[0] = pair_off[N];
+            out[0] = pair_ctr ? *pair_ctr : pair_off[N];
             out[1] = out_off[N];
         }
         if (m <= M) out[2 + m] = out_off[map_off[m]];

@@ -89,6 +89,17 @@ def test_same_bits_with_other_parameters(engine, fp64_engine, over, kind):
     _same(engine.run(e, p), fp64_engine.run(e, p))
 
 
+@pytest.mark.parametrize("kind", ["cluster", "band", "small"])
+def test_same_bits_on_a_fresh_engine(fp64_engine, kind):
+    """The first run's pair buffers are a guess: a map with more pairs goes again."""
+    e = _map(kind)
+    with cvl.Engine() as eng:
+        eng.set_graphs(False)
+        _same(eng.run(e), fp64_engine.run(e))
+        _same(eng.run(e), fp64_engine.run(e))
+        _same(eng.run(e[: len(e) // 2]), fp64_engine.run(e[: len(e) // 2]))
+
+
 def test_same_bits_batched_and_staged(engine, fp64_engine):
     maps = [_map(k) for k in ("small", "cluster", "lattice", "angles", "lines")]
     for maps_ in (maps, maps[:3] + maps[4:]):  # with and without a map outside the certified angles
