@@ -173,6 +173,7 @@ struct cvl_engine {
     bool persist_on = std::getenv("CVL_NO_PERSIST") == nullptr;
     // the transport's k_dx quotient pairs on one reciprocal (CVL_NO_SHARED_QUOTIENTS: divisions)
     bool shared_quot_on = std::getenv("CVL_NO_SHARED_QUOTIENTS") == nullptr;
+    bool served = false;  // a server's engine: others run beside it (copy_result_to_host)
     // decisions on single-precision enclosures (CVL_NO_ENCLOSURES: every bundle in FP64)
     bool enclosures_on = std::getenv("CVL_NO_ENCLOSURES") == nullptr;
     uint64_t ws_epoch = 0;                         // workspace (re)allocations so far
@@ -459,22 +460,22 @@ cudaError_t copy_pieces(void *dst, const void *src, size_t bytes, cudaMemcpyKind
     return cudaSuccess;
 }
 
-// Device -> page-locked host copy of results. RESULT_COPY_SM (the default) copies with a
-// small kernel (RESULT_COPY_BLOCKS blocks), which slows concurrent path kernels far less
-// than a copy-engine transfer does; CVL_RESULT_COPY=ce in the environment selects the
-// copy engine (cudaMemcpyAsync in pieces). A copy that no path kernel runs beside
-// (alone) takes the copy engine, which is faster (53 against 38 GB/s measured).
+// Device -> page-locked host copy of results. The copy engine is the faster way (53 against
+// 38 GB/s), and the kernels write little enough that a transfer beside them hides behind it
+// (24 maps of 8M edges host to host: 49.8 ms, against 66.2 with SM copies). In a server,
+// where other workers' runs wait for the SMs and the link, a small kernel (RESULT_COPY_BLOCKS
+// blocks) leaves the small maps' latency lower (1920x1080 p99 at 50 maps/s 13.3 ms, against
+// 20.3 with the copy engine). CVL_RESULT_COPY=ce or sm in the environment selects one for both.
 constexpr int RESULT_COPY_BLOCKS = 16;
-const bool g_result_copy_sm = [] {
+const int g_result_copy = [] {
     const char *v = std::getenv("CVL_RESULT_COPY");
-    return !(v && std::strcmp(v, "ce") == 0);
+    return !v ? 0 : std::strcmp(v, "ce") == 0 ? 1 : std::strcmp(v, "sm") == 0 ? 2 : 0;
 }();
 
-cudaError_t copy_pieces(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t s);
-
-inline cudaError_t copy_result_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s, bool alone = false) {
+inline cudaError_t copy_result_to_host(const cvl_engine *e, void *dst, const void *src, size_t bytes, cudaStream_t s) {
     if (!bytes) return cudaSuccess;
-    if (alone || !g_result_copy_sm || (bytes & 3) || (((uintptr_t)src | (uintptr_t)dst) & 3))
+    const bool sm = g_result_copy ? g_result_copy == 2 : e->served;
+    if (!sm || (bytes & 3) || (((uintptr_t)src | (uintptr_t)dst) & 3))
         return copy_pieces(dst, src, bytes, cudaMemcpyDeviceToHost, s);
     const int wide = ((((uintptr_t)src | (uintptr_t)dst) | bytes) & 15) == 0 ? 1 : 0;
     k_copy_to_host<<<RESULT_COPY_BLOCKS, 256, 0, s>>>(src, dst, bytes, wide);
@@ -2338,10 +2339,10 @@ int cvl_batch_result_take_map(cvl_batch_result *r, int32_t m, cvl_result **out) 
             std::memcpy(res->chains_p, r->chains + c0 * r->width, sizeof(unsigned) * C * r->width);
             std::memcpy(res->info_p, r->info + c0 * 10, sizeof(double) * C * 10);
         } else {
-            cudaError_t ce = copy_result_to_host(res->chains_p, (const unsigned *)e->chains.p + c0 * r->width,
+            cudaError_t ce = copy_result_to_host(e, res->chains_p, (const unsigned *)e->chains.p + c0 * r->width,
                                                  sizeof(unsigned) * C * r->width, e->stream);
             if (ce == cudaSuccess)
-                ce = copy_result_to_host(res->info_p, (const double *)e->info.p + c0 * 10, sizeof(double) * C * 10,
+                ce = copy_result_to_host(e, res->info_p, (const double *)e->info.p + c0 * 10, sizeof(double) * C * 10,
                                          e->stream);
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
             if (ce != cudaSuccess) {
@@ -2389,6 +2390,10 @@ void cvl_batch_result_free(cvl_batch_result *r) { delete r; }
 int cvl_tuning_bucket(int64_t num_edges) { return bucket_of((long long)num_edges); }
 
 }  // extern "C"
+
+void cvl_engine_set_served(cvl_engine *e) {
+    if (e) e->served = true;
+}
 
 void cvl_engine_set_yield(cvl_engine *e, cvl_yield_fn fn, void *ctx) {
     if (!e) return;
@@ -3237,8 +3242,7 @@ void cvl_contours_free(cvl_contours *c) { delete c; }
 
 
 // =============================================================================
-// Many maps, host to host, with the result copies behind the compute (by SM threads:
-// copy_result_to_host)
+// Many maps, host to host, with the result copies behind the compute
 // =============================================================================
 
 extern "C" int cvl_run_maps(cvl_engine *e, const double *edges, const int32_t *counts, int32_t num_maps,
@@ -3394,13 +3398,12 @@ extern "C" int cvl_run_maps(cvl_engine *e, const double *edges, const int32_t *c
             r->info_p = e->pinned->get(sizeof(double) * (C ? C : 1) * 10);
             if (!r->chains_p || !r->info_p)
                 return cleanup(fail(CVL_ENOMEM, "page-locked result buffers could not be allocated"));
-            if (C) {  // by SM threads beside the next group's compute; the last group's alone
-                const bool alone = g == G - 1;
-                cudaError_t ce = copy_result_to_host(r->chains_p, (const unsigned *)e->chains.p + c0 * W,
-                                                     sizeof(unsigned) * C * W, e->copy_stream, alone);
+            if (C) {  // beside the next group's compute
+                cudaError_t ce = copy_result_to_host(e, r->chains_p, (const unsigned *)e->chains.p + c0 * W,
+                                                     sizeof(unsigned) * C * W, e->copy_stream);
                 if (ce == cudaSuccess)
-                    ce = copy_result_to_host(r->info_p, (const double *)e->info.p + c0 * 10,
-                                             sizeof(double) * C * 10, e->copy_stream, alone);
+                    ce = copy_result_to_host(e, r->info_p, (const double *)e->info.p + c0 * 10,
+                                             sizeof(double) * C * 10, e->copy_stream);
                 if (ce != cudaSuccess) return cleanup(fail(CVL_ECUDA, std::string("result copy: ") + cudaGetErrorString(ce)));
             }
             const MapStats &st = ro.stats[k];

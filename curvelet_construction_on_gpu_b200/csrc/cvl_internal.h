@@ -19,6 +19,9 @@ struct cvl_engine;
 using cvl_yield_fn = void (*)(void *ctx);
 void cvl_engine_set_yield(cvl_engine *e, cvl_yield_fn fn, void *ctx);
 
+// Marks a server's engine: other engines' runs share the device with its own.
+void cvl_engine_set_served(cvl_engine *e);
+
 // Sets aside `bytes` of page-locked host memory in the engine's result arena
 // (one chunk made ahead of time, so results do not pin memory while serving).
 int cvl_engine_reserve_host(cvl_engine *e, size_t bytes);

@@ -350,6 +350,7 @@ int cvl_server_create(const cvl_server_cfg *cfg, const cvl_params *p, cvl_server
             delete s;
             return cvl_fail(rc, msg);
         }
+        cvl_engine_set_served(e);
         s->engines.push_back(e);
         if (w == 0) {
             for (int b = 0; b < CVL_TUNING_BUCKETS; ++b) cvl_engine_get_tuning(e, b, &s->tune[b]);
