@@ -89,6 +89,8 @@ struct FastModel {
     float s0, sR;              // S1 = s0 + sR Rb
     float dtiny;
     int ok;                    // the model is within the enclosures' range
+    unsigned char rank[64];    // best-cell rank of each cell (fill_curvelet_info, :202-219)
+    unsigned char cell_of[64]; // and the cell of each rank
 };
 
 // The enclosures' constants (the bounds above), or ok = 0: outside them the two-kernel
@@ -126,6 +128,20 @@ inline FastModel make_fast(const Model &md) {
     f.s0 = (float)(up * (2.0 * mk * f.d0 + 8.0 * u));
     f.sR = (float)(up * 2.0 * mk * f.dR);
     f.dtiny = (float)(2.0 * u * (5.0 * md.nrad + 6.0 * dm));
+    // the cells ordered by (d, row-major index), with the reference's arithmetic
+    double dist[64];
+    for (int c = 0; c < md.cells; ++c) {
+        const double ddx = md.sx * ((double)(c / md.Q) - ((double)md.P - 1.0) / 2.0);
+        const double ddt = md.st * ((double)(c % md.Q) - ((double)md.Q - 1.0) / 2.0);
+        const double a = ddx * ddx, b = ddt * ddt;
+        dist[c] = a + b;
+    }
+    for (int c = 0; c < md.cells; ++c) {
+        int r = 0;
+        for (int o = 0; o < md.cells; ++o) r += dist[o] < dist[c] || (dist[o] == dist[c] && o < c);
+        f.rank[c] = (unsigned char)r;
+        f.cell_of[r] = (unsigned char)c;
+    }
     f.ok = 1;
     return f;
 }
@@ -155,7 +171,6 @@ struct FastArgs {
     MapStats *stats;
     int count_only;
     unsigned *err;
-    const unsigned short *cell_rank;    // [CELLS_MAX]
     unsigned arena_chunk;               // records a warp reserves at a time
     int tile;                           // consecutive anchors a warp takes at a time
     const RunDims *dims;                // graph runs: the anchors are [0, dims->N)
@@ -203,8 +218,19 @@ __device__ __forceinline__ float rcp_approx(float x) {
 }
 
 // The reference's bounds of one cell of pair (anchor i, neighbour nn), in FP64.
+struct CellAnchor {  // the part of a cell that is the anchor's
+    double d, T2t, sT, cT;
+};
+__device__ __forceinline__ CellAnchor cell_anchor(const Model &md, double T2, int cell) {
+    CellAnchor c;
+    const int ci = cell / md.Q, j = cell - ci * md.Q;
+    c.d = grid_offset(md.sx, ci, md.P);
+    c.T2t = T2 + grid_offset(md.st, j, md.Q);  // :698-702
+    sincos(c.T2t, &c.sT, &c.cT);
+    return c;
+}
 __device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double> &B, double2 cs2, int i, int nn,
-                                           int cell, double &m, double &M) {
+                                           const CellAnchor &c, double &m, double &M) {
     const PairGeom g = pair_geom(md, B.x[i], B.y[i], cs2.x, cs2.y, B.x[nn], B.y[nn], B.sp[nn], B.cp[nn], B.sm[nn],
                                  B.cm[nn]);
     if (g.close) {  // the default bundle (:682-687)
@@ -212,15 +238,14 @@ __device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double
         M = md.max_k;
         return;
     }
-    const int ci = cell / md.Q, j = cell - ci * md.Q;
-    const double T2t = B.th[i] + grid_offset(md.st, j, md.Q);  // :698-702
     const double T0 = B.th[nn];
-    const double s_m = sin(T2t - (T0 - md.dt)), s_p = sin(T2t - (T0 + md.dt));  // :728-729
-    double sT, cT;
-    sincos(T2t, &sT, &cT);
-    const double tt = sT * g.DX - cT * g.DY;  // :705
-    const double d = grid_offset(md.sx, ci, md.P);
-    bundle_cell_fp64<QUOT_DIVIDE>(md, d, 2.0 * d, d * d, transport_column(md, g, tt, s_m, s_p), m, M);
+    const double s_m = sin(c.T2t - (T0 - md.dt)), s_p = sin(c.T2t - (T0 + md.dt));  // :728-729
+    const double tt = c.sT * g.DX - c.cT * g.DY;  // :705
+    bundle_cell_fp64<QUOT_DIVIDE>(md, c.d, 2.0 * c.d, c.d * c.d, transport_column(md, g, tt, s_m, s_p), m, M);
+}
+__device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double> &B, double2 cs2, int i, int nn,
+                                           int cell, double &m, double &M) {
+    exact_cell(md, B, cs2, i, nn, cell_anchor(md, B.th[i], cell), m, M);
 }
 
 // Out of line, for undecided cells: whether the cell is open in the intersection of the
@@ -522,8 +547,8 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
     constexpr int PPR = 4;                   // pairs per round (9 offsets and 64 cells: Q <= 7 samples)
     const int Q = md.Q, pl = lane & (PPR - 1), jl = lane / PPR;  // the lane's pair and sample
     const unsigned lt_mask = (1u << lane) - 1u;
-    const unsigned rank0 = 2 * lane < md.cells ? (unsigned)a.cell_rank[2 * lane] : 0xffffu;
-    const unsigned rank1 = 2 * lane + 1 < md.cells ? (unsigned)a.cell_rank[2 * lane + 1] : 0xffffu;
+    const unsigned rank0 = 2 * lane < md.cells ? (unsigned)a.fm.rank[2 * lane] : 0xffffu;
+    const unsigned rank1 = 2 * lane + 1 < md.cells ? (unsigned)a.fm.rank[2 * lane + 1] : 0xffffu;
     const float h = a.fm.h;
 
     FastCounts counts;
@@ -840,8 +865,8 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
     FastBlockSmem &T = *(FastBlockSmem *)cv_smem;
     FastWideSmem &S = ((FastWideSmem *)(cv_smem + sizeof(FastBlockSmem)))[wib];
     fast_tables(md, T);
-    const unsigned rank0 = 2 * lane < md.cells ? (unsigned)a.cell_rank[2 * lane] : 0xffffu;
-    const unsigned rank1 = 2 * lane + 1 < md.cells ? (unsigned)a.cell_rank[2 * lane + 1] : 0xffffu;
+    const unsigned rank0 = 2 * lane < md.cells ? (unsigned)a.fm.rank[2 * lane] : 0xffffu;
+    const unsigned rank1 = 2 * lane + 1 < md.cells ? (unsigned)a.fm.rank[2 * lane + 1] : 0xffffu;
     const float h = a.fm.h;
     FastCounts counts;
     for (int it = (int)blockIdx.x * FAST_WARPS + wib; it < n_over; it += (int)gridDim.x * FAST_WARPS) {
@@ -992,6 +1017,14 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
 // (e) finalize of k_curvelets' records: chain rows and info rows at anchor-major
 // positions, as k_finalize, with the best cell's k range evaluated here in FP64: the
 // seed's bundle, then the chain's in order, each bound selected as :513-527 does.
+// k_finalize_exact: a lane per curvelet, a warp per tile of 32 anchors (input order). A round
+// of 32 curvelets costs one pair after the other's chain of sines and quotients, which
+// enough warps hide on a large run.
+// k_finalize_small, for runs of up to 64 Ki edges, where latency is what counts: G lanes
+// per curvelet (a power of two, at least group_max_sz), each with one of its pairs, and a
+// warp per 8 anchors. The rows of a round's 32 / G curvelets are consecutive, so they are put
+// together in shared memory and written as one run. (On a 242k-edge map it takes half as long
+// again as k_finalize_exact: what is done once per curvelet leaves most lanes idle.)
 // ---------------------------------------------------------------------------
 struct FinalArgs {
     Model md;
@@ -1004,7 +1037,8 @@ struct FinalArgs {
     const unsigned *rec_base, *run_cnt;
     const unsigned long long *out_off;
     unsigned long long out_cap;
-    const unsigned short *cell_rank;
+    unsigned char cell_of[64];
+    const unsigned *err;  // a run with an error is to be run again, or fails: nothing is written
     unsigned *chains;
     double *info;
     const RunDims *dims;
@@ -1012,12 +1046,8 @@ struct FinalArgs {
 
 __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant__ FinalArgs f) {
     const Model &md = f.md;
-    __shared__ unsigned char cell_of_rank[256];
-    cell_of_rank[threadIdx.x] = 0;
-    __syncthreads();
-    if (threadIdx.x < (unsigned)md.cells) cell_of_rank[f.cell_rank[threadIdx.x] & 0xffu] = (unsigned char)threadIdx.x;
-    __syncthreads();
-    const int N = f.dims ? f.dims->N : f.N, M = f.dims ? f.dims->M : f.M;
+    if (*f.err) return;
+    const int N = f.dims ? f.dims->N : f.N;
     const int W = md.gms + 1;
     const int lane = threadIdx.x & 31;
     const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
@@ -1031,9 +1061,7 @@ __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant
             c0 = f.run_cnt[2 * a];
             const unsigned c1 = f.run_cnt[2 * a + 1];
             dst = f.out_off[a];
-            // (a graph run that is to be run again may have left anchors out: count 0 there,
-            // and run_cnt from an earlier run)
-            if (c0 + c1 > 0 && f.out_off[a + 1] - dst == c0 + c1 && dst + c0 + c1 <= f.out_cap) {
+            if (c0 + c1 > 0 && dst + c0 + c1 <= f.out_cap) {
                 cnt = c0 + c1;
                 rb0 = f.rec_base[2 * a];
                 rb1 = f.rec_base[2 * a + 1];
@@ -1069,7 +1097,7 @@ __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant
             const unsigned long long d = ldst + r;
             const unsigned meta = f.rec_meta[s];
             const int len = (int)(meta & 0xffu);
-            const int cell = (int)cell_of_rank[(meta >> 8) & 0xffu];
+            const int cell = (int)f.cell_of[(meta >> 8) & 0x3fu];
             const unsigned *ids = f.rec_ids + s * (unsigned long long)md.gms;
             unsigned *row = f.chains + d * (unsigned long long)W;
             // the chain row (record_curvelet_chain, :269-276), the best cell's bounds and the length
@@ -1077,8 +1105,9 @@ __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant
             row[1] = (unsigned)(la - lmoff) + 1u;
             const double2 cs2 = f.cs2[i];
             const int seed = (int)ids[0];
+            const CellAnchor ca = cell_anchor(md, f.B.th[i], cell);
             double k_min, k_max;
-            exact_cell(md, f.B, cs2, i, seed, cell, k_min, k_max);
+            exact_cell(md, f.B, cs2, i, seed, ca, k_min, k_max);
             double length = 0.0, px = f.B.x[i], py = f.B.y[i];
             for (int z = 1; z < len; ++z) {
                 const int nn = (int)ids[z];
@@ -1089,7 +1118,7 @@ __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant
                 py = qy;
                 if (nn != seed) {
                     double m, Mx;
-                    exact_cell(md, f.B, cs2, i, nn, cell, m, Mx);
+                    exact_cell(md, f.B, cs2, i, nn, ca, m, Mx);
                     k_min = (k_min < m) ? m : k_min;
                     k_max = (k_max > Mx) ? Mx : k_max;
                 }
@@ -1117,6 +1146,129 @@ __global__ void __launch_bounds__(256, 3) k_finalize_exact(const __grid_constant
             inf[7] = k;
             inf[8] = length;
             inf[9] = quality;
+        }
+    }
+}
+
+constexpr int FINAL_WARPS = 8;
+constexpr int FINAL_ANCHORS = 8;  // of a warp
+template <int G>
+__global__ void __launch_bounds__(FINAL_WARPS * 32, 3) k_finalize_small(const __grid_constant__ FinalArgs f) {
+    constexpr int PER = 32 / G;  // curvelets per round
+    __shared__ double s_info[FINAL_WARPS][PER * 10];
+    __shared__ unsigned s_row[FINAL_WARPS][PER * (G + 1)];
+    const Model &md = f.md;
+    if (*f.err) return;
+    const int N = f.dims ? f.dims->N : f.N;
+    const int W = md.gms + 1;  // <= G + 1
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int q = lane & (G - 1), own = lane / G;
+    const int warp = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
+    const int warps = (int)((gridDim.x * (unsigned)blockDim.x) >> 5);
+    for (long long a0 = (long long)warp * FINAL_ANCHORS; a0 < N; a0 += (long long)warps * FINAL_ANCHORS) {
+        const int a = (int)a0 + lane;
+        unsigned c0 = 0, cnt = 0, rb0 = 0, rb1 = 0;
+        unsigned long long dst = 0;
+        int moff = 0, pos = 0;
+        if (lane < FINAL_ANCHORS && a < N) {
+            c0 = f.run_cnt[2 * a];
+            const unsigned c1 = f.run_cnt[2 * a + 1];
+            dst = f.out_off[a];
+            if (c0 + c1 > 0 && dst + c0 + c1 <= f.out_cap) {
+                cnt = c0 + c1;
+                rb0 = f.rec_base[2 * a];
+                rb1 = f.rec_base[2 * a + 1];
+                pos = f.pos_of[a];
+                moff = f.map_off[f.B.map[pos]];
+            }
+        }
+        unsigned incl = cnt;  // inclusive prefix of the tile's counts
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned o = __shfl_up_sync(FULL, incl, d);
+            if (lane >= d) incl += o;
+        }
+        const unsigned total = __shfl_sync(FULL, incl, 31);
+        // the tile's first row (of its first anchor with curvelets)
+        const unsigned some = __ballot_sync(FULL, cnt > 0);
+        const unsigned long long row0 = __shfl_sync(FULL, dst, some ? __ffs(some) - 1 : 0);
+        for (unsigned e0 = 0; e0 < total; e0 += PER) {
+            const unsigned e = min(e0 + (unsigned)own, total - 1u);
+            int T = 0;  // the anchor of curvelet e: the first lane whose inclusive prefix exceeds e
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+                const unsigned v = __shfl_sync(FULL, incl, T + step - 1);
+                if (v <= e) T += step;
+            }
+            const unsigned r = e - (__shfl_sync(FULL, incl, T) - __shfl_sync(FULL, cnt, T));
+            const unsigned lc0 = __shfl_sync(FULL, c0, T);
+            const unsigned lrb0 = __shfl_sync(FULL, rb0, T), lrb1 = __shfl_sync(FULL, rb1, T);
+            const int lmoff = __shfl_sync(FULL, moff, T);
+            const int i = __shfl_sync(FULL, pos, T);
+            const int la = (int)a0 + T;
+            const unsigned long long s =
+                (r < lc0) ? (unsigned long long)lrb0 + r : (unsigned long long)lrb1 + (r - lc0);
+            const unsigned meta = f.rec_meta[s];
+            const int len = (int)(meta & 0xffu);
+            const int cell = (int)f.cell_of[(meta >> 8) & 0x3fu];
+            const unsigned *ids = f.rec_ids + s * (unsigned long long)md.gms;
+            const int seed = (int)ids[0];
+            // lane 0: the seed's bounds; lane z: the chain's z-th edge, its step's length and
+            // (unless it is the seed) its bounds
+            const int nn = q < len ? (int)ids[q] : seed;
+            const double ax = f.B.x[i], ay = f.B.y[i];
+            double m = 0.0, Mx = 0.0;
+            const bool pair = q == 0 || (q < len && nn != seed);
+            if (pair) exact_cell(md, f.B, f.cs2[i], i, nn, cell, m, Mx);
+            const double qx = f.B.x[nn], qy = f.B.y[nn];
+            double px = __shfl_up_sync(FULL, qx, 1, G), py = __shfl_up_sync(FULL, qy, 1, G);
+            if (q == 1) {  // the first step is from the anchor
+                px = ax;
+                py = ay;
+            }
+            const double step_len = sqrt(sq_dist(px, py, qx, qy));
+            // in the chain's order: the bounds, and the length
+            double k_min = m, k_max = Mx, length = 0.0;
+            const unsigned pairs = __ballot_sync(FULL, pair);
+#pragma unroll
+            for (int z = 1; z < G; ++z) {
+                const double zm = __shfl_sync(FULL, m, z, G), zM = __shfl_sync(FULL, Mx, z, G);
+                const double zl = __shfl_sync(FULL, step_len, z, G);
+                if (pairs >> (own * G + z) & 1u) {
+                    k_min = (k_min < zm) ? zm : k_min;
+                    k_max = (k_max > zM) ? zM : k_max;
+                }
+                if (z < len) length += zl;
+            }
+            // the chain row (record_curvelet_chain, :269-276)
+            unsigned *row = s_row[wib] + own * W;
+            if (q == 0) row[0] = (unsigned)(la - lmoff) + 1u;
+            if (q + 1 < W) row[q + 1] = q == 0 ? (unsigned)(la - lmoff) + 1u : q < len ? (unsigned)(f.B.orig[nn] - lmoff) + 1u : 0u;
+            if (q == 0) {
+                // fill_curvelet_info (:221-255)
+                const double ltheta = f.B.th[i];
+                const int mini = cell / md.Q, minj = cell % md.Q;
+                const double k = (k_max + k_min) / 2.0;
+                const double dx = info_offset(md.sx, mini, md.P);
+                const double dt = info_offset(md.st, minj, md.Q);
+                const double theta = to_2pi(ltheta + dt);
+                double *inf = s_info[wib] + own * 10;
+                inf[0] = (meta >> 24) & 1u ? 1.0 : 0.0;
+                inf[1] = k_max;
+                inf[2] = k_min;
+                inf[3] = ltheta;
+                inf[4] = ax - dx * sin(theta);
+                inf[5] = ay + dx * cos(theta);
+                inf[6] = theta;
+                inf[7] = k;
+                inf[8] = length;
+                inf[9] = (length > 0.0 && len > 0) ? 2.0 / (1.0 * md.nrad / length + 1.0 * length / (double)len) : 0.0;
+            }
+            __syncwarp();
+            const int now = (int)min((unsigned)PER, total - e0);
+            for (int k = lane; k < now * 10; k += 32) f.info[(row0 + e0) * 10ull + k] = s_info[wib][k];
+            for (int k = lane; k < now * W; k += 32) f.chains[(row0 + e0) * (unsigned long long)W + k] = s_row[wib][k];
+            __syncwarp();
         }
     }
 }

@@ -508,7 +508,7 @@ int scan_rec(cvl_engine *e, const TIn *in, size_t n, TOut *out, char *&tmp, size
     }
     const size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     if (nb == 1) {
-        k_scan_tiles<TIn, TOut><<<1, SCAN_THREADS, 0, e->stream>>>(in, n, nullptr, out);
+        k_scan_tiles<TIn, TOut, false><<<1, SCAN_THREADS, 0, e->stream>>>(in, n, nullptr, out);
         return check_launch("k_scan_tiles");
     }
     const size_t need = (2 * nb + 1) * sizeof(TOut);
@@ -519,8 +519,12 @@ int scan_rec(cvl_engine *e, const TIn *in, size_t n, TOut *out, char *&tmp, size
     left -= need;
     k_scan_reduce<TIn, TOut><<<(unsigned)nb, SCAN_THREADS, 0, e->stream>>>(in, n, sums);
     CVL_TRY(check_launch("k_scan_reduce"));
+    if (nb <= SCAN_FEW) {
+        k_scan_tiles<TIn, TOut, false><<<(unsigned)nb, SCAN_THREADS, 0, e->stream>>>(in, n, sums, out);
+        return check_launch("k_scan_tiles");
+    }
     CVL_TRY((scan_rec<TOut, TOut>(e, sums, nb, offs, tmp, left)));
-    k_scan_tiles<TIn, TOut><<<(unsigned)nb, SCAN_THREADS, 0, e->stream>>>(in, n, offs, out);
+    k_scan_tiles<TIn, TOut, true><<<(unsigned)nb, SCAN_THREADS, 0, e->stream>>>(in, n, offs, out);
     return check_launch("k_scan_tiles");
 }
 
@@ -676,6 +680,9 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const BinnedT<doubl
     a.err = (unsigned *)e->err.p;
     a.wide_cnt = (unsigned *)(work + 2) + 1;
     a.wide_list = (int *)e->ncand.p;
+    const long long warps = (long long)e->prop.multiProcessorCount * SEARCH_BLOCKS * SEARCH_WARPS;
+    a.split = 1;
+    while (a.split < 8 && (long long)(md.hash_mask + 1u) / 32 * a.split < warps) a.split *= 2;
     return a;
 }
 // A window within the 3 x 3 hash blocks around its anchor's.
@@ -713,7 +720,7 @@ int launch_curvelets(cvl_engine *e, const FastArgs &a, int blocks, int exact_blo
     return check_launch("k_curvelets_exact");
 }
 
-FinalArgs final_args(const cvl_engine *e, const Model &md, const BinnedT<double> &B, const FastBinned &F, int n, int M,
+FinalArgs final_args(const cvl_engine *e, const Model &md, const FastModel &fm, const BinnedT<double> &B, const FastBinned &F, int n, int M,
                      const int *d_map_off, unsigned long long out_cap) {
     FinalArgs f{};
     f.md = md;
@@ -729,10 +736,25 @@ FinalArgs final_args(const cvl_engine *e, const Model &md, const BinnedT<double>
     f.run_cnt = (const unsigned *)e->run_cnt.p;
     f.out_off = (const unsigned long long *)e->out_off.p;
     f.out_cap = out_cap;
-    f.cell_rank = (const unsigned short *)e->crank.p;
+    std::memcpy(f.cell_of, fm.cell_of, sizeof(f.cell_of));
+    f.err = (const unsigned *)e->err.p;
     f.chains = (unsigned *)e->chains.p;
     f.info = (double *)e->info.p;
     return f;
+}
+
+// n: the most anchors the launch serves (a run's, or its graph's)
+int launch_finalize(cvl_engine *e, const FinalArgs &f, int n) {
+    const int blocks = short_grid(n, 256), small = short_grid(n, FINAL_WARPS * FINAL_ANCHORS);
+    if (n > (64 << 10))
+        k_finalize_exact<<<blocks, 256, 0, e->stream>>>(f);
+    else if (f.md.gms <= 4)
+        k_finalize_small<4><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
+    else if (f.md.gms <= 8)
+        k_finalize_small<8><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
+    else
+        k_finalize_small<16><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
+    return check_launch("k_finalize_exact");
 }
 
 // A run's error bits: CVL_EAGAIN where the two-pass search, or the two-kernel path, is to run.
@@ -767,9 +789,6 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
     MapStats *stats = (MapStats *)e->stats.p;
     const long long per_chunk = std::max<long long>(tn.chunk_pairs / 16, 1024);
     const int launches = e->yield_fn ? (int)((n + per_chunk - 1) / per_chunk) : 1;
-    CVL_TRY(e->alloc(e->crank, sizeof(unsigned short) * CELLS_MAX));
-    k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
-    CVL_TRY(check_launch("k_cell_ranks"));
     // the rows: where the one-pass search put them, or made from the two passes' offsets in
     // the output offsets' buffer (written after the rows' last use)
     unsigned long long *rows = (unsigned long long *)(two_pass ? e->out_off.p : e->pair_off.p);
@@ -821,7 +840,6 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             fa.stats = stats;
             fa.count_only = (mode == 1) ? 1 : 0;
             fa.err = err;
-            fa.cell_rank = (const unsigned short *)e->crank.p;
             fa.arena_chunk = persist ? GROWTH_ARENA_CHUNK : 1;
             fa.tile = persist ? FAST_TILE : 1;
             fa.queue = persist ? queues : nullptr;
@@ -872,8 +890,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
         ro.total_curvelets = C;
         CVL_TRY(e->alloc(e->chains, sizeof(unsigned) * C * (md.gms + 1)));
         CVL_TRY(e->alloc(e->info, sizeof(double) * C * 10));
-        k_finalize_exact<<<short_grid(n, 256), 256, 0, s>>>(final_args(e, md, B, F, n, M, d_map_off, C));
-        CVL_TRY(check_launch("k_finalize_exact"));
+        CVL_TRY(launch_finalize(e, final_args(e, md, fm, B, F, n, M, d_map_off, C), n));
         e->mark("finalize");
         return CVL_OK;
     }
@@ -924,7 +941,6 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->ehash, sizeof(unsigned) * n));
     CVL_TRY(e->alloc(e->bcount, sizeof(unsigned) * (T + 1)));
     CVL_TRY(e->alloc(e->bstart, sizeof(unsigned) * (T + 1)));
-    CVL_TRY(e->alloc(e->bfill, sizeof(unsigned) * (T + 1)));
     CVL_TRY(e->alloc(e->pos_of, sizeof(int) * n));
     CVL_TRY(e->alloc(e->bx, sizeof(R) * n));
     CVL_TRY(e->alloc(e->by, sizeof(R) * n));
@@ -969,7 +985,6 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     }
 
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
-    CVL_CUDA(cudaMemsetAsync(e->bfill.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * M, s));
     CVL_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(unsigned) * 4, s));
     CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 4, s));
@@ -982,7 +997,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(check_launch("k_bin_keys"));
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
-                                     (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B, (int *)e->pos_of.p,
+                                     (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, (int *)e->pos_of.p,
                                      F.e, F.cs2, F.at, nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
@@ -992,7 +1007,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
             const int sms = e->prop.multiProcessorCount;
             // a persistent grid; short blocks where others' work is to be let in
             const SearchArgs sa = search_args(e, md, B, F, n, M, pair_cap);
-            int blocks = short_grid((long long)T, SEARCH_WARPS * 32);
+            int blocks = short_grid((long long)T * sa.split, SEARCH_WARPS * 32);
             if (!e->yield_fn) blocks = std::min(blocks, sms * SEARCH_BLOCKS);
             CVL_TRY(launch_search(e, sa, blocks, sms * 4));
             e->mark("neighbors");
@@ -1381,7 +1396,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     const FastModel fm = e->enclosures_on && search_serves(md) ? make_fast(md) : FastModel{};
     if (fm.ok) md.sbits = SEARCH_SBITS;
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
-        if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off) continue;
+        if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off || w.buf == &cvl_engine::bfill) continue;
         // k_curvelets keeps no bundles, pair flags or numbers in memory
         if (fm.ok && (w.buf == &cvl_engine::bund || w.buf == &cvl_engine::pflag || w.buf == &cvl_engine::pair_anchor ||
                       w.buf == &cvl_engine::rec_k))
@@ -1390,7 +1405,6 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     }
     CVL_TRY(e->alloc(e->gdims, sizeof(RunDims)));
     CVL_TRY(e->alloc(e->gchunks, sizeof(ChunkDims) * (size_t)cap.K));
-    CVL_TRY(e->alloc(e->gread, (size_t)(2 + cap.M + 1) * 8));
     if (!e->gread_host) {
         void *h = nullptr;
         if (cvl_alloc_fault_injected() || cudaMallocHost(&h, graph_readback_bytes() + sizeof(RunDims) + 64) != cudaSuccess) {
@@ -1454,13 +1468,21 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
         const FastBinned F = fm.ok ? fast_binned(e, (size_t)N) : FastBinned{};
         CVL_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         auto enqueue = [&]() -> int {
-            CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
-            CVL_CUDA(cudaMemsetAsync(e->bfill.p, 0, sizeof(unsigned) * (T + 1), s));
-            CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * cap.M, s));
-            CVL_CUDA(cudaMemsetAsync(e->err.p, 0, 16, s));
-            CVL_CUDA(cudaMemsetAsync(e->work.p, 0, 32, s));
-            CVL_CUDA(cudaMemsetAsync(e->count.p, 0, sizeof(unsigned) * N, s));
-            CVL_CUDA(cudaMemsetAsync(e->chunk_start.p, 0, sizeof(int) * (cap.K + 1), s));
+            GraphBegin gbeg{};
+            gbeg.host = dims_h;
+            gbeg.dims = (RunDims *)e->gdims.p;
+            const std::pair<void *, size_t> zero[] = {{e->bcount.p, sizeof(unsigned) * (T + 1)},
+                                                      {e->stats.p, sizeof(MapStats) * cap.M},
+                                                      {e->err.p, 16},
+                                                      {e->work.p, 32},
+                                                      {e->count.p, sizeof(unsigned) * (size_t)N},
+                                                      {e->chunk_start.p, fm.ok ? 0 : sizeof(int) * (cap.K + 1)}};
+            for (int r = 0; r < 6; ++r) {
+                gbeg.zero[r] = (unsigned *)zero[r].first;
+                gbeg.n[r] = (unsigned)(zero[r].second / sizeof(unsigned));
+            }
+            k_graph_begin<<<sms, 256, 0, s>>>(gbeg);
+            CVL_TRY(check_launch("k_graph_begin"));
             const int gb = short_grid(N, 256);
             unsigned *uncertified = (unsigned *)((unsigned long long *)e->work.p + 2);  // zeroed above
             k_bin_keys<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (unsigned *)e->ehash.p,
@@ -1468,7 +1490,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY(check_launch("k_bin_keys"));
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
-                                             (const unsigned *)e->bstart.p, (unsigned *)e->bfill.p, B,
+                                             (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
                                              (int *)e->pos_of.p, F.e, F.cs2, F.at, dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
@@ -1487,7 +1509,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             if (fm.ok) {
                 SearchArgs sa = search_args(e, md, B, F, N, cap.M, (unsigned long long)sh.num_pairs);
                 sa.dims = dd;
-                CVL_TRY(launch_search(e, sa, std::min(short_grid(T, SEARCH_WARPS * 32), sms * SEARCH_BLOCKS), sms));
+                CVL_TRY(launch_search(e, sa, std::min(short_grid((long long)T * sa.split, SEARCH_WARPS * 32), sms * SEARCH_BLOCKS), sms));
             } else {
                 k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
                 CVL_TRY(check_launch("k_nb<COUNT>"));
@@ -1512,8 +1534,10 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 k_nb<double, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
                 CVL_TRY(check_launch("k_nb<FILL>"));
             }
-            k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
-            CVL_TRY(check_launch("k_cell_ranks"));
+            if (!fm.ok) {
+                k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
+                CVL_TRY(check_launch("k_cell_ranks"));
+            }
             Records rec;
             rec.ids = (unsigned *)e->rec_ids.p;
             rec.k = (double *)e->rec_k.p;
@@ -1538,8 +1562,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 fa.count = (unsigned *)e->count.p;
                 fa.stats = stats;
                 fa.err = err;
-                fa.cell_rank = (const unsigned short *)e->crank.p;
-                fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
+                    fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
                 fa.dims = dd;
                 fa.tile = b == 1 ? FAST_TILE : 1;
                 // bucket 1 pulls anchors from the queue; bucket 0's runs are too small for
@@ -1603,10 +1626,9 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->count.p, N,
                                                         (unsigned long long *)e->out_off.p)));
             if (fm.ok) {
-                FinalArgs f = final_args(e, md, B, F, N, cap.M, d_map_off, C_cap);
+                FinalArgs f = final_args(e, md, fm, B, F, N, cap.M, d_map_off, C_cap);
                 f.dims = dd;
-                k_finalize_exact<<<gb, 256, 0, s>>>(f);
-                CVL_TRY(check_launch("k_finalize_exact"));
+                CVL_TRY(launch_finalize(e, f, N));
             } else {
                 k_finalize<double><<<gb, 256, 0, s>>>(md, d_edges, sz, N, d_map_off, cap.M, rec,
                                                       (const unsigned *)e->rec_base.p, (const unsigned *)e->run_cnt.p,
@@ -1614,14 +1636,10 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                                                       (unsigned *)e->chains.p, (double *)e->info.p, dd);
                 CVL_TRY(check_launch("k_finalize"));
             }
-            k_graph_readback<<<(cap.M + 1 + 255) / 256, 256, 0, s>>>(dd, fm.ok ? arena_ctr + 1 : nullptr,
-                                                                     (const unsigned long long *)e->pair_off.p,
-                                                                     (const unsigned long long *)e->out_off.p,
-                                                                     d_map_off, (unsigned long long *)e->gread.p);
-            CVL_TRY(check_launch("k_graph_readback"));
-            CVL_CUDA(cudaMemcpyAsync(rb_h, e->gread.p, (size_t)(2 + cap.M + 1) * 8, cudaMemcpyDeviceToHost, s));
-            CVL_CUDA(cudaMemcpyAsync(stats_h, e->stats.p, sizeof(MapStats) * cap.M, cudaMemcpyDeviceToHost, s));
-            CVL_CUDA(cudaMemcpyAsync(err_h, e->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+            k_graph_end<<<(cap.M + 1 + 255) / 256, 256, 0, s>>>(
+                dd, fm.ok ? arena_ctr + 1 : nullptr, (const unsigned long long *)e->pair_off.p,
+                (const unsigned long long *)e->out_off.p, d_map_off, stats, err, rb_h, stats_h, err_h);
+            CVL_TRY(check_launch("k_graph_end"));
             return CVL_OK;
         };
         const int rc = enqueue();
@@ -1656,7 +1674,6 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     dims_h->N = n;
     dims_h->M = M;
     e->mark("start");
-    CVL_CUDA(cudaMemcpyAsync(e->gdims.p, dims_h, sizeof(RunDims), cudaMemcpyHostToDevice, s));
     CVL_CUDA(cudaGraphLaunch(slot->exec, s));
     e->mark("graph");
     CVL_CUDA(cudaStreamSynchronize(s));

@@ -292,7 +292,7 @@ __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int
 template <typename T>
 __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const int *__restrict__ map_off,
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
-                              const unsigned *__restrict__ bstart, unsigned *__restrict__ bfill, BinnedT<T> B,
+                              const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
                               int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
                               int4 *__restrict__ at, const RunDims *__restrict__ dims) {
     if (dims) {
@@ -301,7 +301,7 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
     }
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
         const unsigned h = ehash[e];
-        const unsigned pos = bstart[h] + atomicAdd(&bfill[h], 1u);
+        const unsigned pos = bstart[h] + atomicSub(&bcount[h], 1u) - 1u;  // (the counts are not needed any more)
         const T x = edges[(size_t)e * sz + 0];
         const T y = edges[(size_t)e * sz + 1];
         const T th = edges[(size_t)e * sz + 2];

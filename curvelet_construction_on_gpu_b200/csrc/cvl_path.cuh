@@ -1110,22 +1110,44 @@ __global__ void k_transport_cells(Model md, const double *__restrict__ ops, int 
 // ---------------------------------------------------------------------------
 // Utility kernels
 // ---------------------------------------------------------------------------
-// The end of a graph run: its pair and curvelet totals and each map's curvelet
-// offset, for the host to read in one copy: out[0] = P (the one-pass search's counter, or
-// the two passes' last offset), out[1] = C,
-// out[2 + m] = out_off[map_off[m]] for m <= M. out_off is the scan over the
-// bucket's N, with zero counts past the run.
-__global__ void k_graph_readback(const RunDims *__restrict__ dims, const unsigned long long *__restrict__ pair_ctr,
-                                 const unsigned long long *__restrict__ pair_off,
-                                 const unsigned long long *__restrict__ out_off, const int *__restrict__ map_off,
-                                 unsigned long long *__restrict__ out) {
+// The start of a graph run: its sizes from page-locked host memory to the device, and
+// everything a run starts from at zero, in one launch.
+struct GraphBegin {
+    const RunDims *host;
+    RunDims *dims;
+    unsigned *zero[6];  // 16-byte aligned
+    unsigned n[6];      // words
+};
+__global__ void k_graph_begin(const __grid_constant__ GraphBegin g) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+    if (t == 0) *g.dims = *g.host;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {
+        for (unsigned k = t; k < g.n[r] / 4; k += all) ((uint4 *)g.zero[r])[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (t < g.n[r] % 4) g.zero[r][g.n[r] / 4 * 4 + t] = 0u;
+    }
+}
+
+// The end of a graph run, written to page-locked host memory: its pair and curvelet totals
+// (the one-pass search's counter, or the two passes' last offset), each map's curvelet
+// offset and statistics, and the error bits: out[0] = P, out[1] = C, out[2 + m] =
+// out_off[map_off[m]] for m <= M. out_off is the scan over the bucket's N, with zero counts
+// past the run.
+__global__ void k_graph_end(const RunDims *__restrict__ dims, const unsigned long long *__restrict__ pair_ctr,
+                            const unsigned long long *__restrict__ pair_off,
+                            const unsigned long long *__restrict__ out_off, const int *__restrict__ map_off,
+                            const MapStats *__restrict__ stats, const unsigned *__restrict__ err,
+                            unsigned long long *__restrict__ out, MapStats *__restrict__ stats_out,
+                            unsigned *__restrict__ err_out) {
     const int N = dims->N, M = dims->M;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m <= M; m += gridDim.x * blockDim.x) {
         if (m == 0) {
             out[0] = pair_ctr ? *pair_ctr : pair_off[N];
             out[1] = out_off[N];
+            *err_out = *err;
         }
-        if (m <= M) out[2 + m] = out_off[map_off[m]];
+        out[2 + m] = out_off[map_off[m]];
+        if (m < M) stats_out[m] = stats[m];
     }
 }
 

@@ -58,6 +58,8 @@ struct SearchArgs {
     unsigned *err;
     unsigned *wide_cnt;               // anchors for k_search_wide
     int *wide_list;
+    int split;                        // warps that share 32 buckets (a power of two, at most 8): on small runs
+                                      // more warps have a bucket to themselves
     const RunDims *dims;
 };
 
@@ -113,10 +115,11 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(con
     const int w = md.w;
     const float scale = 65000.0f / (float)md.rad_sqr;  // (rounding and truncation keep d2's order)
     SearchCounts counts;
-    for (unsigned b0 = (blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5)) * 32; b0 <= md.hash_mask;
-         b0 += gridDim.x * SEARCH_WARPS * 32) {
+    const unsigned warp = blockIdx.x * SEARCH_WARPS + (threadIdx.x >> 5), split = (unsigned)a.split;
+    const unsigned part = (0xffffffffu / ((1u << split) - 1u)) << (warp & (split - 1u));  // every split-th bit
+    for (unsigned b0 = warp / split * 32; b0 <= md.hash_mask; b0 += gridDim.x * SEARCH_WARPS / split * 32) {
         const unsigned bs = a.bstart[b0 + lane], be = a.bstart[b0 + lane + 1];
-        for (unsigned full = __ballot_sync(FULL, be > bs); full; full &= full - 1) {
+        for (unsigned full = __ballot_sync(FULL, be > bs) & part; full; full &= full - 1) {
             const unsigned c1 = __shfl_sync(FULL, be, __ffs(full) - 1);
             for (unsigned c0 = __shfl_sync(FULL, bs, __ffs(full) - 1); c0 < c1; c0 += 32) {
                 const int i = (int)(c0 + lane);
