@@ -104,23 +104,52 @@ __device__ __forceinline__ bool first_of_link(const uint2 *b, unsigned m, unsign
 }
 
 // ---- 2. degrees, the single child / parent ----------------------------------------
-__global__ void k_link_degrees(Graph g) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp per edge, a lane per entry of its bucket (about 12): the entries of one link find
+// each other by a match, their first by a minimum over them. Buckets of more than 32 entries
+// compare entry by entry. (With a thread per edge each comparison was a load from the
+// bucket: 202 us on a 242k-edge map's 3.0M entries, and k_link_list 130 us.)
+__global__ void __launch_bounds__(256) k_link_degrees(Graph g) {
+    const int lane = threadIdx.x & 31;
+    const int u = (int)(blockIdx.x * 8u + (threadIdx.x >> 5));
     if (u >= g.n) return;
     uint2 *b = g.bucket + g.occ_off[u];
     const unsigned m = (unsigned)(g.occ_off[u + 1] - g.occ_off[u]);
     int od = 0, id = 0, ch = -1, pa = -1;
-    for (unsigned i = 0; i < m; ++i) {
-        if (!first_of_link(b, m, i)) continue;
-        b[i].x |= FIRST_OCC;  // only this thread touches edge u's bucket
-        if (b[i].x & DIR_OUT) {
-            ++od;
-            ch = (int)(b[i].x & ID_MASK);
-        } else {
-            ++id;
-            pa = (int)(b[i].x & ID_MASK);
+    if (m <= 32) {
+        const uint2 e = lane < (int)m ? b[lane] : make_uint2(0xffffffffu, 0u);
+        // (lanes past the bucket match each other only: their id is above every edge's)
+        const unsigned same = __match_any_sync(0xffffffffu, lane < (int)m ? e.x & ID_MASK : 0xffffffffu);
+        const bool first = lane < (int)m && __reduce_min_sync(same, e.y) == e.y;
+        if (first) b[lane].x = e.x | FIRST_OCC;  // only this warp touches edge u's bucket
+        const unsigned outs = __ballot_sync(0xffffffffu, first && (e.x & DIR_OUT));
+        const unsigned ins = __ballot_sync(0xffffffffu, first && !(e.x & DIR_OUT));
+        od = __popc(outs);
+        id = __popc(ins);
+        const unsigned w = e.x & ID_MASK;
+        if (outs) ch = (int)__shfl_sync(0xffffffffu, w, __ffs(outs) - 1);
+        if (ins) pa = (int)__shfl_sync(0xffffffffu, w, __ffs(ins) - 1);
+    } else {
+        for (unsigned i = lane; i < m; i += 32) {
+            if (!first_of_link(b, m, i)) continue;
+            const unsigned x = b[i].x;
+            if (x & DIR_OUT) {
+                ++od;
+                ch = (int)(x & ID_MASK);
+            } else {
+                ++id;
+                pa = (int)(x & ID_MASK);
+            }
         }
+        __syncwarp();  // every lane has compared before an entry is marked
+        for (unsigned i = lane; i < m; i += 32)
+            if (first_of_link(b, m, i)) atomicOr(&b[i].x, FIRST_OCC);  // (marks leave ids and occurrences as they are)
+        od = __reduce_add_sync(0xffffffffu, od);
+        id = __reduce_add_sync(0xffffffffu, id);
+        ch = __reduce_max_sync(0xffffffffu, ch);
+        pa = __reduce_max_sync(0xffffffffu, pa);
     }
+    if (lane != 0) return;
+    // (child and parent are read where there is exactly one)
     g.outdeg[u] = od;
     g.indeg[u] = id;
     g.child[u] = ch;
@@ -132,15 +161,31 @@ __global__ void k_link_degrees(Graph g) {
     g.linked[u] = 0;
 }
 
-// the links leaving each edge in creation order (_cLinks), with their votes
-__global__ void k_link_list(Graph g, const unsigned long long *link_off, int *pe, int *ce, int *votes) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+// the links leaving each edge in creation order (_cLinks), with their votes; a warp per edge
+__global__ void __launch_bounds__(256) k_link_list(Graph g, const unsigned long long *link_off, int *pe, int *ce,
+                                                   int *votes) {
+    const int lane = threadIdx.x & 31;
+    const int u = (int)(blockIdx.x * 8u + (threadIdx.x >> 5));
     if (u >= g.n) return;
     const uint2 *b = g.bucket + g.occ_off[u];
     const unsigned m = (unsigned)(g.occ_off[u + 1] - g.occ_off[u]);
     const unsigned long long base = link_off[u];
     constexpr unsigned OUT_FIRST = DIR_OUT | FIRST_OCC;
-    for (unsigned i = 0; i < m; ++i) {
+    if (m <= 32) {
+        const uint2 e = lane < (int)m ? b[lane] : make_uint2(0u, 0u);
+        const unsigned same = __match_any_sync(0xffffffffu, lane < (int)m ? e.x & ID_MASK : 0xffffffffu);
+        const bool mine = (e.x & OUT_FIRST) == OUT_FIRST;
+        unsigned rank = 0;
+        for (unsigned k = __ballot_sync(0xffffffffu, mine); k; k &= k - 1)
+            rank += __shfl_sync(0xffffffffu, e.y, __ffs(k) - 1) < e.y;
+        if (mine) {
+            pe[base + rank] = u;
+            ce[base + rank] = (int)(e.x & ID_MASK);
+            votes[base + rank] = __popc(same);
+        }
+        return;
+    }
+    for (unsigned i = lane; i < m; i += 32) {
         if ((b[i].x & OUT_FIRST) != OUT_FIRST) continue;
         const unsigned w = b[i].x & ID_MASK;
         unsigned rank = 0, vote = 0;
@@ -218,12 +263,16 @@ __device__ void heap_sort(unsigned *a, long long n) {
 // is marked at most once and the start edge is not stored. So a component of m
 // edges and f start edges stores at most m + f ids; m + 2f are reserved.
 __device__ void trace_component(const Graph &g, const FragOut &o, int start) {
+    // (the walk marks the component as seen: k_trace_cycles takes what no path's head reached)
     long long m = 0, f = 0;
     int v = start;
     do {
+        const unsigned char fl = g.flags[v];
+        const int next = g.succ[v];
         ++m;
-        if (g.flags[v] & F_FIRST) ++f;
-        v = g.succ[v];
+        if (fl & F_FIRST) ++f;
+        g.flags[v] = fl | F_SEEN;
+        v = next;
     } while (v >= 0 && v != start);
     if (f == 0) return;
     const unsigned long long fb = atomicAdd(o.first_ctr, (unsigned long long)f);
@@ -307,7 +356,6 @@ __global__ void k_trace_paths(Graph g, FragOut o) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= g.n) return;
     if (!(g.flags[u] & F_LEGAL) || g.pred[u] >= 0) return;
-    for (int v = u; v >= 0; v = g.succ[v]) g.flags[v] |= F_SEEN;
     trace_component(g, o, u);
 }
 

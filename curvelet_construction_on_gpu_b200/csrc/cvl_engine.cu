@@ -2967,10 +2967,11 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
     g.pred = (int *)w.pred.p;
     g.flags = (unsigned char *)w.flags.p;
     g.linked = (unsigned char *)w.linked.p;
-    k_link_degrees<<<nb, 256, 0, s>>>(g);
+    const int nw = (int)((N + 7) / 8);  // a warp per edge
+    k_link_degrees<<<nw, 256, 0, s>>>(g);
     CVL_TRY(check_launch("k_link_degrees"));
     CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)w.outdeg.p, N, (unsigned long long *)w.loff.p)));
-    k_link_list<<<nb, 256, 0, s>>>(g, (const unsigned long long *)w.loff.p, (int *)w.lpe.p, (int *)w.lce.p,
+    k_link_list<<<nw, 256, 0, s>>>(g, (const unsigned long long *)w.loff.p, (int *)w.lpe.p, (int *)w.lce.p,
                                    (int *)w.lvotes.p);
     CVL_TRY(check_launch("k_link_list"));
     k_link_paths<<<nb, 256, 0, s>>>(g);

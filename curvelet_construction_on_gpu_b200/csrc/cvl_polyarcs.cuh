@@ -47,7 +47,7 @@ struct PolyArgs {
 // starts no earlier than the last edge of the one before).
 template <int CPL>
 __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
-    __shared__ double tab[4][4 * QMAX];
+    __shared__ double tab[4][4 * QMAX + 4];
     __shared__ double cell_dx2[CELLS_MAX];
     __shared__ unsigned char cell_j[CELLS_MAX];
     __shared__ unsigned short cell_rank[CELLS_MAX];
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
     cell_tables_init(md, cell_dx2, cell_j, cell_rank);
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    double *sT = tab[wib], *cT = sT + QMAX, *sM = cT + QMAX, *sP = sM + QMAX;
+    double *sT = tab[wib], *cT = sT + QMAX, *sM = cT + QMAX, *sP = sM + QMAX, *own = sP + QMAX;
     bool on[CPL];
     int cj[CPL];
     double cdx2[CPL];
@@ -79,30 +79,50 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
             ++i;
             const double *A = a.edges + (size_t)ia * a.sz;
             const double ax = A[0], ay = A[1], T2 = A[2];
-            const double cosT2 = cvl_cos(T2), sinT2 = cvl_sin(T2);
+            double cosT2 = 0.0, sinT2 = 0.0;
             __syncwarp();  // the previous start's tables are read
-            for (int j = lane; j < md.Q; j += 32) {
-                const double t = T2 + grid_offset(md.st, j, md.Q);  // T2t = T2 + Dt(j)
-                sT[j] = cvl_sin(t);
-                cT[j] = cvl_cos(t);
+            for (int j = lane; j <= md.Q; j += 32) {
+                const double t = j < md.Q ? T2 + grid_offset(md.st, j, md.Q) : T2;  // T2t = T2 + Dt(j)
+                double sv, cv;
+                sincos(t, &sv, &cv);
+                if (j < md.Q) {
+                    sT[j] = sv;
+                    cT[j] = cv;
+                } else {
+                    sinT2 = sv;
+                    cosT2 = cv;
+                }
             }
+            cosT2 = __shfl_sync(FULL, cosT2, md.Q & 31);
+            sinT2 = __shfl_sync(FULL, sinT2, md.Q & 31);
             // form_a_hypothesis(A, B) and its bundle: false when there is no model
-            // (B not ahead of A) or the bundle is empty
-            auto hypothesis = [&](int ib, double *bmin, double *bmax) -> bool {
-                const double *B = a.edges + (size_t)ib * a.sz;
-                const double bx = B[0], by = B[1], T0 = B[2];
+            // (B not ahead of A) or the bundle is empty. The pair's sines and cosines come from
+            // one sincos, a lane each: sin(T2t_j - T0 + dt) in lanes j < Q, sin(T2t_j - T0 - dt)
+            // in the next Q, T0 + dt's and T0 - dt's in the two after them (sincos gives the
+            // values of sin and cos: tests/probes/sincos_identity.cu). Made one call after the
+            // other, they were most of a step, and a long fragment's steps are one chain.
+            auto hypothesis = [&](double bx, double by, double T0, double *bmin, double *bmax) -> bool {
                 // dot(vPointPoint(A, B), A's orientation) > 0: B ahead of A
                 if (direction_class(ax, ay, bx, by, cosT2, sinT2) != 0u) return false;
-                __syncwarp();  // sM / sP of the previous pair are read
-                for (int j = lane; j < md.Q; j += 32) {
-                    const double t = T2 + grid_offset(md.st, j, md.Q);
-                    sM[j] = cvl_sin(t - (T0 - md.dt));
-                    sP[j] = cvl_sin(t - (T0 + md.dt));
+                const double t_p = T0 + md.dt, t_m = T0 - md.dt;
+                __syncwarp();  // the tables of the previous pair are read
+                for (int j = lane; j < 2 * md.Q + 2; j += 32) {
+                    const int jq = j < md.Q ? j : j - md.Q;
+                    const double t = T2 + grid_offset(md.st, jq, md.Q);
+                    const double arg = j < md.Q ? t - t_m : j < 2 * md.Q ? t - t_p : j == 2 * md.Q ? t_p : t_m;
+                    double sv, cv;
+                    sincos(arg, &sv, &cv);
+                    if (j < md.Q) {
+                        sM[j] = sv;
+                    } else if (j < 2 * md.Q) {
+                        sP[j - md.Q] = sv;
+                    } else {
+                        own[2 * (j - 2 * md.Q)] = sv;
+                        own[2 * (j - 2 * md.Q) + 1] = cv;
+                    }
                 }
                 __syncwarp();
-                const double t_p = T0 + md.dt, t_m = T0 - md.dt;
-                const PairGeom g = pair_geom(md, ax, ay, cosT2, sinT2, bx, by, cvl_sin(t_p), cvl_cos(t_p),
-                                             cvl_sin(t_m), cvl_cos(t_m));
+                const PairGeom g = pair_geom(md, ax, ay, cosT2, sinT2, bx, by, own[0], own[1], own[2], own[3]);
                 bool lv = false;
 #pragma unroll
                 for (int u = 0; u < CPL; ++u) {
@@ -117,12 +137,31 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
                 }
                 return g.close || __any_sync(FULL, lv);
             };
+            // the next edge's position and orientation, one step ahead of their use
+            auto edge_at = [&](int q, double &x, double &y, double &th) {
+                if (q < N) {
+                    const double *B = a.edges + (size_t)ids[q] * a.sz;
+                    x = B[0];
+                    y = B[1];
+                    th = B[2];
+                }
+            };
+            double bx = 0.0, by = 0.0, bth = 0.0, nx = 0.0, ny = 0.0, nth = 0.0;
+            edge_at(i, bx, by, bth);
+            edge_at(i + 1, nx, ny, nth);
             double cmin[CPL], cmax[CPL];
-            if (!hypothesis(ids[i], cmin, cmax)) continue;
+            if (!hypothesis(bx, by, bth, cmin, cmax)) continue;
+            // curvelet::compute_properties: every step counts (the anchor is the front)
+            double L = sqrt((ax - bx) * (ax - bx) + (ay - by) * (ay - by));
             int j = i;
             while (j < N - 1) {
+                const double px = bx, py = by;
+                bx = nx;
+                by = ny;
+                bth = nth;
+                edge_at(j + 2, nx, ny, nth);
                 double rmin[CPL], rmax[CPL];
-                if (!hypothesis(ids[j + 1], rmin, rmax)) break;
+                if (!hypothesis(bx, by, bth, rmin, rmax)) break;
                 // CC_curve_model_3d(cm1, cm2): Kmin = std::max, Kmax = std::min
                 bool lv = false;
 #pragma unroll
@@ -137,6 +176,7 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
                     cmin[u] = rmin[u];
                     cmax[u] = rmax[u];
                 }
+                L += sqrt((px - bx) * (px - bx) + (py - by) * (py - by));
                 ++j;
             }
             // compute_best_fit: the open cell of smallest rank
@@ -161,12 +201,6 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
             if (lane == 0) {
                 const int size = j - iA + 1;
                 double k = (kmax + kmin) / 2;  // set_best_fit's _k
-                // curvelet::compute_properties: every step counts (the anchor is the front)
-                double L = 0;
-                for (int q = iA; q < j; ++q) {
-                    const double *P0 = a.edges + (size_t)ids[q] * a.sz, *P1q = a.edges + (size_t)ids[q + 1] * a.sz;
-                    L += sqrt((P0[0] - P1q[0]) * (P0[0] - P1q[0]) + (P0[1] - P1q[1]) * (P0[1] - P1q[1]));
-                }
                 const double quality = 2 / (1.0 * a.rad / L + 1.0 * L / a.token_len / size);
                 // update_best_fit(middle, end) with _pt = the start edge
                 const double *P1 = a.edges + (size_t)ids[iA + size / 2] * a.sz;

@@ -67,6 +67,23 @@ def test_fuzz_vs_restatement(engine, oracle, seed):
         assert _same(a, b), (seed, mg, gap)
 
 
+@pytest.mark.parametrize("entries", [1, 2, 31, 32, 33, 64, 65, 201])
+def test_bucket_sizes_vs_restatement(engine, oracle, entries):
+    """One edge's occurrences at the edges of the warp (up to 32: a match; more: entry by
+    entry), with repeated links in both directions."""
+    n, hub = 240, 230
+    rng = np.random.default_rng(entries)
+    e = np.c_[rng.uniform(0, 6, (n, 3)), np.ones(n)]
+    ch = np.zeros((entries, 3), np.uint32)
+    for a in range(entries):  # a curvelet of two edges: one entry of the hub's bucket
+        other = 200 + (a * 7) % 23
+        ch[a] = (a + 1, hub, other) if a % 3 else (a + 1, other, hub)
+    for mg in (0, 2):
+        a, b = engine.link_contours(e, ch, cvl.ContourParams(mg, 9.0)), oracle.link_contours(e, ch, mg, 9.0)
+        assert b.links[:, 2].sum() == entries
+        assert _same(a, b)
+
+
 def test_plain_hd_full_size(engine, oracle):
     """The 1920x1080 map (about 250k edges, 500k curvelets): fused on the device."""
     e = synth.plain_hd(1000)
