@@ -35,7 +35,7 @@ constexpr unsigned DIR_OUT = 0x80000000u;    // bucket entry: the link leaves th
 constexpr unsigned FIRST_OCC = 0x40000000u;  // bucket entry: the first occurrence of its link
 constexpr unsigned ID_MASK = 0x3fffffffu;    // edge ids below 2^30
 
-enum : unsigned char { F_LEGAL = 1, F_FIRST = 2, F_SEEN = 4 };
+enum : unsigned char { F_LEGAL = 1, F_FIRST = 2, F_SEEN = 4, F_NO_CHILD = 8, F_NO_PARENT = 16 };
 
 constexpr unsigned ERR_ID = 1u;       // a chain id outside the map
 constexpr unsigned ERR_SCRATCH = 2u;  // scratch sizing violated (never expected)
@@ -45,8 +45,16 @@ struct Graph {
     const unsigned long long *occ_off;  // [n + 1]
     uint2 *bucket;                      // (other | DIR_OUT | FIRST_OCC, occ)
     int *outdeg, *indeg, *child, *parent;
-    int *succ, *pred;
-    unsigned char *flags, *linked;
+    unsigned char *flags;
+    struct Hop *hop;                    // [n] what a trace reads of an edge
+};
+
+// An edge as the trace visits it, one 32-byte sector: a trace is one chain of these loads.
+struct __align__(16) Hop {
+    int child, parent;  // of an edge with exactly one
+    unsigned flags;     // F_*
+    unsigned linked;    // marked by a trace (of the edge's own component only)
+    double x, y;
 };
 
 // row length of a chain row (column 0 is the anchor)
@@ -157,8 +165,9 @@ __global__ void __launch_bounds__(256) k_link_degrees(Graph g) {
     unsigned char f = 0;
     if (od <= 1 && id <= 1) f |= F_LEGAL;                  // edgel_is_legal, static part
     if (od == 1 && id == 1 && pa != ch) f |= F_FIRST;      // edgel_is_legal_first_edgel, static part
+    if (od == 0) f |= F_NO_CHILD;
+    if (id == 0) f |= F_NO_PARENT;
     g.flags[u] = f;
-    g.linked[u] = 0;
 }
 
 // the links leaving each edge in creation order (_cLinks), with their votes; a warp per edge
@@ -201,21 +210,29 @@ __global__ void __launch_bounds__(256) k_link_list(Graph g, const unsigned long 
 }
 
 // ---- 3. component structure --------------------------------------------------------
-__global__ void k_link_paths(Graph g) {
+__global__ void k_link_hops(Graph g, const double *edges, int sz) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= g.n) return;
-    int s = -1, p = -1;
-    if (g.flags[u] & F_LEGAL) {
-        if (g.outdeg[u] == 1 && (g.flags[g.child[u]] & F_LEGAL)) s = g.child[u];
-        if (g.indeg[u] == 1 && (g.flags[g.parent[u]] & F_LEGAL)) p = g.parent[u];
-    }
-    g.succ[u] = s;
-    g.pred[u] = p;
+    const double *E = edges + (size_t)u * sz;
+    Hop h;
+    h.child = g.child[u];
+    h.parent = g.parent[u];
+    h.flags = g.flags[u];
+    h.linked = 0u;
+    h.x = E[0];
+    h.y = E[1];
+    g.hop[u] = h;
+}
+
+// the next legal edge of a legal edge's component, forward or backward; -1: none
+__device__ __forceinline__ int succ_of(const Graph &g, const Hop &h) {
+    return !(h.flags & F_NO_CHILD) && (g.hop[h.child].flags & F_LEGAL) ? h.child : -1;
+}
+__device__ __forceinline__ int pred_of(const Graph &g, const Hop &h) {
+    return !(h.flags & F_NO_PARENT) && (g.hop[h.parent].flags & F_LEGAL) ? h.parent : -1;
 }
 
 struct FragOut {
-    const double *edges;  // AoS [n][sz]: x, y in columns 0, 1
-    int sz;
     double thres;         // gap * gap
     unsigned *first_ids;  // scratch for each component's start edges
     unsigned long long *first_ctr;
@@ -228,9 +245,8 @@ struct FragOut {
 };
 
 // sq_distance (original_code/curvelet_utils.hpp:17-20); the library builds with -fmad=false
-__device__ __forceinline__ double pt_sqd(const FragOut &o, int a, int b) {
-    const double *A = o.edges + (size_t)a * o.sz, *B = o.edges + (size_t)b * o.sz;
-    return (A[0] - B[0]) * (A[0] - B[0]) + (A[1] - B[1]) * (A[1] - B[1]);
+__device__ __forceinline__ double pt_sqd(const Hop &A, const Hop &B) {
+    return (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y);
 }
 
 __device__ void heap_sift(unsigned *a, long long i, long long n) {
@@ -262,18 +278,29 @@ __device__ void heap_sort(unsigned *a, long long n) {
 // (the step that ends it) besides the edges it marks; every edge of the component
 // is marked at most once and the start edge is not stored. So a component of m
 // edges and f start edges stores at most m + f ids; m + 2f are reserved.
+// Both its walks are one chain of loads (a hop's child gives the next hop), which bounds
+// the kernel: the longest path of a 242k-edge map took 224 us with the edge's fields in
+// arrays of their own, three loads one after the other to a step, and all start edges sorted.
+// The least start edge's trace usually marks the whole component, so the others are
+// collected and sorted only when it does not.
 __device__ void trace_component(const Graph &g, const FragOut &o, int start) {
     // (the walk marks the component as seen: k_trace_cycles takes what no path's head reached)
     long long m = 0, f = 0;
-    int v = start;
-    do {
-        const unsigned char fl = g.flags[v];
-        const int next = g.succ[v];
+    int v = start, least = 0x7fffffff;
+    Hop h = g.hop[v];
+    for (;;) {
         ++m;
-        if (fl & F_FIRST) ++f;
-        g.flags[v] = fl | F_SEEN;
-        v = next;
-    } while (v >= 0 && v != start);
+        if (h.flags & F_FIRST) {
+            ++f;
+            least = min(least, v);
+        }
+        g.flags[v] = (unsigned char)(h.flags | F_SEEN);
+        if (h.flags & F_NO_CHILD) break;
+        v = h.child;
+        if (v == start) break;
+        h = g.hop[v];
+        if (!(h.flags & F_LEGAL)) break;
+    }
     if (f == 0) return;
     const unsigned long long fb = atomicAdd(o.first_ctr, (unsigned long long)f);
     const unsigned long long rb = atomicAdd(o.region_ctr, (unsigned long long)(m + 2 * f));
@@ -281,81 +308,82 @@ __device__ void trace_component(const Graph &g, const FragOut &o, int start) {
         atomicOr(o.err, ERR_SCRATCH);
         return;
     }
-    unsigned *firsts = o.first_ids + fb;
-    long long k = 0;
-    v = start;
-    do {
-        if (g.flags[v] & F_FIRST) firsts[k++] = (unsigned)v;
-        v = g.succ[v];
-    } while (v >= 0 && v != start);
-    heap_sort(firsts, f);
     int *out = o.region + rb;
-    long long cur = 0;
+    long long cur = 0, marked = 0;  // ids stored, start edges marked
     const long long cap = m + 2 * f;
-#define CVLC_LEGAL(e) ((g.flags[e] & F_LEGAL) && !g.linked[e])
-#define CVLC_PUT(e)                                  \
-    do {                                             \
-        if (cur >= cap) {                            \
-            atomicOr(o.err, ERR_SCRATCH);            \
-            return;                                  \
-        }                                            \
-        out[cur++] = (e);                            \
-    } while (0)
-    for (long long q = 0; q < f; ++q) {
-        const int s = (int)firsts[q];
-        if (g.linked[s]) continue;
+    auto put = [&](int e) {
+        if (cur < cap) out[cur] = e;
+        ++cur;  // (past cap: ERR_SCRATCH below)
+    };
+    auto trace = [&](int s) {
         const long long src = cur;
         int nf = 0, nb = 0;
-        g.linked[s] = 1;
-        int eA = g.child[s], eB;
-        if (pt_sqd(o, s, eA) < o.thres) {
-            CVLC_PUT(eA);
+        const Hop S = g.hop[s];
+        g.hop[s].linked = 1u;
+        ++marked;
+        int eA = S.child;
+        Hop A = g.hop[eA];
+        if (pt_sqd(S, A) < o.thres) {
+            put(eA);
             ++nf;
         }
-        while (CVLC_LEGAL(eA)) {
-            g.linked[eA] = 1;
-            if (g.outdeg[eA] == 0) break;
-            eB = eA;
-            eA = g.child[eA];
-            if (pt_sqd(o, eB, eA) < o.thres) {
-                CVLC_PUT(eA);
-                ++nf;
-            } else {
-                break;
-            }
+        while ((A.flags & F_LEGAL) && !A.linked) {
+            g.hop[eA].linked = 1u;
+            marked += (A.flags & F_FIRST) != 0;
+            if (A.flags & F_NO_CHILD) break;
+            const Hop B = A;
+            eA = A.child;
+            A = g.hop[eA];
+            if (!(pt_sqd(B, A) < o.thres)) break;
+            put(eA);
+            ++nf;
         }
         if (eA != s) {
-            eA = g.parent[s];
-            if (pt_sqd(o, s, eA) < o.thres) {
-                CVLC_PUT(eA);
+            eA = S.parent;
+            A = g.hop[eA];
+            if (pt_sqd(S, A) < o.thres) {
+                put(eA);
                 ++nb;
             }
-        }
-        while (CVLC_LEGAL(eA)) {
-            g.linked[eA] = 1;
-            if (g.indeg[eA] == 0) break;
-            eB = eA;
-            eA = g.parent[eA];
-            if (pt_sqd(o, eB, eA) < o.thres) {
-                CVLC_PUT(eA);
+            while ((A.flags & F_LEGAL) && !A.linked) {
+                g.hop[eA].linked = 1u;
+                marked += (A.flags & F_FIRST) != 0;
+                if (A.flags & F_NO_PARENT) break;
+                const Hop B = A;
+                eA = A.parent;
+                A = g.hop[eA];
+                if (!(pt_sqd(B, A) < o.thres)) break;
+                put(eA);
                 ++nb;
-            } else {
-                break;
             }
         }
         o.frag_src[s] = rb + src;
         o.frag_nf[s] = nf;
         o.frag_nb[s] = nb;
+    };
+    trace(least);
+    if (marked < f) {
+        unsigned *firsts = o.first_ids + fb;
+        long long k = 0;
+        v = start;
+        do {
+            h = g.hop[v];
+            if ((h.flags & F_FIRST) && !h.linked) firsts[k++] = (unsigned)v;
+            v = succ_of(g, h);
+        } while (v >= 0 && v != start);
+        heap_sort(firsts, k);
+        for (long long q = 0; q < k && marked < f; ++q)
+            if (!g.hop[firsts[q]].linked) trace((int)firsts[q]);
     }
-#undef CVLC_PUT
-#undef CVLC_LEGAL
+    if (cur > cap) atomicOr(o.err, ERR_SCRATCH);
 }
 
 // components that are paths: entered at their head (no legal predecessor)
 __global__ void k_trace_paths(Graph g, FragOut o) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= g.n) return;
-    if (!(g.flags[u] & F_LEGAL) || g.pred[u] >= 0) return;
+    const Hop h = g.hop[u];
+    if (!(h.flags & F_LEGAL) || pred_of(g, h) >= 0) return;
     trace_component(g, o, u);
 }
 
@@ -365,17 +393,17 @@ __global__ void k_trace_cycles(Graph g, FragOut o) {
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= g.n) return;
     if (!(g.flags[u] & F_LEGAL) || (g.flags[u] & F_SEEN)) return;
-    int a = g.succ[u], b = g.pred[u];
+    int a = succ_of(g, g.hop[u]), b = pred_of(g, g.hop[u]);
     for (;;) {
         if (a < 0 || b < 0) return;  // not a cycle (cannot happen for an unseen legal edge)
         if (a == u) break;           // walked all the way round: u is the smallest
         if (a < u || b < u) return;
         if (a == b) break;           // the two walks met
-        a = g.succ[a];
+        a = succ_of(g, g.hop[a]);
         if (a == u) break;
         if (a < u) return;
         if (a == b) break;
-        b = g.pred[b];
+        b = pred_of(g, g.hop[b]);
     }
     trace_component(g, o, u);
 }

@@ -146,12 +146,12 @@ struct cvl_engine {
     cudaEvent_t copied[2] = {nullptr, nullptr};
     // downstream stage (link graph, contour fragments)
     struct ContourBufs {
-        DBuf chains_in, cnt, off, cursor, bucket, outdeg, indeg, child, parent, succ, pred, flags, linked, firsts,
+        DBuf chains_in, cnt, off, cursor, bucket, outdeg, indeg, child, parent, flags, hop, firsts,
             region, ctr, fsrc, fnf, fnb, isfrag, flen, fidx, idoff, loff, lpe, lce, lvotes, fragoff, fragids, err,
             pstart, psize, pinfo, pcount, poff, pstart2, psize2, pinfo2;
         DBuf *all(int i) {
-            DBuf *b[] = {&chains_in, &cnt, &off, &cursor, &bucket, &outdeg, &indeg, &child, &parent, &succ,
-                         &pred, &flags, &linked, &firsts, &region, &ctr, &fsrc, &fnf, &fnb, &isfrag,
+            DBuf *b[] = {&chains_in, &cnt, &off, &cursor, &bucket, &outdeg, &indeg, &child, &parent, &flags,
+                         &hop, &firsts, &region, &ctr, &fsrc, &fnf, &fnb, &isfrag,
                          &flen, &fidx, &idoff, &loff, &lpe, &lce, &lvotes, &fragoff, &fragids, &err,
                          &pstart, &psize, &pinfo, &pcount, &poff, &pstart2, &psize2, &pinfo2};
             return i < (int)(sizeof(b) / sizeof(b[0])) ? b[i] : nullptr;
@@ -2913,10 +2913,8 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
     CVL_TRY(e->alloc(w.indeg, sizeof(int) * N));
     CVL_TRY(e->alloc(w.child, sizeof(int) * N));
     CVL_TRY(e->alloc(w.parent, sizeof(int) * N));
-    CVL_TRY(e->alloc(w.succ, sizeof(int) * N));
-    CVL_TRY(e->alloc(w.pred, sizeof(int) * N));
     CVL_TRY(e->alloc(w.flags, N));
-    CVL_TRY(e->alloc(w.linked, N));
+    CVL_TRY(e->alloc(w.hop, sizeof(Hop) * N));
     CVL_TRY(e->alloc(w.loff, sizeof(unsigned long long) * (N + 1)));
     CVL_TRY(e->alloc(w.lpe, sizeof(int) * std::max<unsigned long long>(occ_cap / 2, 1)));
     CVL_TRY(e->alloc(w.lce, sizeof(int) * std::max<unsigned long long>(occ_cap / 2, 1)));
@@ -2963,10 +2961,8 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
     g.indeg = (int *)w.indeg.p;
     g.child = (int *)w.child.p;
     g.parent = (int *)w.parent.p;
-    g.succ = (int *)w.succ.p;
-    g.pred = (int *)w.pred.p;
     g.flags = (unsigned char *)w.flags.p;
-    g.linked = (unsigned char *)w.linked.p;
+    g.hop = (Hop *)w.hop.p;
     const int nw = (int)((N + 7) / 8);  // a warp per edge
     k_link_degrees<<<nw, 256, 0, s>>>(g);
     CVL_TRY(check_launch("k_link_degrees"));
@@ -2974,11 +2970,9 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
     k_link_list<<<nw, 256, 0, s>>>(g, (const unsigned long long *)w.loff.p, (int *)w.lpe.p, (int *)w.lce.p,
                                    (int *)w.lvotes.p);
     CVL_TRY(check_launch("k_link_list"));
-    k_link_paths<<<nb, 256, 0, s>>>(g);
-    CVL_TRY(check_launch("k_link_paths"));
+    k_link_hops<<<nb, 256, 0, s>>>(g, d_edges, sz);
+    CVL_TRY(check_launch("k_link_hops"));
     FragOut o;
-    o.edges = d_edges;
-    o.sz = sz;
     o.thres = cp.gap * cp.gap;
     o.first_ids = (unsigned *)w.firsts.p;
     o.first_ctr = (unsigned long long *)w.ctr.p;
