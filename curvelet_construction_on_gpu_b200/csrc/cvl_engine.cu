@@ -601,13 +601,14 @@ using bundles_fn = int (*)(cvl_engine *, BundleArgsT<T> &, int);
 template <typename T>
 using growth_fn = int (*)(cvl_engine *, GrowthArgsT<T> &, size_t, int);
 
-// Float mode (a parity mode) runs the default variants only.
+// Float mode (a parity mode) runs one variant per grid size: up to 64 cells two seeds together and 64
+// registers (on a 242k-edge map 0.65 ms, against 0.72 for four seeds and 0.86 for four at 96).
 void pick_kernels(int cpl, const cvl_tuning &, bundles_fn<float> &bf, growth_fn<float> &gf) {
     switch (cpl) {
-        case 1: bf = launch_bundles<float, 1, 4>; gf = launch_growth<float, 1, 4, 4>; break;
+        case 1: bf = launch_bundles<float, 1, 4>; gf = launch_growth<float, 1, 2, 8>; break;
         case 3: bf = launch_bundles<float, 3, 4>; gf = launch_growth<float, 3, 4, 4>; break;
         case 4: bf = launch_bundles<float, 4, 4>; gf = launch_growth<float, 4, 4, 4>; break;
-        default: bf = launch_bundles<float, 2, 4>; gf = launch_growth<float, 2, 4, 4>; break;
+        default: bf = launch_bundles<float, 2, 4>; gf = launch_growth<float, 2, 2, 8>; break;
     }
 }
 

@@ -343,15 +343,22 @@ __global__ void __launch_bounds__(BUNDLE_THREADS, MINB * (256 / BUNDLE_THREADS))
     constexpr int BW = 2 * 32 * CPL;
     extern __shared__ __align__(16) unsigned char bn_smem[];
     T *s_b = (T *)bn_smem;  // [PPB][BW]: the block's bundles until their validity is known
-    __shared__ T s_dx2[CELLS_MAX], s_dx2_2[CELLS_MAX], s_dx2sq[CELLS_MAX];
+    constexpr bool F64 = std::is_same<T, double>::value;
+    __shared__ T s_dx2[CELLS_MAX], s_dx2_2[F64 ? CELLS_MAX : 1], s_dx2sq[F64 ? CELLS_MAX : 1];
+    __shared__ double s_m2d[F64 ? 1 : CELLS_MAX], s_sqd[F64 ? 1 : CELLS_MAX];  // float mode: -2 d, d * d
     // each staged pair's flags (bit 0 open, bit 1 close), two sets used in turn by
     // successive tiles: a tile clears the other set after its first barrier
     __shared__ unsigned char s_flag[2][BUNDLE_THREADS];
     for (int i = threadIdx.x; i < md.P; i += blockDim.x) {
         const T d = grid_offset(md.sx, i, md.P);  // delta_x2 (:697)
         s_dx2[i] = d;
-        s_dx2_2[i] = T(2) * d;
-        s_dx2sq[i] = d * d;
+        if constexpr (F64) {
+            s_dx2_2[i] = T(2) * d;
+            s_dx2sq[i] = d * d;
+        } else {
+            s_m2d[i] = -2.0 * (double)d;
+            s_sqd[i] = (double)(d * d);
+        }
     }
     for (int t = threadIdx.x; t < BUNDLE_THREADS; t += blockDim.x) s_flag[0][t] = s_flag[1][t] = 0;
     __syncthreads();
@@ -401,24 +408,31 @@ __global__ void __launch_bounds__(BUNDLE_THREADS, MINB * (256 / BUNDLE_THREADS))
                 const T tt = sTj * g2.DX - cTj * g2.DY;     // :705
                 T *dst = s_b + pl * BW;
                 bool open = false;
-                if constexpr (!std::is_same<T, double>::value) {
-                    // float mode: :693-809 with their C++ types
+                if constexpr (!F64) {
+                    // float mode: :693-809 with their C++ types. Branch 2's denominator (:774) is
+                    // branch 1's (:711) with each term's sign turned, which turns the sign of every
+                    // rounded sum, then halved; so one sequence serves both, with the column's
+                    // terms signed once, and a warp's lanes do not part. The conversions and
+                    // reciprocals go through one slow pipe (67% busy, what bounded the kernel
+                    // with its offsets converted in every cell: 1.11 -> 0.80 ms on a 242k-edge
+                    // map's 2.9M pairs).
+                    const double ttd = g2.branch1 ? (double)tt : -(double)tt;
+                    const double sx2 = g2.branch1 ? (double)g2.DX2 : -(double)g2.DX2;
+                    const double sy2 = g2.branch1 ? (double)g2.DY2 : -(double)g2.DY2;
+                    const double sdx2 = g2.branch1 ? -(double)md.dx2 : (double)md.dx2;
+                    const double half = g2.branch1 ? 1.0 : -0.5;
+                    const T two = g2.branch1 ? T(2) : T(1);
                     for (int i = 0; i < md.P; ++i) {
                         const T delta_x2 = s_dx2[i];
                         const T ttmdx2 = tt - delta_x2;
-                        const T sq = s_dx2sq[i];  // delta_x2 * delta_x2, a T product
-                        T k_dx_min, k_dx_max;
-                        if (g2.branch1) {
-                            const T eq = (T)(((((-2.0 * (double)delta_x2) * (double)tt + (double)g2.DX2) +
-                                               (double)g2.DY2) - (double)md.dx2) + (double)sq);       // :711
-                            k_dx_min = (T)((2.0 * (double)(ttmdx2 - md.dx)) / (double)eq);           // :714
-                            k_dx_max = (T)((2.0 * (double)(ttmdx2 + md.dx)) / (double)eq);           // :715
-                        } else {
-                            const T eq = (T)(-(((((2.0 * (double)delta_x2) * (double)tt - (double)g2.DX2) -
-                                                 (double)g2.DY2) + (double)md.dx2) - (double)sq) / 2.0);  // :774
-                            k_dx_min = (ttmdx2 - md.dx) / eq;                                        // :777
-                            k_dx_max = (ttmdx2 + md.dx) / eq;                                        // :778
-                        }
+                        const double sq = s_sqd[i];  // delta_x2 * delta_x2, a T product
+                        const T eq = (T)(((((s_m2d[i] * ttd + sx2) + sy2) + sdx2) + (g2.branch1 ? sq : -sq)) * half);
+                        // :714-715, a double quotient of two floats rounded to float: that is
+                        // their float quotient (53 bits hold twice a float's 24 and two more,
+                        // so the first rounding cannot change the second; the doubling is exact);
+                        // :777-778 are float quotients
+                        const T k_dx_min = two * (ttmdx2 - md.dx) / eq;
+                        const T k_dx_max = two * (ttmdx2 + md.dx) / eq;
                         const T km = s_m / (-s_m * delta_x2 + g2.cos_m_DX + g2.sin_m_DY);
                         const T kp = s_p / (-s_p * delta_x2 + g2.cos_p_DX + g2.sin_p_DY);
                         T bmin = -md.max_k, bmax = md.max_k;
@@ -553,7 +567,7 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
     int *seed_orig = (int *)(base + (size_t)md.max_cand * 28);         // [max_cand]
     unsigned short *chains = (unsigned short *)(base + (size_t)md.max_cand * 32);  // [max_cand][gms]
     constexpr int BW = 2 * 32 * CPL;
-    constexpr unsigned CLOSE_BIT = 0x80000000u;
+    constexpr unsigned CLOSE_BIT = 0x80000000u, SKIP_BIT = 0x40000000u;
 
     unsigned rank_l[CPL];
     bool on_l[CPL];
@@ -639,7 +653,7 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
             // a run with fewer than two seeds, or group_max_sz <= 2, grows none.
             if (!a.count_only && ns > 1 && md.gms > 2) {
                 auto load_bundle = [&](int s, T *mn, T *mx) {
-                    const unsigned sq = seed_q[s_base + s_step * s];
+                    const unsigned sq = seed_q[s_base + s_step * s] & ~SKIP_BIT;
                     if (sq & CLOSE_BIT) {
 #pragma unroll
                         for (int u = 0; u < CPL; ++u) {
@@ -655,14 +669,19 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                         }
                     }
                 };
-                for (int g0 = 0; g0 < ns; g0 += K) {
-                    T cmin[K][CPL], cmax[K][CPL];
-                    unsigned len[K];
+                // Seed 0 walks alone. Another seed of its chain C has the same chain: its walk
+                // takes and refuses the same seeds (what it joins is a part of C, whose cells are
+                // open together; for what C's walk refused its bundle holds at least as much), and
+                // first-wins drops it. The seeds not in C walk K at a time.
+                auto walk_group = [&](auto kk, const int *sid, int n_sid) {
+                    constexpr int KK = decltype(kk)::value;
+                    T cmin[KK][CPL], cmax[KK][CPL];
+                    unsigned len[KK];
                     unsigned done = 0;
 #pragma unroll
-                    for (int q = 0; q < K; ++q) {
-                        const int s = g0 + q;
-                        if (s < ns) {
+                    for (int q = 0; q < KK; ++q) {
+                        if (q < n_sid) {
+                            const int s = sid[q];
                             load_bundle(s, cmin[q], cmax[q]);
                             len[q] = 1;  // the anchor (:485)
                             if (lane == 0) chains[(size_t)s * md.gms] = 0xffffu;
@@ -678,14 +697,14 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                     // a seed takes a bundle
                     unsigned copen = 0;
 #pragma unroll
-                    for (int q = 0; q < K; ++q)
+                    for (int q = 0; q < KK; ++q)
 #pragma unroll
                         for (int u = 0; u < CPL; ++u)
                             copen |= (on_l[u] && cmax[q][u] > cmin[q][u]) ? 1u << (q * CPL + u) : 0u;
                     // the walk's bundles, one ahead: r + 1 loads while r is intersected
                     T nmin[CPL], nmax[CPL];
                     load_bundle(0, nmin, nmax);
-                    for (int r = 0; r < ns && done != (1u << K) - 1u; ++r) {
+                    for (int r = 0; r < ns && done != (1u << KK) - 1u; ++r) {
                         T rmin[CPL], rmax[CPL];
 #pragma unroll
                         for (int u = 0; u < CPL; ++u) {
@@ -702,7 +721,7 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                         for (int u = 0; u < CPL; ++u) ropen[u] = rmax[u] > rmin[u];
                         unsigned bits = 0;
 #pragma unroll
-                        for (int q = 0; q < K; ++q) {
+                        for (int q = 0; q < KK; ++q) {
                             bool lv = false;
 #pragma unroll
                             for (int u = 0; u < CPL; ++u)
@@ -712,9 +731,9 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                         }
                         bits = __reduce_or_sync(FULL, bits);  // bundle_intersection_valid_check (:845-854)
 #pragma unroll
-                        for (int q = 0; q < K; ++q) {
+                        for (int q = 0; q < KK; ++q) {
                             if (done & (1u << q)) continue;
-                            const int s = g0 + q;
+                            const int s = sid[q];
                             if (r == s) {
                                 // the seed itself joins without intersection (:496-511)
                                 if (lane == 0) chains[(size_t)s * md.gms + len[q]] = (unsigned short)r;
@@ -742,9 +761,9 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                     // among open cells; none -> cell 0, mini = minj = 0, :202-204),
                     // k_max, k_min, and the length tag of its chain (len > 2, :549)
 #pragma unroll
-                    for (int q = 0; q < K; ++q) {
-                        const int s = g0 + q;
-                        if (s >= ns) continue;
+                    for (int q = 0; q < KK; ++q) {
+                        if (q >= n_sid) continue;
+                        const int s = sid[q];
                         unsigned best = 0xffffu;
 #pragma unroll
                         for (int u = 0; u < CPL; ++u)
@@ -781,8 +800,8 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                     __syncwarp();
                     // dedup: a chain identical to an earlier seed's chain of this run is
                     // dropped (the first one wins, check_curvelet_exist, :876-916)
-                    const int g1 = (g0 + K < ns) ? g0 + K : ns;
-                    for (int s = g0; s < g1; ++s) {
+                    for (int q = 0; q < n_sid; ++q) {
+                        const int s = sid[q];
                         double *rs = res + (size_t)s * 3;
                         const unsigned meta = (unsigned)rs[2];
                         if (meta == 0u) continue;
@@ -804,7 +823,32 @@ __global__ void __launch_bounds__(GROWTH_THREADS, 4 * MINB) k_growth(GrowthArgsT
                         }
                     }
                     __syncwarp();
+                };
+                int sid[K] = {};
+                walk_group(std::integral_constant<int, 1>{}, sid, 1);
+                for (unsigned z = 1 + lane; z < (chains[0] & 0xffu) && chains[0] != 0xffffu; z += 32)
+                    if (chains[z] != 0) seed_q[s_base + s_step * (int)chains[z]] |= SKIP_BIT;
+                __syncwarp();
+                for (int s = 1; s < ns;) {
+                    int n_sid = 0;
+                    for (; s < ns && n_sid < K; ++s) {
+                        if (seed_q[s_base + s_step * s] & SKIP_BIT) {
+                            if (lane == 0) {
+                                res[(size_t)s * 3 + 2] = 0.0;
+                                chains[(size_t)s * md.gms] = 0xffffu;
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < K; ++q) sid[q] = q == n_sid ? s : sid[q];
+                            ++n_sid;
+                        }
+                    }
+                    if (n_sid > 1)
+                        walk_group(std::integral_constant<int, K>{}, sid, n_sid);
+                    else if (n_sid == 1)
+                        walk_group(std::integral_constant<int, 1>{}, sid, 1);
                 }
+                __syncwarp();
                 // flush: the run's records go, in seed order, to the warp's current arena
                 // chunk; a new chunk (one atomic) when it has no room
                 unsigned long long rbase = 0;

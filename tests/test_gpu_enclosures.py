@@ -110,3 +110,15 @@ def test_same_bits_batched_and_staged(engine, fp64_engine):
         g = engine.build_neighbor_graph(m)
         assert engine.form_pairwise_bundles(g, cvl.CurveletParams()) == \
             fp64_engine.form_pairwise_bundles(fp64_engine.build_neighbor_graph(m), cvl.CurveletParams())
+
+
+@pytest.mark.parametrize("gms", [2, 3, 4, 7, 16])
+@pytest.mark.parametrize("kind", ["band", "lattice", "lines"])
+def test_general_path_against_the_oracle(fp64_engine, oracle, kind, gms):
+    """k_growth, which leaves out the seeds of the first seed's chain: chains that fill up
+    (gms 3, 4) and that do not, runs of ties and of one seed."""
+    e = _map(kind)
+    r = fp64_engine.run(e, cvl.CurveletParams(group_max_sz=gms))
+    o = oracle.run(e, nthreads=4, group_max_sz=gms)
+    assert (r.num_curvelets, r.valid_pairs) == (o.num_curvelets, o.valid_pairs)
+    assert np.array_equal(r.chains, o.chains)
