@@ -148,12 +148,12 @@ struct cvl_engine {
     struct ContourBufs {
         DBuf chains_in, cnt, off, cursor, bucket, outdeg, indeg, child, parent, flags, hop, firsts,
             region, ctr, fsrc, fnf, fnb, isfrag, flen, fidx, idoff, loff, lpe, lce, lvotes, fragoff, fragids, err,
-            pstart, psize, pinfo, pcount, poff, pstart2, psize2, pinfo2;
+            pstart, psize, pfit, pcount, poff, pstart2, psize2, pinfo2;
         DBuf *all(int i) {
             DBuf *b[] = {&chains_in, &cnt, &off, &cursor, &bucket, &outdeg, &indeg, &child, &parent, &flags,
                          &hop, &firsts, &region, &ctr, &fsrc, &fnf, &fnb, &isfrag,
                          &flen, &fidx, &idoff, &loff, &lpe, &lce, &lvotes, &fragoff, &fragids, &err,
-                         &pstart, &psize, &pinfo, &pcount, &poff, &pstart2, &psize2, &pinfo2};
+                         &pstart, &psize, &pfit, &pcount, &poff, &pstart2, &psize2, &pinfo2};
             return i < (int)(sizeof(b) / sizeof(b[0])) ? b[i] : nullptr;
         }
     } cw;
@@ -2923,7 +2923,7 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
     CVL_TRY(e->alloc(w.firsts, sizeof(unsigned) * N));
     const unsigned long long region_cap = 3ull * N + 16;
     CVL_TRY(e->alloc(w.region, sizeof(int) * region_cap));
-    CVL_TRY(e->alloc(w.ctr, sizeof(unsigned long long) * 2));
+    CVL_TRY(e->alloc(w.ctr, sizeof(unsigned long long) * 3));  // start edges, region, polyarc queue
     CVL_TRY(e->alloc(w.fsrc, sizeof(unsigned long long) * N));
     CVL_TRY(e->alloc(w.fnf, sizeof(int) * N));
     CVL_TRY(e->alloc(w.fnb, sizeof(int) * N));
@@ -2937,7 +2937,7 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
 
     CVL_CUDA(cudaMemsetAsync(w.cnt.p, 0, sizeof(unsigned) * N, s));
     CVL_CUDA(cudaMemsetAsync(w.cursor.p, 0, sizeof(unsigned) * N, s));
-    CVL_CUDA(cudaMemsetAsync(w.ctr.p, 0, sizeof(unsigned long long) * 2, s));
+    CVL_CUDA(cudaMemsetAsync(w.ctr.p, 0, sizeof(unsigned long long) * 3, s));
     CVL_CUDA(cudaMemsetAsync(w.fnf.p, 0xff, sizeof(int) * N, s));  // -1: no fragment starts here
     CVL_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(unsigned) * 4, s));
     unsigned *err = (unsigned *)w.err.p;
@@ -3063,7 +3063,7 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
         const unsigned long long slots = h_ids - h_frags;  // at most N - 1 per fragment of N edges
         CVL_TRY(e->alloc(w.pstart, sizeof(long long) * std::max<unsigned long long>(slots, 1)));
         CVL_TRY(e->alloc(w.psize, sizeof(int) * std::max<unsigned long long>(slots, 1)));
-        CVL_TRY(e->alloc(w.pinfo, sizeof(double) * 12 * std::max<unsigned long long>(slots, 1)));
+        CVL_TRY(e->alloc(w.pfit, sizeof(double) * 3 * std::max<unsigned long long>(slots, 1)));
         CVL_TRY(e->alloc(w.pcount, sizeof(unsigned) * h_frags));
         CVL_TRY(e->alloc(w.poff, sizeof(unsigned long long) * (h_frags + 1)));
         PolyArgs pa;
@@ -3077,9 +3077,10 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
         pa.token_len = cp.token_len;
         pa.poly_start = (long long *)w.pstart.p;
         pa.poly_size = (int *)w.psize.p;
-        pa.poly_info = (double *)w.pinfo.p;
+        pa.poly_fit = (double *)w.pfit.p;
         pa.poly_count = (unsigned *)w.pcount.p;
-        const int pb = (int)std::max(1u, (h_frags + 3) / 4);
+        pa.queue = (unsigned *)((unsigned long long *)w.ctr.p + 2);
+        const int pb = (int)std::min<unsigned>((h_frags + 3) / 4, (unsigned)e->prop.multiProcessorCount * 4u);
         switch (pcpl) {
             case 1: k_polyarcs<1><<<pb, 128, 0, s>>>(pa); break;
             case 3: k_polyarcs<3><<<pb, 128, 0, s>>>(pa); break;
@@ -3096,10 +3097,10 @@ int contours_on_device(cvl_engine *e, const double *d_edges, int n, int sz, cons
         CVL_TRY(e->alloc(w.pstart2, sizeof(long long) * std::max<unsigned long long>(h_poly, 1)));
         CVL_TRY(e->alloc(w.psize2, sizeof(int) * std::max<unsigned long long>(h_poly, 1)));
         CVL_TRY(e->alloc(w.pinfo2, sizeof(double) * 12 * std::max<unsigned long long>(h_poly, 1)));
-        k_polyarcs_pack<<<(int)((h_frags + 255) / 256), 256, 0, s>>>(
-            (int)h_frags, (const long long *)w.fragoff.p, (const unsigned *)w.pcount.p,
-            (const unsigned long long *)w.poff.p, (const long long *)w.pstart.p, (const int *)w.psize.p,
-            (const double *)w.pinfo.p, (long long *)w.pstart2.p, (int *)w.psize2.p, (double *)w.pinfo2.p);
+        if (h_poly)
+            k_polyarcs_pack<<<(int)((h_poly + 127) / 128), 128, 0, s>>>(
+                pa, (long long)h_poly, (const unsigned long long *)w.poff.p, (long long *)w.pstart2.p,
+                (int *)w.psize2.p, (double *)w.pinfo2.p);
         CVL_TRY(check_launch("k_polyarcs_pack"));
         e->mark("polyarcs");
         std::vector<long long> st(h_poly);

@@ -15,9 +15,9 @@
 //     stays valid; the next polyarc starts at its last edge;
 //   - its best cell is the open cell of smallest rank (the rank table gives
 //     compute_best_fit's order: nearest the grid centre, first in row-major order);
-//   - the fit: a line or the circle through the start, middle and end edges, on
-//     lane 0, with the reference's operand order (the library builds with
-//     -fmad=false).
+//   - the fit: a line or the circle through the start, middle and end edges, with the
+//     reference's operand order (the library builds with -fmad=false), by a thread per
+//     polyarc where they are packed (k_polyarcs_pack).
 // compute_best_fit_according_to_curvelets runs at the end of every fragment over
 // all polyarcs so far, so a polyarc fitted as an arc with |k| < k_th becomes a
 // line at its next refit, keeping its centre, angle and length; every other fit
@@ -38,13 +38,20 @@ struct PolyArgs {
     double rad, token_len;         // compute_properties' R and token_len
     long long *poly_start;         // [slots]: index into frag_ids of the polyarc's first edge
     int *poly_size;                // [slots]
-    double *poly_info;             // [slots][12]
+    double *poly_fit;              // [slots][3]: the best cell's k_max, k_min, and the length along the edges
     unsigned *poly_count;          // [nfrags]
+    unsigned *queue;               // the next fragment (0 at start)
 };
 
 // The polyarc slots of fragment f start at frag_off[f] - f: a fragment of N edges
 // gives at most N - 1 polyarcs (each spans at least two edges and the next one
 // starts no earlier than the last edge of the one before).
+//
+// A persistent grid whose warps pull fragments from a queue: the cell tables (a rank is a
+// count over all cells) are made once per resident block, and a long fragment holds one
+// warp, not a block. With a block per 4 fragments the tables were a third of the
+// instructions. With the fits on lane 0 of the walking warp and a block per 4 fragments
+// a 242k-edge map's 19k fragments took 325 us, now 253 and 14 in the packing.
 template <int CPL>
 __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
     __shared__ double tab[4][4 * QMAX + 4];
@@ -68,7 +75,11 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
         cdx2[u] = on[u] ? cell_dx2[c] : 0.0;
         rk[u] = on[u] ? cell_rank[c] : 0xffffu;
     }
-    for (int f = blockIdx.x * 4 + wib; f < a.nfrags; f += gridDim.x * 4) {
+    for (;;) {
+        unsigned q = 0;
+        if (lane == 0) q = atomicAdd(a.queue, 1u);
+        const int f = (int)__shfl_sync(FULL, q, 0);
+        if (f >= a.nfrags) break;
         const int *ids = a.frag_ids + a.frag_off[f];
         const int N = (int)(a.frag_off[f + 1] - a.frag_off[f]);
         const long long slot0 = a.frag_off[f] - f;
@@ -199,59 +210,12 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
             const double kmax = __shfl_sync(FULL, mymax, src);
             const double kmin = __shfl_sync(FULL, mymin, src);
             if (lane == 0) {
-                const int size = j - iA + 1;
-                double k = (kmax + kmin) / 2;  // set_best_fit's _k
-                const double quality = 2 / (1.0 * a.rad / L + 1.0 * L / a.token_len / size);
-                // update_best_fit(middle, end) with _pt = the start edge
-                const double *P1 = a.edges + (size_t)ids[iA + size / 2] * a.sz;
-                const double *P2 = a.edges + (size_t)ids[j] * a.sz;
-                double theta, angle = 0.0, cx = 0.0, cy = 0.0;
-                bool arc = false;
-                if (fabs(k) < POLY_K_TH) {
-                    k = 0.0;
-                    theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
-                } else {
-                    const double d1 = ax * ax + ay * ay, d2 = P1[0] * P1[0] + P1[1] * P1[1],
-                                 d3 = P2[0] * P2[0] + P2[1] * P2[1];
-                    const double a11 = 2.0 * (ax - P1[0]), a12 = 2.0 * (ay - P1[1]), a21 = 2.0 * (P2[0] - P1[0]),
-                                 a22 = 2.0 * (P2[1] - P1[1]);
-                    const double b1 = d1 - d2, b2 = d3 - d2;
-                    const double det = a11 * a22 - a21 * a12;
-                    if (fabs(det) < POLY_K_TH) {
-                        k = 0.0;
-                        theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
-                    } else {
-                        cx = (b1 * a22 - b2 * a12) / det;
-                        cy = (b2 * a11 - b1 * a21) / det;
-                        const double v1x = ax - cx, v1y = ay - cy, v2x = P2[0] - cx, v2y = P2[1] - cy;
-                        const double c = v1x * v2y - v1y * v2x, d = v1x * v2x + v1y * v2y;
-                        angle = cvl_atan2(fabs(c), d);
-                        theta = cvl_atan2(c * v1x, -c * v1y);
-                        k = 1.0 / sqrt(v2x * v2x + v2y * v2y);
-                        arc = true;
-                    }
-                }
-                if (fabs(angle) > 0 && fabs(k) > POLY_K_TH && arc) L = angle / fabs(k);  // update_length
-                if (arc && fabs(k) < POLY_K_TH && f < a.nfrags - 1) {  // the refit of a later fragment
-                    k = 0.0;
-                    theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
-                }
                 const long long s = slot0 + count;
                 a.poly_start[s] = a.frag_off[f] + iA;
-                a.poly_size[s] = size;
-                double *row = a.poly_info + (size_t)s * 12;
-                row[0] = 1.0;   // forward
-                row[1] = kmax;  // _ref_pt after compute_best_fit: the best cell's k range
-                row[2] = kmin;
-                row[3] = T2;    // _ref_theta
-                row[4] = ax;    // _pt: the start edge
-                row[5] = ay;
-                row[6] = theta;
-                row[7] = k;
-                row[8] = L;
-                row[9] = quality;
-                row[10] = arc ? cx : 0.0;
-                row[11] = arc ? cy : 0.0;
+                a.poly_size[s] = j - iA + 1;
+                a.poly_fit[3 * s] = kmax;
+                a.poly_fit[3 * s + 1] = kmin;
+                a.poly_fit[3 * s + 2] = L;
             }
             ++count;
             i = j;
@@ -260,21 +224,78 @@ __global__ void __launch_bounds__(128) k_polyarcs(PolyArgs a) {
     }
 }
 
-// polyarcs of all fragments packed in order (fragment, then start)
-__global__ void k_polyarcs_pack(int nfrags, const long long *__restrict__ frag_off,
-                                const unsigned *__restrict__ poly_count, const unsigned long long *__restrict__ poly_off,
-                                const long long *__restrict__ start_in, const int *__restrict__ size_in,
-                                const double *__restrict__ info_in, long long *__restrict__ start_out,
-                                int *__restrict__ size_out, double *__restrict__ info_out) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nfrags) return;
-    const long long s0 = frag_off[f] - f;
-    const unsigned long long d0 = poly_off[f];
-    for (unsigned q = 0; q < poly_count[f]; ++q) {
-        start_out[d0 + q] = start_in[s0 + q];
-        size_out[d0 + q] = size_in[s0 + q];
-        for (int c = 0; c < 12; ++c) info_out[(d0 + q) * 12 + c] = info_in[(s0 + q) * 12 + c];
+// polyarcs of all fragments packed in order (fragment, then start), and their fits; a
+// thread per polyarc
+__global__ void __launch_bounds__(128) k_polyarcs_pack(PolyArgs a, long long n_poly,
+                                                       const unsigned long long *__restrict__ poly_off,
+                                                       long long *__restrict__ start_out, int *__restrict__ size_out,
+                                                       double *__restrict__ info_out) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= n_poly) return;
+    int f = 0;  // the last fragment with poly_off[f] <= p (it has polyarcs: the next one's are past p)
+    for (int lo = 0, hi = a.nfrags; hi - lo > 1;) {
+        const int mid = (lo + hi) >> 1;
+        if ((long long)poly_off[mid] <= p) lo = mid; else hi = mid;
+        f = lo;
     }
+    const long long s = a.frag_off[f] - f + (p - (long long)poly_off[f]);
+    const long long start = a.poly_start[s];
+    const int size = a.poly_size[s];
+    const double kmax = a.poly_fit[3 * s], kmin = a.poly_fit[3 * s + 1];
+    double L = a.poly_fit[3 * s + 2];
+    start_out[p] = start;
+    size_out[p] = size;
+    const int *ids = a.frag_ids + start;
+    const double *A = a.edges + (size_t)ids[0] * a.sz;
+    const double ax = A[0], ay = A[1], T2 = A[2];
+    double k = (kmax + kmin) / 2;  // set_best_fit's _k
+    const double quality = 2 / (1.0 * a.rad / L + 1.0 * L / a.token_len / size);
+    // update_best_fit(middle, end) with _pt = the start edge
+    const double *P1 = a.edges + (size_t)ids[size / 2] * a.sz;
+    const double *P2 = a.edges + (size_t)ids[size - 1] * a.sz;
+    double theta, angle = 0.0, cx = 0.0, cy = 0.0;
+    bool arc = false;
+    if (fabs(k) < POLY_K_TH) {
+        k = 0.0;
+        theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
+    } else {
+        const double d1 = ax * ax + ay * ay, d2 = P1[0] * P1[0] + P1[1] * P1[1], d3 = P2[0] * P2[0] + P2[1] * P2[1];
+        const double a11 = 2.0 * (ax - P1[0]), a12 = 2.0 * (ay - P1[1]), a21 = 2.0 * (P2[0] - P1[0]),
+                     a22 = 2.0 * (P2[1] - P1[1]);
+        const double b1 = d1 - d2, b2 = d3 - d2;
+        const double det = a11 * a22 - a21 * a12;
+        if (fabs(det) < POLY_K_TH) {
+            k = 0.0;
+            theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
+        } else {
+            cx = (b1 * a22 - b2 * a12) / det;
+            cy = (b2 * a11 - b1 * a21) / det;
+            const double v1x = ax - cx, v1y = ay - cy, v2x = P2[0] - cx, v2y = P2[1] - cy;
+            const double c = v1x * v2y - v1y * v2x, d = v1x * v2x + v1y * v2y;
+            angle = cvl_atan2(fabs(c), d);
+            theta = cvl_atan2(c * v1x, -c * v1y);
+            k = 1.0 / sqrt(v2x * v2x + v2y * v2y);
+            arc = true;
+        }
+    }
+    if (fabs(angle) > 0 && fabs(k) > POLY_K_TH && arc) L = angle / fabs(k);  // update_length
+    if (arc && fabs(k) < POLY_K_TH && f < a.nfrags - 1) {  // the refit of a later fragment
+        k = 0.0;
+        theta = cvl_atan2(P2[1] - ay, P2[0] - ax);
+    }
+    double *row = info_out + p * 12;
+    row[0] = 1.0;   // forward
+    row[1] = kmax;  // _ref_pt after compute_best_fit: the best cell's k range
+    row[2] = kmin;
+    row[3] = T2;    // _ref_theta
+    row[4] = ax;    // _pt: the start edge
+    row[5] = ay;
+    row[6] = theta;
+    row[7] = k;
+    row[8] = L;
+    row[9] = quality;
+    row[10] = arc ? cx : 0.0;
+    row[11] = arc ? cy : 0.0;
 }
 
 }  // namespace cvl
