@@ -74,6 +74,10 @@ constexpr int FAST_SLOTS = 16;
 constexpr int FAST_WARPS = 4;
 constexpr int FAST_BLOCKS = 5;
 constexpr int FAST_EXACT_BLOCKS = 3;
+// bundle slots of a k_curvelets_exact warp, as many as three blocks of an SM have room for (a
+// seed past them has its bundle made again at every visit: with 4 slots a 3.2M-edge run's
+// two kernels took 14.64 ms, with these 14.48; 16 or 24 in two blocks: 14.82)
+constexpr int FAST_WIDE_SLOTS = 14;
 constexpr int FAST_TILE = 4;     // consecutive anchors a queue-pulling warp takes at a time
 // e0 / max_k: larger leaves more comparisons undecided, smaller more columns to be made anew
 // (2^-13 to 2^-15 measured alike)
@@ -197,7 +201,7 @@ struct FastSmem {
     unsigned short list[2 * CAP];    // the first run's pairs, then the second's: k | flags
     unsigned char seed[2][CAP];      // list position of each run's seeds
 };
-struct FastWideSmem : FastSmem<FAST_WIDE, 4> {
+struct FastWideSmem : FastSmem<FAST_WIDE, FAST_WIDE_SLOTS> {
     unsigned cur[FAST_WIDE / 32], skip[FAST_WIDE / 32];
     unsigned mask[FAST_WIDE][FAST_WIDE / 32], meta[FAST_WIDE];  // accepted chains
 };
@@ -633,6 +637,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
                     const float slo = fmaf(tj.x, g1.x, tj.y * g1.y), shi = fmaf(tj.x, g2.x, tj.y * g2.y);
                     {
                         float emin = 1e30f, dlmin = 1e30f, dhmin = 1e30f;
+                        float pe = 0.0f, pl_ = 0.0f, ph = 0.0f, pw = 0.0f;  // of the cell before: two cells to a min
 #pragma unroll
                         for (int k = 0; k < FAST_P; ++k) {
                             const float e1 = fmaf(a.fm.d[k], t2, g0.z + a.fm.d2[k]);
@@ -641,10 +646,22 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
                             const float klo = (t2 + a.fm.c2[k]) * nre, khi = fmaf(nre, a.fm.ndx_4, klo);
                             const float tlo = slo * rcp_approx(dlo), thi = shi * rcp_approx(dhi);
                             const float n = min3(-klo, -tlo, a.fm.mk), M = min3(khi, thi, a.fm.mk);
-                            emin = fminf(emin, e1);
-                            dlmin = fminf(dlmin, fabsf(dlo));
-                            dhmin = fminf(dhmin, fabsf(dhi));
-                            wmax = fmaxf(wmax, n + M);
+                            if (k & 1) {
+                                emin = min3(emin, pe, e1);
+                                dlmin = min3(dlmin, fabsf(pl_), fabsf(dlo));
+                                dhmin = min3(dhmin, fabsf(ph), fabsf(dhi));
+                                wmax = max3(wmax, pw, n + M);
+                            } else if (k == FAST_P - 1) {
+                                emin = fminf(emin, e1);
+                                dlmin = fminf(dlmin, fabsf(dlo));
+                                dhmin = fminf(dhmin, fabsf(dhi));
+                                wmax = fmaxf(wmax, n + M);
+                            } else {
+                                pe = e1;
+                                pl_ = dlo;
+                                ph = dhi;
+                                pw = n + M;
+                            }
                             b[k] = make_float2(n, M);
                         }
                         bool bad = on && !(emin >= g0.w && dlmin >= (fabsf(slo) >= g2.w ? a.fm.dtiny : g1.w) &&
@@ -715,10 +732,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
                 // The walk of bundle c over seeds [r, r_end): each whose bundle meets c's in an open
                 // cell (:832-854) is taken, and c becomes the intersection; at most room.
                 auto walk = [&](float4 &c, unsigned &mask, int &room, int r, int r_end) {
-                    const float4 *src = slots + r * (SLOT_PITCH / 2);
-                    for (; r < r_end; ++r, src += SLOT_PITCH / 2) {
-                        float4 b;
-                        if (r < lim) b = *src; else b = load_far(r);
+                    auto step = [&](float4 b) {
                         b.x = fminf(c.x, b.x);
                         b.y = fminf(c.y, b.y);
                         b.z = fminf(c.z, b.z);
@@ -727,11 +741,17 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
                         if (__any_sync(FULL, w > h)) {
                             c = b;
                             mask |= 1u << r;
-                            if (--room == 0) break;
+                            --room;
                         } else {
                             undecided = fmaxf(undecided, w);
                         }
+                    };
+                    const float4 *src = slots + r * (SLOT_PITCH / 2);
+                    for (const int near = min(r_end, lim); r < near; ++r, src += SLOT_PITCH / 2) {
+                        step(*src);
+                        if (room == 0) return;
                     }
+                    for (; r < r_end && room > 0; ++r) step(load_far(r));
                 };
                 // a chain of more than two edges that no earlier seed of the run has (first-wins,
                 // :876-916): its best cell is the open one of least rank (:202-219)
@@ -856,7 +876,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelets_exact(const __grid_constant__ FastArgs a) {
     extern __shared__ __align__(16) unsigned char cv_smem[];
-    constexpr int SLOTS = 4;
+    constexpr int SLOTS = FAST_WIDE_SLOTS;
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (a.uncertified && (*a.uncertified & UNCERT_ANGLE)) return;
