@@ -681,9 +681,8 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const BinnedT<doubl
     a.err = (unsigned *)e->err.p;
     a.wide_cnt = (unsigned *)(work + 2) + 1;
     a.wide_list = (int *)e->ncand.p;
-    const long long warps = (long long)e->prop.multiProcessorCount * SEARCH_BLOCKS * SEARCH_WARPS;
-    a.split = 1;
-    while (a.split < 8 && (long long)(md.hash_mask + 1u) / 32 * a.split < warps) a.split *= 2;
+    a.buckets = (const unsigned *)e->deg.p;
+    a.bucket_cnt = (const unsigned *)(work + 4);
     return a;
 }
 // A window within the 3 x 3 hash blocks around its anchor's.
@@ -962,7 +961,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->out_off, sizeof(unsigned long long) * (n + 1)));
     CVL_TRY(e->alloc(e->stats, sizeof(MapStats) * M));
     CVL_TRY(e->alloc(e->err, sizeof(unsigned) * 4));
-    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 4));  // arena counter, -, work queues
+    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 5));  // arena, pairs, certification and wide anchors, queues, buckets
 
     BinnedT<R> B;
     B.x = (R *)e->bx.p;
@@ -988,7 +987,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * M, s));
     CVL_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(unsigned) * 4, s));
-    CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 4, s));
+    CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 5, s));
 
     // ---- (a) binning
     const int gb = short_grid(n, 256);
@@ -999,7 +998,8 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, (int *)e->pos_of.p,
-                                     F.e, F.cs2, F.at, nullptr);
+                                     F.e, F.cs2, F.at, pair_cap ? (unsigned *)e->deg.p : nullptr,
+                                     (unsigned *)((unsigned long long *)e->work.p + 4), nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
 
@@ -1008,8 +1008,8 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
             const int sms = e->prop.multiProcessorCount;
             // a persistent grid; short blocks where others' work is to be let in
             const SearchArgs sa = search_args(e, md, B, F, n, M, pair_cap);
-            int blocks = short_grid((long long)T * sa.split, SEARCH_WARPS * 32);
-            if (!e->yield_fn) blocks = std::min(blocks, sms * SEARCH_BLOCKS);
+            int blocks = short_grid(std::min<long long>(n, T), SEARCH_WARPS * 4);
+            if (!e->yield_fn) blocks = std::min(short_grid(std::min<long long>(n, T), SEARCH_WARPS), sms * SEARCH_BLOCKS);
             CVL_TRY(launch_search(e, sa, blocks, sms * 4));
             e->mark("neighbors");
             ro.stats.assign(M, MapStats{});
@@ -1314,7 +1314,7 @@ std::vector<WsItem> workspace_plan(const cvl_tuning *tune, unsigned long long ar
     add(&E::out_off, 8 * (n + 1));
     add(&E::stats, sizeof(MapStats) * M);
     add(&E::err, 16);
-    add(&E::work, 32);
+    add(&E::work, 40);
     add(&E::scan_tmp, (T / SCAN_TILE + 64) * 4 * sizeof(unsigned long long) + 4096);  // the largest scan: T
     add(&E::chunk_start, 4 * (4096 + 1));
     // pair-sized (after the count)
@@ -1475,7 +1475,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             const std::pair<void *, size_t> zero[] = {{e->bcount.p, sizeof(unsigned) * (T + 1)},
                                                       {e->stats.p, sizeof(MapStats) * cap.M},
                                                       {e->err.p, 16},
-                                                      {e->work.p, 32},
+                                                      {e->work.p, 40},
                                                       {e->count.p, sizeof(unsigned) * (size_t)N},
                                                       {e->chunk_start.p, fm.ok ? 0 : sizeof(int) * (cap.K + 1)}};
             for (int r = 0; r < 6; ++r) {
@@ -1492,7 +1492,9 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
-                                             (int *)e->pos_of.p, F.e, F.cs2, F.at, dd);
+                                             (int *)e->pos_of.p, F.e, F.cs2, F.at,
+                                             fm.ok ? (unsigned *)e->deg.p : nullptr,
+                                             (unsigned *)((unsigned long long *)e->work.p + 4), dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;
@@ -1510,7 +1512,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             if (fm.ok) {
                 SearchArgs sa = search_args(e, md, B, F, N, cap.M, (unsigned long long)sh.num_pairs);
                 sa.dims = dd;
-                CVL_TRY(launch_search(e, sa, std::min(short_grid((long long)T * sa.split, SEARCH_WARPS * 32), sms * SEARCH_BLOCKS), sms));
+                CVL_TRY(launch_search(e, sa, std::min(short_grid(std::min<long long>(N, T), SEARCH_WARPS), sms * SEARCH_BLOCKS), sms));
             } else {
                 k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
                 CVL_TRY(check_launch("k_nb<COUNT>"));

@@ -294,14 +294,17 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
                               int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
-                              int4 *__restrict__ at, const RunDims *__restrict__ dims) {
+                              int4 *__restrict__ at, unsigned *__restrict__ buckets, unsigned *__restrict__ bucket_cnt,
+                              const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
         M = dims->M;
     }
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
         const unsigned h = ehash[e];
-        const unsigned pos = bstart[h] + atomicSub(&bcount[h], 1u) - 1u;  // (the counts are not needed any more)
+        const unsigned left = atomicSub(&bcount[h], 1u);  // (the counts are not needed any more)
+        const unsigned pos = bstart[h] + left - 1u;
+        if (buckets && left == 1u) buckets[atomicAdd(bucket_cnt, 1u)] = h;  // each bucket that holds edges, once
         const T x = edges[(size_t)e * sz + 0];
         const T y = edges[(size_t)e * sz + 1];
         const T th = edges[(size_t)e * sz + 2];
