@@ -162,7 +162,7 @@ struct FastBinned {
 struct FastArgs {
     Model md;
     FastModel fm;
-    BinnedT<double> B;
+    EdgeRecords B;
     FastBinned F;
     int a_begin, a_end;
     const unsigned long long *row;      // [N] the anchors' rows (pack_row)
@@ -233,7 +233,7 @@ __device__ __forceinline__ CellAnchor cell_anchor(const Model &md, double T2, in
     sincos(c.T2t, &c.sT, &c.cT);
     return c;
 }
-__device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double> &B, double2 cs2, int i, int nn,
+__device__ __forceinline__ void exact_cell(const Model &md, const EdgeRecords &B, double2 cs2, int i, int nn,
                                            const CellAnchor &c, double &m, double &M) {
     const PairGeom g = pair_geom(md, B.x[i], B.y[i], cs2.x, cs2.y, B.x[nn], B.y[nn], B.sp[nn], B.cp[nn], B.sm[nn],
                                  B.cm[nn]);
@@ -247,7 +247,7 @@ __device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double
     const double tt = c.sT * g.DX - c.cT * g.DY;  // :705
     bundle_cell_fp64<QUOT_DIVIDE>(md, c.d, 2.0 * c.d, c.d * c.d, transport_column(md, g, tt, s_m, s_p), m, M);
 }
-__device__ __forceinline__ void exact_cell(const Model &md, const BinnedT<double> &B, double2 cs2, int i, int nn,
+__device__ __forceinline__ void exact_cell(const Model &md, const EdgeRecords &B, double2 cs2, int i, int nn,
                                            int cell, double &m, double &M) {
     exact_cell(md, B, cs2, i, nn, cell_anchor(md, B.th[i], cell), m, M);
 }
@@ -1048,7 +1048,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
 // ---------------------------------------------------------------------------
 struct FinalArgs {
     Model md;
-    BinnedT<double> B;
+    EdgeRecords B;
     const double2 *cs2;
     const int *pos_of;  // input index -> internal
     int N, M;

@@ -659,8 +659,42 @@ inline FastBinned fast_binned(const cvl_engine *e, size_t n) {
     F.at = (int4 *)(F.cs2 + n);
     return F;
 }
+// The edges' records, in the buffer of the record arena's bounds, which k_curvelets does not
+// use: 64 bytes an edge of its 80. (A run that turns out to need the bundle path sizes and
+// writes that buffer only after it has binned its edges into arrays.)
+inline EdgeRecords edge_records(const cvl_engine *e, const FastBinned &F) {
+    double *r = (double *)e->rec_k.p;
+    EdgeRecords B;
+    B.x = {r};
+    B.y = {r + 1};
+    B.th = {r + 2};
+    B.sp = {r + 3};
+    B.cp = {r + 4};
+    B.sm = {r + 5};
+    B.cm = {r + 6};
+    B.e = F.e;
+    B.at = F.at;
+    B.map = {(const int *)F.at + 3};
+    B.orig = (int *)e->orig_of.p;
+    return B;
+}
+template <typename R>
+BinnedT<R> binned_arrays(const cvl_engine *e) {
+    BinnedT<R> B;
+    B.x = (R *)e->bx.p;
+    B.y = (R *)e->by.p;
+    B.th = (R *)e->bth.p;
+    B.sp = (R *)e->bsp.p;
+    B.cp = (R *)e->bcp.p;
+    B.sm = (R *)e->bsm.p;
+    B.cm = (R *)e->bcm.p;
+    B.cell = (int2 *)e->bcell.p;
+    B.orig = (int *)e->orig_of.p;
+    B.map = (int *)e->bmap.p;
+    return B;
+}
 // The one-pass search: pairs into csr_ids / pcls (pair_cap of them), rows into fast_rows.
-SearchArgs search_args(const cvl_engine *e, const Model &md, const BinnedT<double> &B, const FastBinned &F, int n, int M,
+SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &B, const FastBinned &F, int n, int M,
                        unsigned long long pair_cap) {
     SearchArgs a{};
     unsigned long long *work = (unsigned long long *)e->work.p;
@@ -720,7 +754,7 @@ int launch_curvelets(cvl_engine *e, const FastArgs &a, int blocks, int exact_blo
     return check_launch("k_curvelets_exact");
 }
 
-FinalArgs final_args(const cvl_engine *e, const Model &md, const FastModel &fm, const BinnedT<double> &B, const FastBinned &F, int n, int M,
+FinalArgs final_args(const cvl_engine *e, const Model &md, const FastModel &fm, const EdgeRecords &B, const FastBinned &F, int n, int M,
                      const int *d_map_off, unsigned long long out_cap) {
     FinalArgs f{};
     f.md = md;
@@ -776,7 +810,7 @@ void fast_totals(RunOut &ro) {
 // (c) + (d) + (e) of a direct run by k_curvelets and k_finalize_exact; a run with a yield
 // hook goes chunk by chunk of anchors (about chunk_pairs pairs at 16 per edge), on short blocks.
 // CVL_EAGAIN: the pairs did not fit, or an orientation is outside the enclosures' range.
-int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, const BinnedT<double> &B, const Model &md,
+int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, const EdgeRecords &B, const Model &md,
                     int n, int M, const int *d_map_off, const std::vector<int32_t> &map_off_host, int mode,
                     const cvl_tuning &tn, bool two_pass, RunOut &ro) {
     cudaStream_t s = e->stream;
@@ -942,16 +976,19 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->bcount, sizeof(unsigned) * (T + 1)));
     CVL_TRY(e->alloc(e->bstart, sizeof(unsigned) * (T + 1)));
     CVL_TRY(e->alloc(e->pos_of, sizeof(int) * n));
-    CVL_TRY(e->alloc(e->bx, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->by, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bth, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bsp, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bcp, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bsm, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bcm, sizeof(R) * n));
-    CVL_TRY(e->alloc(e->bcell, sizeof(int2) * n));
+    if (fm.ok) CVL_TRY(e->alloc(e->rec_k, sizeof(double) * EDGE_RECORD * n));
+    if (!pair_cap) {  // the search's arrays
+        CVL_TRY(e->alloc(e->bx, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->by, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bth, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bsp, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bcp, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bsm, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bcm, sizeof(R) * n));
+        CVL_TRY(e->alloc(e->bcell, sizeof(int2) * n));
+        CVL_TRY(e->alloc(e->bmap, sizeof(int) * n));
+    }
     CVL_TRY(e->alloc(e->orig_of, sizeof(int) * n));
-    CVL_TRY(e->alloc(e->bmap, sizeof(int) * n));
     CVL_TRY(e->alloc(e->ncand, sizeof(unsigned) * n));
     CVL_TRY(e->alloc(e->deg, sizeof(unsigned) * n));
     CVL_TRY(e->alloc(e->pair_off, sizeof(unsigned long long) * (n + 1)));
@@ -963,17 +1000,6 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->err, sizeof(unsigned) * 4));
     CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 5));  // arena, pairs, certification and wide anchors, queues, buckets
 
-    BinnedT<R> B;
-    B.x = (R *)e->bx.p;
-    B.y = (R *)e->by.p;
-    B.th = (R *)e->bth.p;
-    B.sp = (R *)e->bsp.p;
-    B.cp = (R *)e->bcp.p;
-    B.sm = (R *)e->bsm.p;
-    B.cm = (R *)e->bcm.p;
-    B.cell = (int2 *)e->bcell.p;
-    B.orig = (int *)e->orig_of.p;
-    B.map = (int *)e->bmap.p;
     unsigned *err = (unsigned *)e->err.p;
     MapStats *stats = (MapStats *)e->stats.p;
     unsigned long long *arena_ctr = (unsigned long long *)e->work.p;
@@ -983,6 +1009,14 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         CVL_TRY(e->alloc(e->atrig, sizeof(R) * (size_t)n * (2 * md.Q + 2)));
         F = fast_binned(e, (size_t)n);
     }
+    BinnedT<R> B = binned_arrays<R>(e);
+    EdgeRecords FB{};
+    double2 *rec_out = nullptr;
+    if (fm.ok) {
+        FB = edge_records(e, F);
+        rec_out = (double2 *)e->rec_k.p;
+    }
+    if (pair_cap) B.x = nullptr;  // no arrays
 
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * M, s));
@@ -997,7 +1031,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(check_launch("k_bin_keys"));
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
-                                     (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, (int *)e->pos_of.p,
+                                     (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, rec_out, (int *)e->pos_of.p,
                                      F.e, F.cs2, F.at, pair_cap ? (unsigned *)e->deg.p : nullptr,
                                      (unsigned *)((unsigned long long *)e->work.p + 4), nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
@@ -1007,13 +1041,13 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         if (pair_cap) {
             const int sms = e->prop.multiProcessorCount;
             // a persistent grid; short blocks where others' work is to be let in
-            const SearchArgs sa = search_args(e, md, B, F, n, M, pair_cap);
+            const SearchArgs sa = search_args(e, md, FB, F, n, M, pair_cap);
             int blocks = short_grid(std::min<long long>(n, T), SEARCH_WARPS * 4);
             if (!e->yield_fn) blocks = std::min(short_grid(std::min<long long>(n, T), SEARCH_WARPS), sms * SEARCH_BLOCKS);
             CVL_TRY(launch_search(e, sa, blocks, sms * 4));
             e->mark("neighbors");
             ro.stats.assign(M, MapStats{});
-            const int rc = run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, false, ro);
+            const int rc = run_fast_chunks(e, fm, F, FB, md, n, M, d_map_off, map_off_host, mode, tn, false, ro);
             if (rc != CVL_EAGAIN) return rc;
             // the two passes, or once more with the pairs' own count of room
             unsigned long long need = 0;
@@ -1106,7 +1140,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
 
     if constexpr (std::is_same<R, double>::value) {
         if (fast)
-            return run_fast_chunks(e, fm, F, B, md, n, M, d_map_off, map_off_host, mode, tn, true, ro);
+            return run_fast_chunks(e, fm, F, FB, md, n, M, d_map_off, map_off_host, mode, tn, true, ro);
     }
 
     // ---- (c) + (d) per chunk
@@ -1398,12 +1432,15 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     if (fm.ok) md.sbits = SEARCH_SBITS;
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
         if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off || w.buf == &cvl_engine::bfill) continue;
-        // k_curvelets keeps no bundles, pair flags or numbers in memory
-        if (fm.ok && (w.buf == &cvl_engine::bund || w.buf == &cvl_engine::pflag || w.buf == &cvl_engine::pair_anchor ||
-                      w.buf == &cvl_engine::rec_k))
-            continue;
+        // k_curvelets keeps no bundles, pair flags or numbers in memory, its edges in records
+        const DBuf cvl_engine::*unused[] = {
+            &cvl_engine::bund, &cvl_engine::pflag, &cvl_engine::pair_anchor, &cvl_engine::rec_k, &cvl_engine::bx,
+            &cvl_engine::by, &cvl_engine::bth, &cvl_engine::bsp, &cvl_engine::bcp, &cvl_engine::bsm, &cvl_engine::bcm,
+            &cvl_engine::bcell, &cvl_engine::bmap};
+        if (fm.ok && std::find(std::begin(unused), std::end(unused), w.buf) != std::end(unused)) continue;
         CVL_TRY(e->alloc(e->*(w.buf), w.bytes));
     }
+    if (fm.ok) CVL_TRY(e->alloc(e->rec_k, sizeof(double) * EDGE_RECORD * (size_t)cap.N));
     CVL_TRY(e->alloc(e->gdims, sizeof(RunDims)));
     CVL_TRY(e->alloc(e->gchunks, sizeof(ChunkDims) * (size_t)cap.K));
     if (!e->gread_host) {
@@ -1448,17 +1485,6 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
         CVL_CUDA(cudaFuncSetAttribute(k_nb<double, NB_COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb_smem));
         CVL_CUDA(cudaFuncSetAttribute(k_nb<double, NB_FILL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nb_smem));
         const size_t gsmem = (size_t)(GROWTH_THREADS / 32) * growth_smem_per_warp(md.max_cand, md.gms);
-        BinnedT<double> B;
-        B.x = (double *)e->bx.p;
-        B.y = (double *)e->by.p;
-        B.th = (double *)e->bth.p;
-        B.sp = (double *)e->bsp.p;
-        B.cp = (double *)e->bcp.p;
-        B.sm = (double *)e->bsm.p;
-        B.cm = (double *)e->bcm.p;
-        B.cell = (int2 *)e->bcell.p;
-        B.orig = (int *)e->orig_of.p;
-        B.map = (int *)e->bmap.p;
         unsigned *err = (unsigned *)e->err.p;
         MapStats *stats = (MapStats *)e->stats.p;
         unsigned long long *arena_ctr = (unsigned long long *)e->work.p;
@@ -1467,6 +1493,12 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
         const int sms = e->prop.multiProcessorCount;
         const int N = cap.N;
         const FastBinned F = fm.ok ? fast_binned(e, (size_t)N) : FastBinned{};
+        BinnedT<double> B = binned_arrays<double>(e);
+        EdgeRecords FB{};
+        if (fm.ok) {
+            FB = edge_records(e, F);
+            B.x = nullptr;  // no arrays
+        }
         CVL_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         auto enqueue = [&]() -> int {
             GraphBegin gbeg{};
@@ -1492,7 +1524,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
-                                             (int *)e->pos_of.p, F.e, F.cs2, F.at,
+                                             fm.ok ? (double2 *)e->rec_k.p : nullptr, (int *)e->pos_of.p, F.e, F.cs2, F.at,
                                              fm.ok ? (unsigned *)e->deg.p : nullptr,
                                              (unsigned *)((unsigned long long *)e->work.p + 4), dd);
             CVL_TRY(check_launch("k_bin_scatter"));
@@ -1510,7 +1542,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             na.pair_cap = (unsigned long long)sh.num_pairs;
             const int gn = std::min(short_grid(N, (long long)nb_wpb * 4), sms * 8);
             if (fm.ok) {
-                SearchArgs sa = search_args(e, md, B, F, N, cap.M, (unsigned long long)sh.num_pairs);
+                SearchArgs sa = search_args(e, md, FB, F, N, cap.M, (unsigned long long)sh.num_pairs);
                 sa.dims = dd;
                 CVL_TRY(launch_search(e, sa, std::min(short_grid(std::min<long long>(N, T), SEARCH_WARPS), sms * SEARCH_BLOCKS), sms));
             } else {
@@ -1551,7 +1583,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 FastArgs fa{};
                 fa.md = md;
                 fa.fm = fm;
-                fa.B = B;
+                fa.B = FB;
                 fa.F = F;
                 fa.row = (const unsigned long long *)e->pair_off.p;
                 fa.csr_ids = (const int *)e->csr_ids.p;
@@ -1629,7 +1661,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->count.p, N,
                                                         (unsigned long long *)e->out_off.p)));
             if (fm.ok) {
-                FinalArgs f = final_args(e, md, fm, B, F, N, cap.M, d_map_off, C_cap);
+                FinalArgs f = final_args(e, md, fm, FB, F, N, cap.M, d_map_off, C_cap);
                 f.dims = dd;
                 CVL_TRY(launch_finalize(e, f, N));
             } else {

@@ -104,6 +104,37 @@ struct __align__(16) FastEdge {
     float cm, sm, cp, sp;
 };
 
+// A field of records of STRIDE scalars.
+template <typename V, int STRIDE>
+struct RecordField {
+    V *p;
+    __device__ __forceinline__ V &operator[](int i) const { return p[(size_t)i * STRIDE]; }
+};
+// The edges as k_search, k_curvelets_exact and k_finalize_exact read them: those gather an
+// edge's fields at random, so they lie in one record of two whole sectors (in an array per
+// field, as k_nb and k_bundles read them, the scatter wrote ten places an edge and a gather
+// touched six sectors: binning of a 3.65M-edge map 0.80 -> 0.47 ms, its finalize 1.95 -> 1.81).
+constexpr int EDGE_RECORD = 8;
+struct EdgeRecords {
+    RecordField<double, EDGE_RECORD> x, y, th, sp, cp, sm, cm;
+    const FastEdge *e;
+    const int4 *at;  // pixel cell, input index, map
+    RecordField<const int, 4> map;
+    int *orig;
+};
+template <typename T>
+__device__ __forceinline__ int4 edge_place(const BinnedT<T> &B, int j) {
+    const int2 c = B.cell[j];
+    return make_int4(c.x, c.y, 0, B.map[j]);
+}
+__device__ __forceinline__ int4 edge_place(const EdgeRecords &B, int j) { return B.at[j]; }
+__device__ __forceinline__ double edge_x(const EdgeRecords &B, int j) { return B.e[j].x; }
+__device__ __forceinline__ double edge_y(const EdgeRecords &B, int j) { return B.e[j].y; }
+template <typename T>
+__device__ __forceinline__ T edge_x(const BinnedT<T> &B, int j) { return B.x[j]; }
+template <typename T>
+__device__ __forceinline__ T edge_y(const BinnedT<T> &B, int j) { return B.y[j]; }
+
 // The sizes of a run that a captured graph replays (one graph per size bucket
 // serves every run within the bucket): the kernels launched for the bucket's
 // capacity read the run's own sizes from device memory at their start. nullptr
@@ -293,7 +324,7 @@ template <typename T>
 __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const int *__restrict__ map_off,
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
-                              int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
+                              double2 *__restrict__ rec, int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
                               int4 *__restrict__ at, unsigned *__restrict__ buckets, unsigned *__restrict__ bucket_cnt,
                               const RunDims *__restrict__ dims) {
     if (dims) {
@@ -308,9 +339,6 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
         const T x = edges[(size_t)e * sz + 0];
         const T y = edges[(size_t)e * sz + 1];
         const T th = edges[(size_t)e * sz + 2];
-        B.x[pos] = x;
-        B.y[pos] = y;
-        B.th[pos] = th;
         // T0 +- dt and their sin/cos (cpu_curvelet.hpp:655-656, 730-733), once per edge
         const T t_p = th + md.dt;
         const T t_m = th - md.dt;
@@ -318,21 +346,33 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
         T sp, cp, sm, cm;
         sincos(t_p, &sp, &cp);
         sincos(t_m, &sm, &cm);
-        B.sp[pos] = sp;
-        B.cp[pos] = cp;
-        B.sm[pos] = sm;
-        B.cm[pos] = cm;
+        if (rec) {
+            double2 *r = rec + (size_t)pos * (EDGE_RECORD / 2);
+            r[0] = make_double2((double)x, (double)y);
+            r[1] = make_double2((double)th, (double)sp);
+            r[2] = make_double2((double)cp, (double)sm);
+            r[3] = make_double2((double)cm, 0.0);
+        }
+        const int2 cell = make_int2(lrint_dev(x), lrint_dev(y));
+        const int m = map_of(map_off, M, e);
+        if (B.x) {
+            B.x[pos] = x;
+            B.y[pos] = y;
+            B.th[pos] = th;
+            B.sp[pos] = sp;
+            B.cp[pos] = cp;
+            B.sm[pos] = sm;
+            B.cm[pos] = cm;
+            B.cell[pos] = cell;
+            B.map[pos] = m;
+        }
         if (fe) {
             fe[pos] = FastEdge{(double)x, (double)y, (float)cm, (float)sm, (float)cp, (float)sp};
             double s2, c2;
             sincos((double)th, &s2, &c2);
             cs2[pos] = make_double2(c2, s2);
         }
-        const int2 cell = make_int2(lrint_dev(x), lrint_dev(y));
-        const int m = map_of(map_off, M, e);
-        B.cell[pos] = cell;
         B.orig[pos] = e;
-        B.map[pos] = m;
         if (fe) at[pos] = make_int4(cell.x, cell.y, e, m);
         pos_of[e] = (int)pos;
     }
@@ -369,8 +409,8 @@ __host__ __device__ inline size_t nbr_smem_per_warp(int max_cand) {
 // reference predicate. The window's bucket ranges (up to 32 per round) are
 // loaded by the lanes at once; entries are enumerated over their prefix sums.
 // WANT_KEY: compute the scan key (a counting pass needs none).
-template <bool WANT_KEY = true, typename T, typename F>
-__device__ __forceinline__ void for_window_candidates(const ModelT<T> &md, const BinnedT<T> &B, const unsigned *bstart,
+template <bool WANT_KEY = true, typename T, typename BIN, typename F>
+__device__ __forceinline__ void for_window_candidates(const ModelT<T> &md, const BIN &B, const unsigned *bstart,
                                                       int i, int m, int2 ac, T ax, T ay, int lane, F &&f) {
     const int bx0 = (ac.x - md.w) >> md.sbits, bx1 = (ac.x + md.w) >> md.sbits;
     const int by0 = (ac.y - md.w) >> md.sbits, by1 = (ac.y + md.w) >> md.sbits;
@@ -412,14 +452,14 @@ __device__ __forceinline__ void for_window_candidates(const ModelT<T> &md, const
             unsigned long long key = 0;
             const int j = (int)(sb + (e - pre));
             if (e < total && j != i) {
-                const int2 cc = B.cell[j];
+                const int4 cc = edge_place(B, j);
                 // the entry's own block must be the visited one (a bucket can hold
                 // several blocks, and two window blocks can share a bucket)
-                if (B.map[j] == m && (cc.x >> md.sbits) == vbx && (cc.y >> md.sbits) == vby &&
+                if (cc.w == m && (cc.x >> md.sbits) == vbx && (cc.y >> md.sbits) == vby &&
                     abs(cc.x - ac.x) <= md.w && abs(cc.y - ac.y) <= md.w) {
-                    d2 = sq_dist(ax, ay, B.x[j], B.y[j]);  // sq_dist(te, ne), preprocess.hpp:160
+                    d2 = sq_dist(ax, ay, edge_x(B, j), edge_y(B, j));  // sq_dist(te, ne), preprocess.hpp:160
                     ok = !(d2 > md.rad_sqr);               // preprocess.hpp:161-163
-                    if (WANT_KEY) key = scan_key(cc, ac.x, ac.y, md.w, B.orig[j]);
+                    if (WANT_KEY) key = scan_key(make_int2(cc.x, cc.y), ac.x, ac.y, md.w, B.orig[j]);
                 }
             }
             f(ok, j, d2, key);
@@ -430,8 +470,8 @@ __device__ __forceinline__ void for_window_candidates(const ModelT<T> &md, const
 // Truncation (preprocess.hpp:165-167): keep the first max_cand candidates in
 // window-scan order. Walks the window pixel cell by pixel cell; inside the cell
 // where the cap is crossed keeps the lowest edge indices. Returns the count kept.
-template <typename T>
-__device__ __noinline__ unsigned gather_truncated(const ModelT<T> &md, const BinnedT<T> &B, const unsigned *bstart,
+template <typename T, typename BIN>
+__device__ __noinline__ unsigned gather_truncated(const ModelT<T> &md, const BIN &B, const unsigned *bstart,
                                                   int i, int m, int2 ac, T ax, T ay, int lane, NbrSmemT<T> S,
                                                   unsigned *err) {
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -448,8 +488,9 @@ __device__ __noinline__ unsigned gather_truncated(const ModelT<T> &md, const Bin
             const int j = base + lane;
             bool ok = false;
             if (j < b1 && j != i) {
-                const int2 cc = B.cell[j];
-                ok = B.map[j] == m && cc.x == px && cc.y == py && !(sq_dist(ax, ay, B.x[j], B.y[j]) > md.rad_sqr);
+                const int4 cc = edge_place(B, j);
+                ok = cc.w == m && cc.x == px && cc.y == py &&
+                     !(sq_dist(ax, ay, edge_x(B, j), edge_y(B, j)) > md.rad_sqr);
             }
             c += __popc(__ballot_sync(FULL, ok));
         }
@@ -460,9 +501,9 @@ __device__ __noinline__ unsigned gather_truncated(const ModelT<T> &md, const Bin
             T d2 = 0;
             int oj = 0;
             if (j < b1 && j != i) {
-                const int2 cc = B.cell[j];
-                if (B.map[j] == m && cc.x == px && cc.y == py) {
-                    d2 = sq_dist(ax, ay, B.x[j], B.y[j]);
+                const int4 cc = edge_place(B, j);
+                if (cc.w == m && cc.x == px && cc.y == py) {
+                    d2 = sq_dist(ax, ay, edge_x(B, j), edge_y(B, j));
                     ok = !(d2 > md.rad_sqr);
                     oj = B.orig[j];
                 }
@@ -472,9 +513,9 @@ __device__ __noinline__ unsigned gather_truncated(const ModelT<T> &md, const Bin
                 unsigned rk = 0;
                 for (int k = b0; k < b1; ++k) {
                     if (k == i) continue;
-                    const int2 ck = B.cell[k];
-                    if (B.map[k] == m && ck.x == px && ck.y == py && B.orig[k] < oj &&
-                        !(sq_dist(ax, ay, B.x[k], B.y[k]) > md.rad_sqr))
+                    const int4 ck = edge_place(B, k);
+                    if (ck.w == m && ck.x == px && ck.y == py && B.orig[k] < oj &&
+                        !(sq_dist(ax, ay, edge_x(B, k), edge_y(B, k)) > md.rad_sqr))
                         ++rk;
                 }
                 ok = rk < need;

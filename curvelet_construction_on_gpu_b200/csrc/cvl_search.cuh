@@ -43,7 +43,7 @@ constexpr unsigned long long NO_ROW = ~0ull;  // no room was left for the row (E
 
 struct SearchArgs {
     Model md;
-    BinnedT<double> B;
+    EdgeRecords B;
     const FastEdge *e;                // [N]
     const double2 *cs2;               // [N]
     const int4 *at;                   // [N] pixel cell, input index, map
@@ -291,8 +291,9 @@ __global__ void __launch_bounds__(256) k_search_wide(const __grid_constant__ Sea
     SearchCounts counts;
     for (int it = (int)blockIdx.x * 8 + wib; it < n_wide; it += (int)gridDim.x * 8) {
         const int i = a.wide_list[it];
-        const int m = a.B.map[i];
-        const int2 ac = a.B.cell[i];
+        const int4 at = a.at[i];
+        const int m = at.w;
+        const int2 ac = make_int2(at.x, at.y);
         const double ax = a.e[i].x, ay = a.e[i].y;
         unsigned n = 0;
         __syncwarp();
