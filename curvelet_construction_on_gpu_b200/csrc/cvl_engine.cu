@@ -715,8 +715,11 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &
     a.err = (unsigned *)e->err.p;
     a.wide_cnt = (unsigned *)(work + 2) + 1;
     a.wide_list = (int *)e->ncand.p;
-    a.buckets = (const unsigned *)e->deg.p;
-    a.bucket_cnt = (const unsigned *)(work + 4);
+    a.items = (const unsigned *)e->deg.p;
+    a.item_cnt = (const unsigned *)(work + 4);
+    a.queue = (unsigned *)(work + 4) + 1;
+    a.item_size = search_item(n);
+    a.pulls = ~0u;
     return a;
 }
 // A window within the 3 x 3 hash blocks around its anchor's.
@@ -1033,7 +1036,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, rec_out, (int *)e->pos_of.p,
                                      F.e, F.cs2, F.at, pair_cap ? (unsigned *)e->deg.p : nullptr,
-                                     (unsigned *)((unsigned long long *)e->work.p + 4), nullptr);
+                                     (unsigned *)((unsigned long long *)e->work.p + 4), search_item(n), nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
 
@@ -1041,9 +1044,13 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         if (pair_cap) {
             const int sms = e->prop.multiProcessorCount;
             // a persistent grid; short blocks where others' work is to be let in
-            const SearchArgs sa = search_args(e, md, FB, F, n, M, pair_cap);
-            int blocks = short_grid(std::min<long long>(n, T), SEARCH_WARPS * 4);
-            if (!e->yield_fn) blocks = std::min(short_grid(std::min<long long>(n, T), SEARCH_WARPS), sms * SEARCH_BLOCKS);
+            SearchArgs sa = search_args(e, md, FB, F, n, M, pair_cap);
+            const long long items = std::min<long long>(n, (long long)T + n / search_item(n));  // at most
+            int blocks = std::min(short_grid(items, SEARCH_WARPS), sms * SEARCH_BLOCKS);
+            if (e->yield_fn) {
+                sa.pulls = 4;
+                blocks = short_grid(items, SEARCH_WARPS * sa.pulls);
+            }
             CVL_TRY(launch_search(e, sa, blocks, sms * 4));
             e->mark("neighbors");
             ro.stats.assign(M, MapStats{});
@@ -1526,7 +1533,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
                                              fm.ok ? (double2 *)e->rec_k.p : nullptr, (int *)e->pos_of.p, F.e, F.cs2, F.at,
                                              fm.ok ? (unsigned *)e->deg.p : nullptr,
-                                             (unsigned *)((unsigned long long *)e->work.p + 4), dd);
+                                             (unsigned *)((unsigned long long *)e->work.p + 4), search_item(N), dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;
@@ -1544,7 +1551,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             if (fm.ok) {
                 SearchArgs sa = search_args(e, md, FB, F, N, cap.M, (unsigned long long)sh.num_pairs);
                 sa.dims = dd;
-                CVL_TRY(launch_search(e, sa, std::min(short_grid(std::min<long long>(N, T), SEARCH_WARPS), sms * SEARCH_BLOCKS), sms));
+                CVL_TRY(launch_search(e, sa, std::min(short_grid(N, SEARCH_WARPS), sms * SEARCH_BLOCKS), sms));
             } else {
                 k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
                 CVL_TRY(check_launch("k_nb<COUNT>"));

@@ -325,7 +325,8 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
                               double2 *__restrict__ rec, int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
-                              int4 *__restrict__ at, unsigned *__restrict__ buckets, unsigned *__restrict__ bucket_cnt,
+                              int4 *__restrict__ at, unsigned *__restrict__ items, unsigned *__restrict__ item_cnt,
+                              unsigned item_size,
                               const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
@@ -335,7 +336,7 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
         const unsigned h = ehash[e];
         const unsigned left = atomicSub(&bcount[h], 1u);  // (the counts are not needed any more)
         const unsigned pos = bstart[h] + left - 1u;
-        if (buckets && left == 1u) buckets[atomicAdd(bucket_cnt, 1u)] = h;  // each bucket that holds edges, once
+        if (items && ((left - 1u) & (item_size - 1u)) == 0u) items[atomicAdd(item_cnt, 1u)] = pos;  // k_search's
         const T x = edges[(size_t)e * sz + 0];
         const T y = edges[(size_t)e * sz + 1];
         const T th = edges[(size_t)e * sz + 2];

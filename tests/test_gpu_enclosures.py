@@ -122,3 +122,18 @@ def test_general_path_against_the_oracle(fp64_engine, oracle, kind, gms):
     o = oracle.run(e, nthreads=4, group_max_sz=gms)
     assert (r.num_curvelets, r.valid_pairs) == (o.num_curvelets, o.valid_pairs)
     assert np.array_equal(r.chains, o.chains)
+
+
+@pytest.mark.parametrize("run_edges", [0, 70000])
+@pytest.mark.parametrize("block_edges", [1, 7, 8, 9, 31, 32, 33, 40, 65])
+def test_search_items(engine, fp64_engine, block_edges, run_edges):
+    """Hash blocks (8 x 8 px) of as many edges as k_search's items hold (8, on runs of more than
+    64 Ki edges 32), one more and one less, apart and side by side, against the two-pass search."""
+    rng = np.random.default_rng(block_edges)
+    blocks = np.array([(b, r) for r in range(6) for b in range(12) if (b + r) % 3])
+    xy = (blocks[:, None, :] * 8 + rng.uniform(-0.45, 7.45, (len(blocks), block_edges, 2))).reshape(-1, 2)
+    e = _rows(xy[:, 0], xy[:, 1], rng.normal(0.3, 0.3, len(xy)))
+    if run_edges:  # single edges elsewhere
+        k = np.arange(run_edges)
+        e = np.concatenate([e, _rows(200.0 + 5 * (k % 300), 200.0 + 5 * (k // 300), 0.0)])
+    _same(engine.run(e), fp64_engine.run(e))
