@@ -180,6 +180,7 @@ struct FastArgs {
     const RunDims *dims;                // graph runs: the anchors are [0, dims->N)
     unsigned *queue;                    // QUEUE: tiles taken so far
     unsigned *over_cnt;                 // anchors k_curvelets leaves to k_curvelets_exact
+    unsigned *over_queue;               // the next of them (0 at start)
     int *over_list;
     const unsigned *uncertified;        // bit 1: an orientation is outside the certified range
 };
@@ -889,7 +890,11 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
     const unsigned rank1 = 2 * lane + 1 < md.cells ? (unsigned)a.fm.rank[2 * lane + 1] : 0xffffu;
     const float h = a.fm.h;
     FastCounts counts;
-    for (int it = (int)blockIdx.x * FAST_WARPS + wib; it < n_over; it += (int)gridDim.x * FAST_WARPS) {
+    for (;;) {
+        unsigned it = 0;
+        if (lane == 0) it = atomicAdd(a.over_queue, 1u);
+        it = __shfl_sync(FULL, it, 0);
+        if (it >= (unsigned)n_over) break;
         const int i = a.over_list[it];
         const unsigned long long row = a.row[i];
         const unsigned long long off = row & ((1ull << 48) - 1ull);

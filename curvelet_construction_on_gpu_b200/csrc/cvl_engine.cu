@@ -716,8 +716,8 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &
     a.wide_cnt = (unsigned *)(work + 2) + 1;
     a.wide_list = (int *)e->ncand.p;
     a.items = (const unsigned *)e->deg.p;
-    a.item_cnt = (const unsigned *)(work + 4);
-    a.queue = (unsigned *)(work + 4) + 1;
+    a.item_cnt = (const unsigned *)(work + 5);
+    a.queue = (unsigned *)(work + 5) + 1;
     a.item_size = search_item(n);
     a.pulls = ~0u;
     return a;
@@ -821,7 +821,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
     const bool persist = persistent_chunks(e, n);
     const int blocks = sms * FAST_BLOCKS;
     unsigned long long *work = (unsigned long long *)e->work.p;
-    unsigned *queues = (unsigned *)(work + 3);  // anchors taken, anchors pushed to the wide variant
+    unsigned *queues = (unsigned *)(work + 3);  // anchors taken; anchors left to k_curvelets_exact, and taken there
     unsigned *err = (unsigned *)e->err.p;
     MapStats *stats = (MapStats *)e->stats.p;
     const long long per_chunk = std::max<long long>(tn.chunk_pairs / 16, 1024);
@@ -856,7 +856,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
                 CVL_CUDA(cudaEventSynchronize(e->chunk_done));
                 e->yield_fn(e->yield_ctx);
             }
-            CVL_CUDA(cudaMemsetAsync(queues, 0, 2 * sizeof(unsigned), s));
+            CVL_CUDA(cudaMemsetAsync(queues, 0, 3 * sizeof(unsigned), s));
             FastArgs fa{};
             fa.md = md;
             fa.fm = fm;
@@ -881,6 +881,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             fa.tile = persist ? FAST_TILE : 1;
             fa.queue = persist ? queues : nullptr;
             fa.over_cnt = queues + 1;
+            fa.over_queue = queues + 2;
             fa.over_list = (int *)e->deg.p;  // (not read any more)
             fa.uncertified = (const unsigned *)(work + 2);
             const int grid = persist ? blocks : short_grid(a1 - a0, (long long)FAST_WARPS * tn.anchors_per_warp);
@@ -1001,7 +1002,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->out_off, sizeof(unsigned long long) * (n + 1)));
     CVL_TRY(e->alloc(e->stats, sizeof(MapStats) * M));
     CVL_TRY(e->alloc(e->err, sizeof(unsigned) * 4));
-    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 5));  // arena, pairs, certification and wide anchors, queues, buckets
+    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 6));  // arena, pairs, certification and wide anchors, queues (3), items
 
     unsigned *err = (unsigned *)e->err.p;
     MapStats *stats = (MapStats *)e->stats.p;
@@ -1024,7 +1025,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_CUDA(cudaMemsetAsync(e->bcount.p, 0, sizeof(unsigned) * (T + 1), s));
     CVL_CUDA(cudaMemsetAsync(e->stats.p, 0, sizeof(MapStats) * M, s));
     CVL_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(unsigned) * 4, s));
-    CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 5, s));
+    CVL_CUDA(cudaMemsetAsync(e->work.p, 0, sizeof(unsigned long long) * 6, s));
 
     // ---- (a) binning
     const int gb = short_grid(n, 256);
@@ -1036,7 +1037,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, rec_out, (int *)e->pos_of.p,
                                      F.e, F.cs2, F.at, pair_cap ? (unsigned *)e->deg.p : nullptr,
-                                     (unsigned *)((unsigned long long *)e->work.p + 4), search_item(n), nullptr);
+                                     (unsigned *)((unsigned long long *)e->work.p + 5), search_item(n), nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
 
@@ -1355,7 +1356,7 @@ std::vector<WsItem> workspace_plan(const cvl_tuning *tune, unsigned long long ar
     add(&E::out_off, 8 * (n + 1));
     add(&E::stats, sizeof(MapStats) * M);
     add(&E::err, 16);
-    add(&E::work, 40);
+    add(&E::work, 48);
     add(&E::scan_tmp, (T / SCAN_TILE + 64) * 4 * sizeof(unsigned long long) + 4096);  // the largest scan: T
     add(&E::chunk_start, 4 * (4096 + 1));
     // pair-sized (after the count)
@@ -1514,7 +1515,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             const std::pair<void *, size_t> zero[] = {{e->bcount.p, sizeof(unsigned) * (T + 1)},
                                                       {e->stats.p, sizeof(MapStats) * cap.M},
                                                       {e->err.p, 16},
-                                                      {e->work.p, 40},
+                                                      {e->work.p, 48},
                                                       {e->count.p, sizeof(unsigned) * (size_t)N},
                                                       {e->chunk_start.p, fm.ok ? 0 : sizeof(int) * (cap.K + 1)}};
             for (int r = 0; r < 6; ++r) {
@@ -1533,7 +1534,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
                                              fm.ok ? (double2 *)e->rec_k.p : nullptr, (int *)e->pos_of.p, F.e, F.cs2, F.at,
                                              fm.ok ? (unsigned *)e->deg.p : nullptr,
-                                             (unsigned *)((unsigned long long *)e->work.p + 4), search_item(N), dd);
+                                             (unsigned *)((unsigned long long *)e->work.p + 5), search_item(N), dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;
@@ -1611,6 +1612,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 // the atomics to pay
                 fa.queue = b == 1 ? queues : nullptr;
                 fa.over_cnt = queues + 1;
+                fa.over_queue = queues + 2;
                 fa.over_list = (int *)e->deg.p;
                 fa.uncertified = uncertified;  // a run outside the certified angles goes kernel by kernel
                 CVL_TRY(launch_curvelets(e, fa, sms * FAST_BLOCKS, sms * FAST_EXACT_BLOCKS));
