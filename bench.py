@@ -49,20 +49,17 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "edges/s"
-# per computed (non-close) pair: 63 cells x 20 FP64 flops, divisions counted as 1
+# per computed (non-close) pair: 63 cells x 20 flops, divisions counted as 1
 FLOPS_PER_PAIR_CELL = 20
-# DRAM bytes of k_bundles per computed pair, from one ncu capture of the kernel
-# (--set full, profiles/k_bundles_k_growth_persistent_hd.md) on the 242k-edge
-# 1920x1080 map: dram__bytes_read.sum 0.153864 GB + dram__bytes_write.sum 1.430769 GB
-# over 2,176,780 non-close pairs. The traffic is the valid pairs' bundle writes
-# (1,008 B each, about half of the computed pairs) plus the pair/anchor reads, so it
-# scales with the pairs a launch processes.
-BUNDLE_DRAM_BYTES_PER_PAIR = (0.153864e9 + 1.430769e9) / 2_176_780
-# FP64-pipe instructions of k_bundles per cell, from the same capture: the pipe was
-# active 51.553% of 1,750,328 active cycles per SM on 148 SMs (each issues 2 FP64
-# warp-instructions a cycle), 30.73 active lanes per warp-instruction, 2,176,780 x 63
-# cells. A division costs about 10 of them, which the algorithmic count takes as 1 flop.
-BUNDLE_FP64_INSTR_PER_CELL = 0.51553 * 1_750_328 * 148 * 2 * 30.73 / (2_176_780 * 63)
+# k_curvelets on the 242k-edge 1920x1080 map, one ncu capture (--set full,
+# profiles/k_curvelets_k_search_hd.md): warp instructions and DRAM bytes per edge. The
+# bundles stay on the chip, so the traffic is the pairs' ids and classes, the edges and the
+# records.
+CURVELETS_WARP_INSTR_PER_EDGE = 392_889_469 / 242_059
+CURVELETS_DRAM_BYTES_PER_EDGE = (30.807296e6 + 0.557312e6) / 242_059
+# FP32 lanes and warp-instruction issue slots of one SM per cycle
+SM_FP32_LANES = 128
+SM_ISSUE_SLOTS = 4
 
 
 def _args():
@@ -400,6 +397,11 @@ def run_reference(args, maps, cfg, world, rank):
     print(json.dumps(line))
 
 
+def _sm_count() -> int:
+    import torch
+    return int(torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count)
+
+
 def _stage_sums(times) -> dict:
     """Per-stage device ms of one run, summed over chunks."""
     out = {}
@@ -619,7 +621,7 @@ def path_hbm(n_edges: int, n_curv: int, ms_per_step: float, peaks: dict, edge_by
             "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in peaks else "fallback 6650 GB/s",
             "work": f"{edge_bytes} B per edge in + 100 B per curvelet out",
-            "note": "the path is bound by its FP64 bundle transport and by latency, not by HBM"}
+            "note": "the path is bound by k_curvelets' issue slots and by latency, not by HBM"}
 
 
 def run_ours(args, maps, cfg, world, rank, local, pg):
@@ -635,7 +637,7 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
         r.close()
     _barrier(pg)
     _progress("timed steps")
-    step_ms, kern, launches, bundle_launches = [], [], 0, 1
+    step_ms, kern, launches, curv_launches = [], [], 0, 1
     with _Clocks(local) as clk:
         for _ in range(args.steps):
             eng.flush_l2()
@@ -644,7 +646,7 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
             step_ms.append(st["device_ms"])
             launches = int(st["launches"])
             kt = eng.kernel_times()
-            bundle_launches = sum(1 for name, _ in kt if name == "bundles")
+            curv_launches = sum(1 for name, _ in kt if name == "curvelets")
             kern.append(_stage_sums(kt))
             r.close()
     _barrier(pg)
@@ -655,7 +657,6 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
     stats = last.stats()
     n_curv = int(stats["num_curvelets"])
     nonclose = int(stats["total_pairs"]) - int(stats["close_pairs"])
-    valid_nonclose = int(stats["valid_pairs"]) - int(stats["close_pairs"])
     last.close()
 
     plain = None
@@ -735,11 +736,13 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
 
     if rank != 0:
         return
-    curv_ms = float(np.mean([k.get("bundles", 0.0) for k in kern]))
+    curv_ms = float(np.mean([k.get("curvelets", 0.0) for k in kern]))
     flops = FLOPS_PER_PAIR_CELL * 63 * nonclose
     achieved = flops / (curv_ms / 1e3) / 1e12 if curv_ms > 0 else 0.0
-    launches_b = max(1, int(bundle_launches))
     clocks = clk.summary()
+    sms, hz = _sm_count(), 1e6 * float(clocks.get("sm_mhz") or 1965.0)
+    fp32_peak = sms * SM_FP32_LANES * 2 * hz / 1e12
+    issue_peak = sms * SM_ISSUE_SLOTS * hz
     stage_ms = {k: float(np.mean([d.get(k, 0.0) for d in kern])) for k in kern[0]} if kern else {}
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
@@ -750,24 +753,21 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
                            "valid_pairs_per_gpu": int(stats["valid_pairs"])},
         "curvelets_per_s": n_curv * world * args.steps / (sum_ms / 1e3),
         "stage_ms": stage_ms,
-        "roofline": {"bound": "fp64", "kernel": "k_bundles", "achieved": achieved, "peak": fp64_peak,
-                     "unit": "TFLOP/s", "frac": (achieved / fp64_peak) if fp64_peak else None,
-                     "peak_source": "measured DFMA loop (cvl_measure_fp64_peak), 2 flops per FMA",
+        "roofline": {"bound": "issue", "kernel": "k_curvelets (with k_curvelets_exact)", "achieved": achieved,
+                     "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
+                     "peak_source": f"{sms} SMs x {SM_FP32_LANES} FP32 lanes x 2 x the sampled clock",
                      "work": f"{FLOPS_PER_PAIR_CELL} flops x 63 cells x {nonclose} non-close pairs, "
-                             f"{launches_b} launch(es) per step",
-                     "traffic": BUNDLE_DRAM_BYTES_PER_PAIR * nonclose / launches_b,
+                             f"{max(1, int(curv_launches))} launch(es) per step; growth not counted",
+                     "traffic": CURVELETS_DRAM_BYTES_PER_EDGE * n_edges / max(1, int(curv_launches)),
                      "traffic_unit": "bytes per launch",
-                     "traffic_source": "ncu dram bytes of k_bundles on the 242k-edge map, per non-close pair, "
-                                       "times this workload's pairs per launch",
-                     "algorithmic_bytes": (1008.0 * valid_nonclose + 10.0 * nonclose) / launches_b,
-                     "algorithmic_bytes_note": "1,008 B of bundle per valid non-close pair written, 10 B per "
-                                               "computed pair of ids and flags",
-                     "fp64_pipe": {
-                         "instr_per_cell": BUNDLE_FP64_INSTR_PER_CELL,
-                         "frac": (BUNDLE_FP64_INSTR_PER_CELL * 63 * nonclose / (curv_ms / 1e3)
-                                  / (fp64_peak * 1e12 / 2.0)) if (fp64_peak and curv_ms > 0) else None,
-                         "note": "FP64-pipe instructions per cell from ncu, scaled to this run's k_bundles time, "
-                                 "against the DFMA issue peak (measured TFLOP/s / 2)"}},
+                     "traffic_source": "ncu dram bytes of k_curvelets on the 242k-edge map, per edge",
+                     "issue": {
+                         "warp_instr_per_edge": CURVELETS_WARP_INSTR_PER_EDGE,
+                         "frac": (CURVELETS_WARP_INSTR_PER_EDGE * n_edges / (curv_ms / 1e3) / issue_peak)
+                         if curv_ms > 0 else None,
+                         "note": "warp instructions per edge from ncu on the 242k-edge map, over this run's "
+                                 "curvelets stage, against 4 a cycle and SM; denser maps take more per edge"},
+                     "fp64_peak_tflops": fp64_peak},
         "path_hbm": path_hbm(n_edges, n_curv, sum_ms / args.steps, _measured_peaks(),
                              edge_bytes=8 * int(maps[0].shape[1])),
         "gpu_launches": launches,

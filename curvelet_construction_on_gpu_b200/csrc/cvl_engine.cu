@@ -2,11 +2,14 @@
 //
 // One engine = one CUDA device + one stream + a grow-only device workspace.
 // A run over a ragged batch of maps (a single map for the plain form):
-//   H2D edges -> (a) binning -> (b) neighbour count, scan -> [sync: pair total]
-//   -> (b) neighbour fill -> (c+d) fused bundles/growth/dedup/record
-//   -> scan of per-anchor counts -> [sync: curvelet total] -> (e) finalize -> D2H
-// The two syncs size the CSR/record and output buffers exactly; everything
-// else stays on the device.
+//   H2D edges -> (a) binning -> (b) one-pass neighbour search -> (c + d) bundles, growth,
+//   dedup and record in one kernel -> scan of per-anchor counts -> [sync: curvelet total]
+//   -> (e) finalize -> D2H
+// for double runs on grids k_curvelets serves (make_fast, search_serves); pairs that do not
+// fit their buffers, and orientations outside the enclosures' range, send a run to
+//   (b) neighbour count, scan -> [sync: pair total] -> fill
+// and the latter, float runs and other grids on to bundles and growth as two kernels per chunk.
+// Runs of up to 512 Ki edges replay the path as a CUDA graph with one synchronisation.
 #include <algorithm>
 #include <atomic>
 #include <chrono>

@@ -4,9 +4,10 @@
 // Pipeline over a ragged batch of M edge maps (M = 1 for the plain form):
 //   (a) k_bin_keys / k_bin_scatter  counting sort of the edges into S x S
 //       pixel-cell blocks (S a power of two >= the window half width + 1) of a
-//       spatial hash; SoA FP64 edge arrays in bucket order; per-edge
-//       sin/cos(theta +- dt) computed once;
-//   (b) k_nb<COUNT> / k_nb<FILL>     warp per anchor: the window's bucket
+//       spatial hash; the edges in bucket order, as records for the one-pass search
+//       (cvl_search.cuh) and k_curvelets (cvl_curvelets.cuh), as an array per field for
+//       the kernels here; per-edge sin/cos(theta +- dt) computed once;
+//   (b) k_nb<COUNT> / k_nb<FILL>     the two-pass search, warp per anchor: the window's bucket
 //       ranges are loaded by all lanes at once, then the candidates are
 //       enumerated 32 at a time with the reference's predicate (7x7 pixel
 //       window, not self, not d^2 > r^2; preprocess.hpp:129-167). COUNT writes
@@ -15,7 +16,7 @@
 //       (:165-167), rank-sorts them by (d^2, scan position) (:172-176) and
 //       writes the CSR row, each pair's direction-run class
 //       (cpu_curvelet.hpp:454-462) and the anchor's sin/cos(T2 + delta_t2_j).
-//   (c) + (d) + (e) are in cvl_path.cuh.
+//   (c) + (d) + (e) are in cvl_curvelets.cuh and, for float runs and other grids, cvl_path.cuh.
 //
 // Every FP64 expression keeps the reference's operand order; the library is
 // compiled with -fmad=false so no multiply-add is contracted, and uses IEEE

@@ -1,9 +1,9 @@
 // cvl_search.cuh -- sm_100a kernels of the curvelet path: (b) the neighbour search in one
 // pass, for the runs k_curvelets serves (cvl_curvelets.cuh).
 //
-// k_search: a warp per item, 32 or fewer anchors of a hash bucket, a lane per anchor. The anchors of one 8-pixel hash
-// block share their candidates: the edges of the 3 x 3 blocks around it that lie within w
-// pixels of it. The warp loads those once, keeps them in shared memory, and every lane tests
+// k_search: a warp per item, 32 or fewer anchors of a hash bucket, a lane per anchor. The
+// anchors of one 8-pixel hash block share their candidates: the edges of the 3 x 3 blocks
+// around it that lie within w pixels of it. The warp loads those once, keeps them in shared memory, and every lane tests
 // them with the reference's predicate (preprocess.hpp:129-167), reading each at the same time
 // as the others (a broadcast), and appends its neighbours to its column of a table. The rows
 // of the anchors are allocated together and back to back, so the warp writes them as one

@@ -471,7 +471,9 @@ int cvl_write_edges_binary(const char *path, const double *edges, int64_t num_ed
 /* ---- tuning and the autotuner -------------------------------------------
  * No reference counterpart. An engine keeps one tuning per size bucket of the
  * batch (its total edges); every tuning gives the same results bit for bit,
- * only the time changes. cvl_engine_autotune searches them on a
+ * only the time changes. Double runs on the default grid make bundles and chains in one
+ * kernel with a hash block of 8: there only anchors_per_warp and chunk_pairs matter, and
+ * those only where a run yields to others. The other knobs are float runs' and other grids'. cvl_engine_autotune searches them on a
  * device-resident batch by timing the whole path, and installs the best. */
 #define CVL_TUNING_BUCKETS 4          /* batches of <= 64 Ki, <= 512 Ki, <= 4 Mi, and more edges */
 typedef struct cvl_tuning {
@@ -562,8 +564,8 @@ int cvl_engine_last_kernel_times(cvl_engine *e, const char **names, double *ms, 
 int cvl_engine_last_launch_count(cvl_engine *e);
 
 /* Measures the device's FP64 FMA throughput (TFLOP/s, 2 flops per FMA) with a
- * register-resident dependent-chain loop; the roofline denominator for the
- * FP64-bound bundle kernel. */
+ * register-resident dependent-chain loop; the denominator for FP64-bound kernels
+ * (the bundle kernel of grids other than the default). */
 int cvl_measure_fp64_peak(cvl_engine *e, double *tflops);
 
 /* ---- Downstream: curvelets -> edgel link graph -> contour fragments ----------
