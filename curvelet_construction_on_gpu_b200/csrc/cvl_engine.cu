@@ -123,7 +123,7 @@ struct cvl_engine {
     std::shared_ptr<PinnedPool> pinned = std::make_shared<PinnedPool>();
 
     // workspace
-    DBuf edges, map_off, ehash, bcount, bstart, bfill, pos_of, orig_of;
+    DBuf edges, map_off, ehash, bcount, bstart, pos_of, orig_of;
     DBuf bx, by, bth, bsp, bcp, bsm, bcm, bcell, bmap;
     DBuf ncand, deg, pair_off, csr_ids, csr_d2, rec_ids, rec_k, rec_meta, count, out_off;
     DBuf chains, info, stats, err, work, scratch, scratch_chain, scratch_res, scan_tmp, flush, deg_orig, off_orig,
@@ -181,7 +181,7 @@ struct cvl_engine {
     bool enclosures_on = std::getenv("CVL_NO_ENCLOSURES") == nullptr;
     uint64_t ws_epoch = 0;                         // workspace (re)allocations so far
     uint64_t graph_replays = 0, graph_fallbacks = 0, graph_captures = 0, graph_clock = 0;
-    DBuf gdims, gchunks, gread;
+    DBuf gdims, gchunks;
     unsigned char *gread_host = nullptr;           // page-locked: the runs' sizes and the readback
 
     // per-kernel timing of the last run
@@ -258,11 +258,11 @@ struct cvl_engine {
     }
 
     void release_all() {
-        DBuf *all[] = {&edges, &map_off, &ehash, &bcount, &bstart, &bfill, &pos_of, &orig_of, &bx, &by, &bth, &bsp,
+        DBuf *all[] = {&edges, &map_off, &ehash, &bcount, &bstart, &pos_of, &orig_of, &bx, &by, &bth, &bsp,
                        &bcp, &bsm, &bcm, &bcell, &bmap, &ncand, &deg, &pair_off, &csr_ids, &csr_d2, &rec_ids,
                        &rec_k, &rec_meta, &count, &out_off, &chains, &info, &stats, &err, &work, &scratch,
                        &scratch_chain, &scratch_res, &run_cnt, &rec_base, &pcls, &pflag, &pair_anchor, &atrig, &bund, &chunk_start, &crank, &scan_tmp, &flush, &deg_orig, &off_orig, &gids, &gd2, &pairs_in, &pb_min,
-                       &pb_max, &pb_valid, &chains_alt, &info_alt, &edges_alt, &gdims, &gchunks, &gread};
+                       &pb_max, &pb_valid, &chains_alt, &info_alt, &edges_alt, &gdims, &gchunks};
         for (DBuf *b : all) {
             if (b->p) cudaFreeAsync(b->p, stream);
             b->p = nullptr;
@@ -1344,7 +1344,6 @@ std::vector<WsItem> workspace_plan(const cvl_tuning *tune, unsigned long long ar
     add(&E::ehash, 4 * n);
     add(&E::bcount, 4 * (T + 1));
     add(&E::bstart, 4 * (T + 1));
-    add(&E::bfill, 4 * (T + 1));
     add(&E::pos_of, 4 * n);
     for (DBuf E::*b : {&E::bx, &E::by, &E::bth, &E::bsp, &E::bcp, &E::bsm, &E::bcm}) add(b, R * n);
     add(&E::bcell, 8 * n);
@@ -1442,7 +1441,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     const FastModel fm = e->enclosures_on && search_serves(md) ? make_fast(md) : FastModel{};
     if (fm.ok) md.sbits = SEARCH_SBITS;
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
-        if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off || w.buf == &cvl_engine::bfill) continue;
+        if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off) continue;
         // k_curvelets keeps no bundles, pair flags or numbers in memory, its edges in records
         const DBuf cvl_engine::*unused[] = {
             &cvl_engine::bund, &cvl_engine::pflag, &cvl_engine::pair_anchor, &cvl_engine::rec_k, &cvl_engine::bx,
@@ -1769,7 +1768,6 @@ std::vector<WsItem> workspace_plan_with_graphs(const cvl_tuning *tune, unsigned 
         }
         v.push_back({&cvl_engine::gdims, sizeof(RunDims), false});
         v.push_back({&cvl_engine::gchunks, sizeof(ChunkDims) * (size_t)cap.K, false});
-        v.push_back({&cvl_engine::gread, (size_t)(2 + cap.M + 1) * 8, false});
     }
     return v;
 }
