@@ -535,6 +535,7 @@ struct FastCounts {
 // ---------------------------------------------------------------------------
 template <bool QUEUE>
 __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(const __grid_constant__ FastArgs a) {
+    if (*a.err & ERR_NONFINITE) return;  // no rows (cvl_search.cuh)
     extern __shared__ __align__(16) unsigned char cv_smem[];
     using Smem = FastSmem<FAST_CAP, FAST_SLOTS>;
     const Model &md = a.md;
@@ -876,6 +877,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
 // per lane. It takes the same comparisons and settles the undecided ones in FP64.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelets_exact(const __grid_constant__ FastArgs a) {
+    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char cv_smem[];
     constexpr int SLOTS = FAST_WIDE_SLOTS;
     const Model &md = a.md;

@@ -10,6 +10,12 @@
 // coalesced run, a lane per pair, each with its rank by (distance, scan order) in its
 // anchor's column and its classes.
 //
+// A run with a non-finite edge fails (ERR_NONFINITE, final since k_bin_keys), and no kernel
+// from here on may read what it left: k_bin_keys puts such an edge into bucket 0, whatever its
+// cell, so an item that it heads has another bucket's end, its neighbours' distances have no
+// order, and rows stay unwritten. k_search, k_search_wide, k_curvelets and k_curvelets_exact
+// leave at once. (On finite edges an item's head has its bucket's hash, and no item crosses it.)
+//
 // Rows are in no order, so the search needs no counting pass, no scan of the degrees and
 // no host synchronisation before the pairs' buffers are sized: a run whose rows do not fit
 // raises ERR_CAPACITY and goes again by the two passes (k_nb<COUNT>, k_nb<FILL>).
@@ -62,7 +68,7 @@ struct SearchArgs {
     MapStats *stats;
     unsigned *err;
     unsigned *wide_cnt;               // anchors for k_search_wide
-    int *wide_list;
+    int *wide_list;                   // [N]: an anchor is of one item, and is listed once
     const unsigned *items;            // each run of up to item_size anchors of a bucket, by its first (k_bin_scatter)
     const unsigned *item_cnt;
     unsigned item_size;               // a power of two, at most 32
@@ -114,6 +120,7 @@ struct SearchCounts {
 };
 
 __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(const __grid_constant__ SearchArgs a) {
+    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char se_smem[];
     SearchSmem &S = ((SearchSmem *)se_smem)[threadIdx.x >> 5];
     const Model &md = a.md;
@@ -288,6 +295,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(con
 // The anchors k_search left, a warp each: their candidates counted, then gathered and ranked
 // as k_nb<FILL> does.
 __global__ void __launch_bounds__(256) k_search_wide(const __grid_constant__ SearchArgs a) {
+    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char sw_smem[];
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
