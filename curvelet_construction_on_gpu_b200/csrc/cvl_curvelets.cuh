@@ -42,8 +42,9 @@
 // so that each bound is off by at most e0 max(1, |k| / max_k): by e0 where it lies
 // within [-max_k, max_k]; a larger one is recognised as larger (2^-14 of its size is
 // less than its distance past max_k plus e0), and clamps or closes the cell either way.
-// |D| below Dthr is accepted too when |s| >= S1 = 2 max_k Dthr + 8u and |D| >= Dtiny >
-// dD: then |k| > 1.4 max_k with the sign of its quotient certain.
+// |D| below Dthr is accepted too when |s| >= S1 = 2 max_k Dthr + 8u and |D| >= Dtiny > dD
+// at the longest pair's R (pair_radius): then |k| > 1.4 max_k with the sign of its
+// quotient certain.
 // Where a column fails, it is made once more with e1, the numerators, s and D computed in
 // FP64 and rounded once each (fine_column): then a quotient is off by 12u |k|, and by the
 // angles' 2^-41 over |D| or e1, so that |D| >= 2^-24 and e1 >= 2^-22 suffice.
@@ -57,14 +58,13 @@
 // and anything between is undecided: a few tests in ten thousand.
 #pragma once
 
+#include "cvl_enclosures.h"
 #include "cvl_path.cuh"
 #include "cvl_search.cuh"
 
 namespace cvl {
 
-constexpr int FAST_P = 9;        // grid offsets of the column code (the default grid)
-constexpr int FAST_CAP = 32;     // pairs of a direction run k_curvelets takes
-constexpr int FAST_WIDE = 128;   // and k_curvelets_exact (max_candidates <= 128)
+constexpr int FAST_CAP = 32;     // pairs of a direction run k_curvelets takes (k_curvelets_exact: FAST_WIDE)
 // Bundles of an anchor's seeds kept in shared memory (later seeds' are recomputed), warps per
 // block and blocks per SM. The kernel is bound by its issue slots; 5 blocks (96 registers, no
 // spills) with 16 slots measured best: 1.42 ms on a 735k-edge map and 14.6 ms on a dense
@@ -79,76 +79,6 @@ constexpr int FAST_EXACT_BLOCKS = 3;
 // two kernels took 14.64 ms, with these 14.48; 16 or 24 in two blocks: 14.82)
 constexpr int FAST_WIDE_SLOTS = 14;
 constexpr int FAST_TILE = 4;     // consecutive anchors a queue-pulling warp takes at a time
-// e0 / max_k: larger leaves more comparisons undecided, smaller more columns to be made anew
-// (2^-13 to 2^-15 measured alike)
-constexpr double FAST_E0 = 0x1p-14;
-
-// The single-precision model, made on the host from the FP64 one (make_fast).
-struct FastModel {
-    float d[FAST_P], d2[FAST_P], c2[FAST_P];  // each offset's d, d^2, 2d + 2dx
-    float mk, h;               // max_k, 2.04 e0
-    float dx2, dx_2, ndx_4;    // dx^2, 2 dx, -4 dx
-    float e0, eR, eRR;         // Ethr = e0 + eR Rb + eRR Rb^2
-    float d0, dR;              // Dthr = d0 + dR Rb
-    float s0, sR;              // S1 = s0 + sR Rb
-    float dtiny;
-    int ok;                    // the model is within the enclosures' range
-    unsigned char rank[64];    // best-cell rank of each cell (fill_curvelet_info, :202-219)
-    unsigned char cell_of[64]; // and the cell of each rank
-};
-
-// The enclosures' constants (the bounds above), or ok = 0: outside them the two-kernel
-// path runs (other grids, cells no curvelet may take, extreme parameters).
-inline FastModel make_fast(const Model &md) {
-    FastModel f{};
-    const double u = 0x1p-24, mk = md.max_k, dx = md.dx, up = 1.02;
-    const double dm = md.sx * ((double)md.P - 1.0) / 2.0;
-    bool ok = md.P == FAST_P && md.Q >= 3 && md.cells <= 64 && md.max_cand <= FAST_WIDE && mk >= 0x1p-10 &&
-              mk <= 0x1p10 && md.nrad >= 0x1p-10 && md.nrad <= 64.0 && dx >= 0x1p-20 && dx <= 64.0 && dm <= 64.0 &&
-              md.dt >= -64.0 && md.dt <= 64.0 && md.st * md.Q <= 128.0;
-    for (int c = 0; c < md.cells && ok; ++c) {  // every cell may be the best one (:207-219)
-        const double ddx = md.sx * ((double)(c / md.Q) - ((double)md.P - 1.0) / 2.0);
-        const double ddt = md.st * ((double)(c % md.Q) - ((double)md.Q - 1.0) / 2.0);
-        ok = ddx * ddx + ddt * ddt < 100.0;
-    }
-    if (!ok) return f;
-    for (int i = 0; i < FAST_P; ++i) {
-        const double d = md.sx * ((double)i - ((double)md.P - 1.0) / 2.0);
-        f.d[i] = (float)d;
-        f.d2[i] = (float)(d * d);
-        f.c2[i] = (float)(2.0 * d + 2.0 * dx);
-    }
-    const double e0 = FAST_E0 * mk, den = e0 - 8.0 * u * mk;
-    f.mk = (float)mk;
-    f.h = (float)(2.04 * e0);
-    f.dx2 = (float)md.dx2;
-    f.dx_2 = (float)(2.0 * dx);
-    f.ndx_4 = (float)(-4.0 * dx);
-    f.e0 = (float)(up * u * (4.0 * dm + 16.0 * dx + mk * (3.0 * dm * dm + 6.0 * dx * dx)) / den);
-    f.eR = (float)(up * u * (10.0 + mk * 12.0 * dm) / den);
-    f.eRR = (float)(up * u * mk * 7.0 / den);
-    f.d0 = (float)(up * u * (4.0 + mk * 6.0 * dm) / den);
-    f.dR = (float)(up * u * mk * 5.0 / den);
-    f.s0 = (float)(up * (2.0 * mk * f.d0 + 8.0 * u));
-    f.sR = (float)(up * 2.0 * mk * f.dR);
-    f.dtiny = (float)(2.0 * u * (5.0 * md.nrad + 6.0 * dm));
-    // the cells ordered by (d, row-major index), with the reference's arithmetic
-    double dist[64];
-    for (int c = 0; c < md.cells; ++c) {
-        const double ddx = md.sx * ((double)(c / md.Q) - ((double)md.P - 1.0) / 2.0);
-        const double ddt = md.st * ((double)(c % md.Q) - ((double)md.Q - 1.0) / 2.0);
-        const double a = ddx * ddx, b = ddt * ddt;
-        dist[c] = a + b;
-    }
-    for (int c = 0; c < md.cells; ++c) {
-        int r = 0;
-        for (int o = 0; o < md.cells; ++o) r += dist[o] < dist[c] || (dist[o] == dist[c] && o < c);
-        f.rank[c] = (unsigned char)r;
-        f.cell_of[r] = (unsigned char)c;
-    }
-    f.ok = 1;
-    return f;
-}
 
 struct FastBinned {
     FastEdge *e;     // [N], bucket order

@@ -721,6 +721,7 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &
     a.items = (const unsigned *)e->deg.p;
     a.item_cnt = (const unsigned *)(work + 5);
     a.queue = (unsigned *)(work + 5) + 1;
+    a.scale = (float)(65000.0 / (pair_radius(md) * pair_radius(md)));
     a.item_size = search_item(n);
     a.pulls = ~0u;
     return a;

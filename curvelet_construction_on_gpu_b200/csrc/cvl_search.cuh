@@ -71,6 +71,7 @@ struct SearchArgs {
     int *wide_list;                   // [N]: an anchor is of one item, and is listed once
     const unsigned *items;            // each run of up to item_size anchors of a bucket, by its first (k_bin_scatter)
     const unsigned *item_cnt;
+    float scale;                      // 65,000 over the longest pair's d2 (rounding and truncation keep d2's order)
     unsigned item_size;               // a power of two, at most 32
     unsigned *queue;                  // the next item (0 at start)
     unsigned pulls;                   // items a warp takes at most
@@ -128,7 +129,6 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(con
     const unsigned lt_mask = (1u << lane) - 1u;
     const int cap = min(SEARCH_CAP, md.max_cand - 1);  // (a list of max_cand or more counts as cut)
     const int w = md.w;
-    const float scale = 65000.0f / (float)md.rad_sqr;  // (rounding and truncation keep d2's order)
     SearchCounts counts;
     // The heaviest block has 13 to 19 times the mean's work (anchors x candidates), so warps pull
     // items from a queue: a dense 3.65M-edge map's search 3.10 -> 2.48 ms, a 735k-edge one's
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(con
                         const double d2 = sq_dist(ax, ay, p.x, p.y);  // preprocess.hpp:160
                         if (!(d2 > md.rad_sqr) && S.cj[k] != i) {     // :161-163
                             if (n < cap) {
-                                S.d2[n][lane] = (unsigned short)((float)d2 * scale);
+                                S.d2[n][lane] = (unsigned short)((float)d2 * a.scale);
                                 S.id[n][lane] = (unsigned char)k;
                             }
                             ++n;

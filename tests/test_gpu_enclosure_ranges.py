@@ -1,0 +1,58 @@
+"""The fused path at the ends of what its enclosures cover, against an engine that makes
+every bundle in FP64 (CVL_NO_ENCLOSURES): the same counts, chains and info bits. Each case
+asserts from the stage names that the ordinary engine did run the fused kernels."""
+import numpy as np
+import pytest
+
+import curvelet_construction_on_gpu_b200 as cvl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engines():
+    with pytest.MonkeyPatch.context() as m:
+        m.setenv("CVL_NO_ENCLOSURES", "1")
+        fp64 = cvl.Engine()
+    fused = cvl.Engine()
+    fused.set_graphs(False)  # stage by stage, so that the stages can be told
+    yield fused, fp64
+    fused.close()
+    fp64.close()
+
+
+def _stages(eng):
+    return {name for name, _ in eng.kernel_times()}
+
+
+def _assert_fused(eng):
+    s = _stages(eng)
+    assert "curvelets" in s and "bundles" not in s, s
+
+
+def _same(a, b):
+    for name in ("valid_pairs", "total_neighbor_pairs", "max_num_of_neighbors", "truncated_anchors", "num_curvelets"):
+        assert getattr(a, name) == getattr(b, name), name
+    assert np.array_equal(a.chains, b.chains)
+    assert np.array_equal(np.asarray(a.info).view(np.int64), np.asarray(b.info).view(np.int64))
+
+
+def _scatter(n, size, seed):
+    rng = np.random.default_rng(seed)
+    return np.column_stack([rng.uniform(0, size, (n, 2)), rng.uniform(-np.pi, np.pi, n), np.ones(n)])
+
+
+@pytest.mark.parametrize("nrad", [0.5, 3.5])
+@pytest.mark.parametrize("rad,window,edges,size", [(8.0, 8, 30000, 600), (40.0, 8, 30000, 600), (40.0, 32, 6000, 1000)])
+def test_search_radius_apart_from_nrad(engines, rad, window, edges, size, nrad):
+    """Staged calls, whose neighbour lists have a radius of their own."""
+    fused, fp64 = engines
+    e = _scatter(edges, size, 3)
+    p = cvl.CurveletParams(nrad=nrad)
+    got, want = (eng.build_neighbor_graph(e, rad, window, 128) for eng in engines)
+    n = fused.form_pairwise_bundles(got, p)
+    _assert_fused(fused)
+    assert n == fp64.form_pairwise_bundles(want, p) > 0
+    r = fused.build_curvelets(got, p)
+    _assert_fused(fused)
+    _same(r, fp64.build_curvelets(want, p))
