@@ -46,8 +46,16 @@
 // at the longest pair's R (pair_radius): then |k| > 1.4 max_k with the sign of its
 // quotient certain.
 // Where a column fails, it is made once more with e1, the numerators, s and D computed in
-// FP64 and rounded once each (fine_column): then a quotient is off by 12u |k|, and by the
-// angles' 2^-41 over |D| or e1, so that |D| >= 2^-24 and e1 >= 2^-22 suffice.
+// FP64 and rounded once each (fine_column). Its roundings to single precision leave a
+// quotient off by 12u |k|. Its FP64 quantities differ from the reference's by their own
+// rounding and by that of the reference's angles: half an ulp of T2t, and half one of
+// T2t - (T0 -+ dt), so at most 2^-52 (|T2| + |T0| + dt + max |dt_j|). With
+// eps = 2^-51 (|T2| + |T0| + dt + max |dt_j| + 4) for both,
+//   s: eps    D: eps (R + dm) =: fD    N: eps (3R + dm + dx) =: fN
+//   e1: eps (R^2 + 3 dm R + dm^2 + dx^2) =: fE
+// at the longest pair's R, and, as above, a cell is accepted when
+//   e1 >= (fN + max_k fE) / (e0 - 12u max_k),  |D| >= (eps + max_k fD) / (e0 - 12u max_k).
+// (2^-27 and 2^-30 for the default parameters and orientations within a turn.)
 // The FP64 path's own rounding (2^-50 of these magnitudes), the addition theorem on
 // its rounded angles (|theta| <= 2^10, checked when binning: 2^-41) and higher orders
 // of u are covered by 2% on Ethr, Dthr and S1.
@@ -323,8 +331,12 @@ __device__ __forceinline__ float4 lane_bundle(const FastArgs &a, const float4 *g
 
 // A column's cells from quantities computed in FP64 and rounded once. Returns whether the
 // enclosures hold.
-__device__ __forceinline__ bool fine_column(const FastArgs &a, double2 cs, double2 c2, FastEdge ae, int nn, bool branch1,
-                                            float2 *b, float &wmax) {
+__device__ __forceinline__ bool fine_column(const FastArgs &a, double2 cs, int i, int nn, bool branch1, float2 *b,
+                                            float &wmax) {
+    const double2 c2 = a.F.cs2[i];
+    const FastEdge ae = a.F.e[i];
+    const float ang = (float)(fabs(a.B.th[i]) + fabs(a.B.th[nn])) + a.fm.fa;
+    const float ethr = a.fm.fe * ang, dthr = a.fm.fd * ang;
     const double sT = fma(c2.y, cs.x, c2.x * cs.y), cT = fma(c2.x, cs.x, -(c2.y * cs.y));
     const double X = ae.x - a.F.e[nn].x, Y = ae.y - a.F.e[nn].y;
     const double cm = a.B.cm[nn], sm = a.B.sm[nn], cp = a.B.cp[nn], sp = a.B.sp[nn];
@@ -344,7 +356,7 @@ __device__ __forceinline__ bool fine_column(const FastArgs &a, double2 cs, doubl
         const float re = rcp_approx(e1);
         const float n = min3((float)(N + 2.0 * a.md.dx) * re, -(slof * rcp_approx(dlo)), a.fm.mk);
         const float M = min3((float)(2.0 * a.md.dx - N) * re, shif * rcp_approx(dhi), a.fm.mk);
-        ok = ok && e1 >= 0x1p-22f && fabsf(dlo) >= 0x1p-24f && fabsf(dhi) >= 0x1p-24f;
+        ok = ok && e1 >= ethr && fabsf(dlo) >= dthr && fabsf(dhi) >= dthr;
         wmax = fmaxf(wmax, n + M);
         b[k] = make_float2(n, M);
     }
@@ -599,7 +611,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
                         bool bad = on && !(emin >= g0.w && dlmin >= (fabsf(slo) >= g2.w ? a.fm.dtiny : g1.w) &&
                                            dhmin >= (fabsf(shi) >= g2.w ? a.fm.dtiny : g1.w));
                         if (__any_sync(FULL, bad)) {
-                            if (bad && !fine_column(a, T.cs[jl], a.F.cs2[i], a.F.e[i], S.nn[p], list[p] & L_BRANCH1, b, wmax))
+                            if (bad && !fine_column(a, T.cs[jl], i, S.nn[p], list[p] & L_BRANCH1, b, wmax))
                                 undecided = 1e30f;
                         }
                     }

@@ -22,6 +22,7 @@ struct FastModel {
     float d0, dR;              // Dthr = d0 + dR Rb
     float s0, sR;              // S1 = s0 + sR Rb
     float dtiny;
+    float fe, fd, fa;          // fine_column's thresholds of e1 and D: fe, fd times |T2| + |T0| + fa
     int ok;                    // the model is within the enclosures' range
     unsigned char rank[64];    // best-cell rank of each cell (fill_curvelet_info, :202-219)
     unsigned char cell_of[64]; // and the cell of each rank
@@ -71,6 +72,11 @@ FastModel make_fast(const M &md) {
     f.s0 = (float)(up * (2.0 * mk * f.d0 + 8.0 * u));
     f.sR = (float)(up * 2.0 * mk * f.dR);
     f.dtiny = (float)(2.0 * u * (5.0 * R + 6.0 * dm));
+    // fine_column: eps = 2^-51 (|T2| + |T0| + fa), the FP64 quantities' errors in its terms
+    const double fine = up * 0x1p-51 / (e0 - 12.0 * u * mk);
+    f.fe = (float)(fine * (3.0 * R + dm + dx + mk * (R * R + 3.0 * dm * R + dm * dm + dx * dx)));
+    f.fd = (float)(fine * (1.0 + mk * (R + dm)));
+    f.fa = (float)(up * (4.0 + std::fabs((double)md.dt) + md.st * ((double)md.Q - 1.0) / 2.0));
     // the cells ordered by (d, row-major index), with the reference's arithmetic
     double dist[64];
     for (int c = 0; c < md.cells; ++c) {

@@ -30,7 +30,7 @@ class _M(C.Structure):
 class _F(C.Structure):
     _fields_ = [("d", C.c_float * 9), ("d2", C.c_float * 9), ("c2", C.c_float * 9)] + \
                [(k, C.c_float) for k in ("mk", "h", "dx2", "dx_2", "ndx_4", "e0", "eR", "eRR", "d0", "dR", "s0", "sR",
-                                         "dtiny")] + \
+                                         "dtiny", "fe", "fd", "fa")] + \
                [("ok", C.c_int), ("rank", C.c_ubyte * 64), ("cell_of", C.c_ubyte * 64)]
 
 
@@ -61,8 +61,7 @@ def _r(x):
 
 
 def _rcp(x, rng):
-    with np.errstate(divide="ignore"):
-        y = _r(1.0 / x)  # rcp.approx: within 2u of 1/x
+    y = _r(1.0 / x)  # rcp.approx: within 2u of 1/x
     return _r(y * (1.0 + rng.choice([-1.0, 0.0, 1.0], y.shape) * U))
 
 
@@ -71,25 +70,34 @@ def _offset(s, k, n):
 
 
 def _pairs(rng, m, R, n, turns):
-    """DX, DY, T2, T0 and a cell (i, j) each: a third of them at random, a third with a k_dt
-    denominator of that cell near 0, and a third with its e1 near 0 (where such a pair is not a
-    close one). Orientations within `turns` turns."""
-    T2 = rng.uniform(-np.pi, np.pi, n) + 2 * np.pi * rng.integers(-turns, turns + 1, n)
-    T0 = rng.uniform(-np.pi, np.pi, n) + 2 * np.pi * rng.integers(-turns, turns + 1, n)
+    """DX, DY, T2, T0 and a cell (i, j) each, a fifth of them each (where it is not a close pair):
+    at random; a k_dt denominator D of the cell near 0; its e1 near 0; D near 0 and s with it,
+    so that k_dt is about max_k; e1 near 0 and a k_dx numerator with it. Orientations
+    within `turns` turns."""
+    def turn():
+        return 2 * np.pi * rng.integers(-turns, turns + 1, n)
+
+    def sign():
+        return rng.choice([-1.0, 1.0], n)
+
+    T2, T0 = rng.uniform(-np.pi, np.pi, n) + turn(), rng.uniform(-np.pi, np.pi, n) + turn()
     i, j = rng.integers(0, m.P, n), rng.integers(0, m.Q, n)
     d, T2t = _offset(m.sx, i, m.P), T2 + _offset(m.st, j, m.Q)
     sT, cT = np.sin(T2t), np.cos(T2t)
     r, phi = R * np.sqrt(rng.uniform(0, 1, n)), rng.uniform(-np.pi, np.pi, n)
-    DX, DY = r * np.cos(phi), r * np.sin(phi)
-    tiny = rng.choice([-1.0, 1.0], n) * 10.0 ** rng.uniform(-11, -2, n)
-    e = np.arange(n) % 3 == 2  # e1 = (tt - d)^2 + v^2 - dx^2, with tt and v along (sT, -cT) and (cT, sT)
-    tt, v = d + (m.dx + tiny) * np.cos(phi), (m.dx + tiny) * np.sin(phi)
-    DX, DY = np.where(e, sT * tt + cT * v, DX), np.where(e, sT * v - cT * tt, DY)
+    tt, v = r * np.cos(phi), r * np.sin(phi)  # DX, DY along (sT, -cT) and (cT, sT)
+    kind = np.arange(n) % 5
+    tiny, k = sign() * 10.0 ** rng.uniform(-11, -2, n), m.max_k * rng.uniform(-1.5, 1.5, n)
+    # e1 = (tt - d)^2 + v^2 - dx^2, and D is v where s is 0
+    side, e = sign(), np.abs(tiny)
+    tt = np.where(kind == 2, d + (m.dx + tiny) * np.cos(phi), np.where(kind == 4, d + side * (m.dx + k * e / 2), tt))
+    v = np.where(kind == 2, (m.dx + tiny) * np.sin(phi), np.where(kind == 3, tiny, np.where(
+        kind == 4, sign() * np.sqrt(np.maximum(e * (1 - k * m.dx) - (k * e / 2) ** 2, 0)), v)))
+    DX, DY = sT * tt + cT * v, sT * v - cT * tt
     # D = a cos t + b sin t, with t = T0 -+ dt, a = DX - d sin T2t, b = DY + d cos T2t
-    z = np.arange(n) % 3 == 1
     a, b = DX - d * sT, DY + d * cT
-    t = np.arctan2(b, a) + np.pi / 2 + tiny / np.hypot(a, b) + 2 * np.pi * rng.integers(-turns, turns + 1, n)
-    T0 = np.where(z, t + rng.choice([-1.0, 1.0], n) * m.dt, T0)
+    t = np.where(kind == 1, np.arctan2(b, a) + np.pi / 2 + tiny / np.maximum(np.hypot(a, b), 1e-9), T2t - k * tiny) + turn()
+    T0 = np.where((kind == 1) | (kind == 3), t + sign() * m.dt, T0)
     keep = (DX * DX + DY * DY >= 4 * m.dx2) & (DX * DX + DY * DY <= R * R)
     return tuple(x[keep] for x in (DX, DY, T2, T0, i, j))
 
@@ -104,6 +112,12 @@ def _want(m, DX, DY, T2, T0, i, j):
         s = np.sin(T2t - t)
         out.append(s / (-s * d + np.cos(t) * DX + np.sin(t) * DY))
     return out
+
+
+@pytest.fixture(autouse=True)
+def _quotients_by_zero():
+    with np.errstate(divide="ignore", invalid="ignore"):
+        yield
 
 
 def _check(m, want, got, ok):
@@ -152,6 +166,39 @@ def test_columns(shim, over):
         got.append(_r(sn * _rcp(D, rng)))
         ok &= (np.abs(D) >= dthr) | ((np.abs(sn) >= S1) & (np.abs(D) >= f.dtiny))
     assert ok.sum() > 0.1 * ok.size
+    _check(m, _want(m, DX, DY, T2, T0, i, j), got, ok)
+
+
+@pytest.mark.parametrize("turns", [0, 1, 16, 160])
+@pytest.mark.parametrize("over", SETS + [dict(max_k=0.002), dict(max_k=2.0 ** -10), dict(max_k=1000.0),
+                                         dict(rad=1e6, w=64, max_k=0.002), dict(dx=0.36, max_k=2.0 ** -10),
+                                         dict(dx=7.2, sx=2.0, max_k=0.002, nrad=30.0, w=30)],
+                         ids=lambda o: "-".join(f"{k}{v:g}" for k, v in o.items()) or "default")
+def test_fine_columns(shim, over, turns):
+    """fine_column: FP64 quantities rounded once, under the thresholds of the pair's angles."""
+    m, f, R = _model(shim, **over)
+    assert f.ok
+    rng = np.random.default_rng(18 + turns)
+    DX, DY, T2, T0, i, j = _pairs(rng, m, R, 300_000, turns)
+    sT, cT = _trig(m, T2, j)
+    d = _offset(m.sx, i, m.P)
+    t2 = -2.0 * (sT * DX - cT * DY)
+    N = t2 + 2.0 * d
+    e1 = _r(d * (t2 + d) + (DX * DX + (DY * DY - m.dx2)))
+    ang = _r(_r(np.abs(T2) + np.abs(T0)) + f.fa)
+    ethr, dthr = _r(f.fe * ang), _r(f.fd * ang)
+    re = _rcp(e1, rng)
+    got, ok = [-_r(_r(N + 2.0 * m.dx) * re), _r(_r(2.0 * m.dx - N) * re)], e1 >= ethr
+    small = (e1 < 100 * ethr)
+    for t in (T0 - m.dt, T0 + m.dt):
+        c, s = np.cos(t), np.sin(t)
+        sn = sT * c - cT * s
+        D = _r(-sn * d + (c * DX + s * DY))
+        got.append(_r(_r(sn) * _rcp(D, rng)))
+        ok &= np.abs(D) >= dthr
+        small |= np.abs(D) < 100 * dthr
+    assert ok.sum() > 0.1 * ok.size
+    assert (ok & small).sum() > 1000  # denominators near the thresholds were drawn
     _check(m, _want(m, DX, DY, T2, T0, i, j), got, ok)
 
 

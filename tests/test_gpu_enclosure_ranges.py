@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import curvelet_construction_on_gpu_b200 as cvl
+from curvelet_construction_on_gpu_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,27 @@ def test_search_radius_apart_from_nrad(engines, rad, window, edges, size, nrad):
     r = fused.build_curvelets(got, p)
     _assert_fused(fused)
     _same(r, fp64.build_curvelets(want, p))
+
+
+def _map(kind):
+    if kind == "small":
+        return synth.plain_small(3)
+    if kind == "lines":  # parallel lines 0.8 to 0.9 px apart: e1 near 0, perpendicular denominators
+        gx, k = np.meshgrid(np.arange(200.0), np.arange(12.0))
+        return np.column_stack([gx.ravel(), (10 + 0.8 * k + 0.002 * k * k).ravel(), (1e-9 * k).ravel(), np.ones(gx.size)])
+    return _scatter(20000, 220, 8)
+
+
+@pytest.mark.parametrize("turns", [0, 16, 159])  # orientations within 2 pi, about 100 and about 1000 rad
+@pytest.mark.parametrize("over", [dict(), dict(max_k=0.002), dict(max_k=2.0 ** -10), dict(max_k=900.0), dict(dx=0.36),
+                                  dict(dx=0.36, max_k=2.0 ** -10), dict(nrad=60.0)],
+                         ids=lambda o: "-".join(f"{k}{v:g}" for k, v in o.items()) or "default")
+@pytest.mark.parametrize("kind", ["small", "lines", "scatter"])
+def test_angles_and_curvatures(engines, kind, over, turns):
+    fused, fp64 = engines
+    e = _map(kind).copy()
+    e[:, 2] += 2 * np.pi * np.random.default_rng(4).integers(-turns, turns + 1, len(e))
+    p = cvl.CurveletParams(**over)
+    r = fused.run(e, p)
+    _assert_fused(fused)
+    _same(r, fp64.run(e, p))
