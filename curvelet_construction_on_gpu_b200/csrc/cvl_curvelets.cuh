@@ -120,7 +120,7 @@ struct FastArgs {
     unsigned *over_cnt;                 // anchors k_curvelets leaves to k_curvelets_exact
     unsigned *over_queue;               // the next of them (0 at start)
     int *over_list;
-    const unsigned *uncertified;        // bit 1: an orientation is outside the certified range
+    const unsigned *unfit;              // UNFIT_*
 };
 
 constexpr unsigned L_KMASK = 0x3ffu, L_NOSEED = 0x2000u, L_CLOSE = 0x4000u, L_BRANCH1 = 0x8000u;
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
     using Smem = FastSmem<FAST_CAP, FAST_SLOTS>;
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (a.uncertified && (*a.uncertified & UNCERT_ANGLE)) {  // the host runs the two-kernel path instead
+    if (*a.unfit & UNFIT_ANGLE) {  // the host runs the two-kernel path instead
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, ERR_CAPACITY);
         return;
     }
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelet
     constexpr int SLOTS = FAST_WIDE_SLOTS;
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (a.uncertified && (*a.uncertified & UNCERT_ANGLE)) return;
+    if (*a.unfit & UNFIT_ANGLE) return;
     const int n_over = (int)*a.over_cnt;
     if ((int)blockIdx.x * FAST_WARPS >= n_over) return;
     FastBlockSmem &T = *(FastBlockSmem *)cv_smem;

@@ -696,6 +696,8 @@ BinnedT<R> binned_arrays(const cvl_engine *e) {
     B.map = (int *)e->bmap.p;
     return B;
 }
+// A run's UNFIT_* flags (beside the queues, cleared with the counters).
+inline unsigned *unfit_of(const cvl_engine *e) { return (unsigned *)((unsigned long long *)e->work.p + 4) + 1; }
 // The one-pass search: pairs into csr_ids / pcls (pair_cap of them), rows into fast_rows.
 SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &B, const FastBinned &F, int n, int M,
                        unsigned long long pair_cap) {
@@ -887,7 +889,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             fa.over_cnt = queues + 1;
             fa.over_queue = queues + 2;
             fa.over_list = (int *)e->deg.p;  // (not read any more)
-            fa.uncertified = (const unsigned *)(work + 2);
+            fa.unfit = unfit_of(e);
             const int grid = persist ? blocks : short_grid(a1 - a0, (long long)FAST_WARPS * tn.anchors_per_warp);
             CVL_TRY(launch_curvelets(e, fa, grid, sms * FAST_EXACT_BLOCKS));
             e->mark("curvelets");
@@ -1006,7 +1008,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     CVL_TRY(e->alloc(e->out_off, sizeof(unsigned long long) * (n + 1)));
     CVL_TRY(e->alloc(e->stats, sizeof(MapStats) * M));
     CVL_TRY(e->alloc(e->err, sizeof(unsigned) * 4));
-    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 6));  // arena, pairs, certification and wide anchors, queues (3), items
+    CVL_TRY(e->alloc(e->work, sizeof(unsigned long long) * 6));  // arena, pairs, certification and wide anchors, queues (3) and UNFIT_*, items
 
     unsigned *err = (unsigned *)e->err.p;
     MapStats *stats = (MapStats *)e->stats.p;
@@ -1035,7 +1037,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     const int gb = short_grid(n, 256);
     unsigned *uncertified = (unsigned *)((unsigned long long *)e->work.p + 2);  // zeroed with the counters
     k_bin_keys<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (unsigned *)e->ehash.p, (unsigned *)e->bcount.p,
-                                  err, uncertified, nullptr);
+                                  err, uncertified, unfit_of(e), nullptr);
     CVL_TRY(check_launch("k_bin_keys"));
     CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
@@ -1110,8 +1112,8 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
                              cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(ro.stats.data(), stats, sizeof(MapStats) * M, cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    unsigned h_uncertified = 0;
-    CVL_CUDA(cudaMemcpyAsync(&h_uncertified, uncertified, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    unsigned h_unfit = 0;
+    CVL_CUDA(cudaMemcpyAsync(&h_unfit, unfit_of(e), sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CVL_CUDA(cudaMemcpyAsync(cstart.data(), e->chunk_start.p, sizeof(int) * (max_chunks + 1), cudaMemcpyDeviceToHost,
                              s));
     CVL_CUDA(cudaStreamSynchronize(s));
@@ -1128,7 +1130,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     // ---- (b) neighbour fill: CSR, pair classes, pair -> anchor, anchor trig
     CVL_TRY(e->alloc(e->csr_ids, sizeof(int) * P));
     if (want_d2) CVL_TRY(e->alloc(e->csr_d2, sizeof(R) * P));
-    const bool fast = fm.ok && !(h_uncertified & UNCERT_ANGLE);
+    const bool fast = fm.ok && !(h_unfit & UNFIT_ANGLE);
     if (path) CVL_TRY(e->alloc(e->pcls, P));
     if (path && !fast) {
         CVL_TRY(e->alloc(e->pflag, P));
@@ -1200,6 +1202,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         for (int c = 0; c <= nchunks; ++c)
             CVL_CUDA(cudaMemcpyAsync(&h_poff[c], (unsigned long long *)e->pair_off.p + cstart[c],
                                      sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+        unsigned h_uncertified = 0;
         CVL_CUDA(cudaMemcpyAsync(&h_uncertified, uncertified, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaStreamSynchronize(s));
         const int shared_quot = (md.shared_quot && !h_uncertified) ? 1 : 0;
@@ -1530,7 +1533,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             const int gb = short_grid(N, 256);
             unsigned *uncertified = (unsigned *)((unsigned long long *)e->work.p + 2);  // zeroed above
             k_bin_keys<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (unsigned *)e->ehash.p,
-                                          (unsigned *)e->bcount.p, err, uncertified, dd);
+                                          (unsigned *)e->bcount.p, err, uncertified, unfit_of(e), dd);
             CVL_TRY(check_launch("k_bin_keys"));
             CVL_TRY((scan<unsigned, unsigned>(e, (const unsigned *)e->bcount.p, T, (unsigned *)e->bstart.p)));
             k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, N, d_map_off, cap.M, md, (const unsigned *)e->ehash.p,
@@ -1617,7 +1620,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 fa.over_cnt = queues + 1;
                 fa.over_queue = queues + 2;
                 fa.over_list = (int *)e->deg.p;
-                fa.uncertified = uncertified;  // a run outside the certified angles goes kernel by kernel
+                fa.unfit = unfit_of(e);  // a run outside the certified angles goes kernel by kernel
                 CVL_TRY(launch_curvelets(e, fa, sms * FAST_BLOCKS, sms * FAST_EXACT_BLOCKS));
             }
             for (int c = 0; c < (fm.ok ? 0 : cap.K); ++c) {

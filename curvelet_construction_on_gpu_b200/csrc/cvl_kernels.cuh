@@ -35,13 +35,14 @@ constexpr int MAPS_SMEM = 256;  // per-block map statistics kept in shared memor
 constexpr double CVL_PI = 3.14159265358979323846;  // curvelet_utils.hpp:10
 
 // Error bits raised by kernels (checked by the host after a run).
-// a run's certification flag: bit 0, an operand outside certify_*'s ranges; bit 1, an
-// orientation beyond +-1024 rad, where the enclosures of cvl_curvelets.cuh do not hold
-constexpr unsigned UNCERT_ANGLE = 2u;
 constexpr unsigned ERR_NONFINITE = 1u;   // non-finite or out-of-range coordinate
 constexpr unsigned ERR_CAPACITY = 2u;    // a device capacity was exceeded
 constexpr unsigned ERR_INTERNAL = 4u;    // an internal invariant failed (bounds check)
 constexpr unsigned ERR_ARENA = 8u;       // the record arena was too small (the host resizes and reruns)
+
+// Why k_curvelets cannot take a run (a word of its own: what sends a run to the two-kernel path
+// does not change how that path forms its quotients, which the certification flag decides).
+constexpr unsigned UNFIT_ANGLE = 1u;  // an orientation beyond +-1024 rad, where the enclosures do not hold
 
 // T is the path's scalar type: double (run_curvelet<double>) or float (the
 // reference's --float mode, run_curvelet<float>, main.cpp:110). In float mode
@@ -292,7 +293,7 @@ __device__ __forceinline__ int map_of(const int *map_off, int M, int e) {
 template <typename T>
 __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int *__restrict__ map_off, int M,
                            ModelT<T> md, unsigned *__restrict__ ehash, unsigned *__restrict__ bcount,
-                           unsigned *__restrict__ err, unsigned *__restrict__ uncertified,
+                           unsigned *__restrict__ err, unsigned *__restrict__ uncertified, unsigned *__restrict__ unfit,
                            const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
@@ -308,10 +309,8 @@ __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int
             atomicAdd(&bcount[0], 1u);
             continue;
         }
-        if (uncertified) {
-            const unsigned un = (certify_coord(x) && certify_coord(y) ? 0u : 1u) | (fabs(th) <= T(1024) ? 0u : UNCERT_ANGLE);
-            if (un) atomicOr(uncertified, un);
-        }
+        if (uncertified && !(certify_coord(x) && certify_coord(y))) atomicOr(uncertified, 1u);
+        if (!(fabs(th) <= T(1024))) atomicOr(unfit, UNFIT_ANGLE);
         const int m = map_of(map_off, M, e);
         const int cx = lrint_dev(x);  // lrint, round half to even (preprocess.hpp:85-86)
         const int cy = lrint_dev(y);
