@@ -477,12 +477,11 @@ struct FastCounts {
 // ---------------------------------------------------------------------------
 template <bool QUEUE>
 __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(const __grid_constant__ FastArgs a) {
-    if (*a.err & ERR_NONFINITE) return;  // no rows (cvl_search.cuh)
     extern __shared__ __align__(16) unsigned char cv_smem[];
     using Smem = FastSmem<FAST_CAP, FAST_SLOTS>;
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (*a.unfit & UNFIT_ANGLE) {  // the host runs the two-kernel path instead
+    if (*a.unfit) {  // no rows; the host runs the two-kernel path instead, or fails
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, ERR_CAPACITY);
         return;
     }
@@ -819,12 +818,11 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
 // per lane. It takes the same comparisons and settles the undecided ones in FP64.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_EXACT_BLOCKS) k_curvelets_exact(const __grid_constant__ FastArgs a) {
-    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char cv_smem[];
     constexpr int SLOTS = FAST_WIDE_SLOTS;
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (*a.unfit & UNFIT_ANGLE) return;
+    if (*a.unfit) return;
     const int n_over = (int)*a.over_cnt;
     if ((int)blockIdx.x * FAST_WARPS >= n_over) return;
     FastBlockSmem &T = *(FastBlockSmem *)cv_smem;

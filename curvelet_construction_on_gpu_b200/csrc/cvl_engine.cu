@@ -1043,7 +1043,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     k_bin_scatter<<<gb, 256, 0, s>>>(d_edges, sz, n, d_map_off, M, md, (const unsigned *)e->ehash.p,
                                      (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B, rec_out, (int *)e->pos_of.p,
                                      F.e, F.cs2, F.at, pair_cap ? (unsigned *)e->deg.p : nullptr,
-                                     (unsigned *)((unsigned long long *)e->work.p + 5), search_item(n), nullptr);
+                                     (unsigned *)((unsigned long long *)e->work.p + 5), search_item(n), unfit_of(e), nullptr);
     CVL_TRY(check_launch("k_bin_scatter"));
     e->mark("bin");
 
@@ -1540,7 +1540,8 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                                              (const unsigned *)e->bstart.p, (unsigned *)e->bcount.p, B,
                                              fm.ok ? (double2 *)e->rec_k.p : nullptr, (int *)e->pos_of.p, F.e, F.cs2, F.at,
                                              fm.ok ? (unsigned *)e->deg.p : nullptr,
-                                             (unsigned *)((unsigned long long *)e->work.p + 5), search_item(N), dd);
+                                             (unsigned *)((unsigned long long *)e->work.p + 5), search_item(N), unfit_of(e),
+                                             dd);
             CVL_TRY(check_launch("k_bin_scatter"));
             NbArgsT<double> na{};
             na.md = md;

@@ -40,9 +40,11 @@ constexpr unsigned ERR_CAPACITY = 2u;    // a device capacity was exceeded
 constexpr unsigned ERR_INTERNAL = 4u;    // an internal invariant failed (bounds check)
 constexpr unsigned ERR_ARENA = 8u;       // the record arena was too small (the host resizes and reruns)
 
-// Why k_curvelets cannot take a run (a word of its own: what sends a run to the two-kernel path
-// does not change how that path forms its quotients, which the certification flag decides).
-constexpr unsigned UNFIT_ANGLE = 1u;  // an orientation beyond +-1024 rad, where the enclosures do not hold
+// Why k_search and k_curvelets cannot take a run: k_bin_keys' verdict, before they start (a word
+// of its own: what sends a run to the two-kernel path does not change how that path
+// forms its quotients, which the certification flag decides).
+constexpr unsigned UNFIT_ANGLE = 1u;      // an orientation beyond +-1024 rad, where the enclosures do not hold
+constexpr unsigned UNFIT_NONFINITE = 2u;  // ERR_NONFINITE
 
 // T is the path's scalar type: double (run_curvelet<double>) or float (the
 // reference's --float mode, run_curvelet<float>, main.cpp:110). In float mode
@@ -305,6 +307,7 @@ __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int
         const T th = edges[(size_t)e * sz + 2];
         if (!isfinite(x) || !isfinite(y) || !isfinite(th) || fabs(x) >= T(1.0e9) || fabs(y) >= T(1.0e9)) {
             atomicOr(err, ERR_NONFINITE);
+            atomicOr(unfit, UNFIT_NONFINITE);
             ehash[e] = 0;
             atomicAdd(&bcount[0], 1u);
             continue;
@@ -326,17 +329,19 @@ __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const 
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
                               double2 *__restrict__ rec, int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
                               int4 *__restrict__ at, unsigned *__restrict__ items, unsigned *__restrict__ item_cnt,
-                              unsigned item_size,
+                              unsigned item_size, const unsigned *__restrict__ unfit,
                               const RunDims *__restrict__ dims) {
     if (dims) {
         N = dims->N;
         M = dims->M;
     }
+    // (k_search takes nothing of a run it cannot take, and the wide list stays empty)
+    const bool list = items && *unfit == 0u;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
         const unsigned h = ehash[e];
         const unsigned left = atomicSub(&bcount[h], 1u);  // (the counts are not needed any more)
         const unsigned pos = bstart[h] + left - 1u;
-        if (items && ((left - 1u) & (item_size - 1u)) == 0u) items[atomicAdd(item_cnt, 1u)] = pos;  // k_search's
+        if (list && ((left - 1u) & (item_size - 1u)) == 0u) items[atomicAdd(item_cnt, 1u)] = pos;  // k_search's
         const T x = edges[(size_t)e * sz + 0];
         const T y = edges[(size_t)e * sz + 1];
         const T th = edges[(size_t)e * sz + 2];

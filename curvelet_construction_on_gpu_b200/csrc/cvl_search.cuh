@@ -10,10 +10,11 @@
 // coalesced run, a lane per pair, each with its rank by (distance, scan order) in its
 // anchor's column and its classes.
 //
-// A run with a non-finite edge fails (ERR_NONFINITE, final since k_bin_keys), and no kernel
-// from here on may read what it left: k_bin_keys puts such an edge into bucket 0, whatever its
-// cell, so an item that it heads has another bucket's end, its neighbours' distances have no
-// order, and rows stay unwritten. k_search, k_search_wide, k_curvelets and k_curvelets_exact
+// A run with a non-finite edge fails (ERR_NONFINITE, final since k_bin_keys), and nothing from
+// here on may read what it left: k_bin_keys puts such an edge into bucket 0, whatever its
+// cell, so an item that it heads would have another bucket's end, its neighbours' distances
+// have no order, and rows would stay unwritten. k_bin_scatter lists no items of such a run, nor
+// of one whose orientations k_curvelets cannot take, and k_curvelets and k_curvelets_exact
 // leave at once. (On finite edges an item's head has its bucket's hash, and no item crosses it.)
 //
 // Rows are in no order, so the search needs no counting pass, no scan of the degrees and
@@ -69,7 +70,8 @@ struct SearchArgs {
     unsigned *err;
     unsigned *wide_cnt;               // anchors for k_search_wide
     int *wide_list;                   // [N]: an anchor is of one item, and is listed once
-    const unsigned *items;            // each run of up to item_size anchors of a bucket, by its first (k_bin_scatter)
+    const unsigned *items;            // each run of up to item_size anchors of a bucket, by its first (k_bin_scatter;
+                                      // none where *unfit)
     const unsigned *item_cnt;
     float scale;                      // 65,000 over the longest pair's d2 (rounding and truncation keep d2's order)
     unsigned item_size;               // a power of two, at most 32
@@ -121,7 +123,6 @@ struct SearchCounts {
 };
 
 __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(const __grid_constant__ SearchArgs a) {
-    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char se_smem[];
     SearchSmem &S = ((SearchSmem *)se_smem)[threadIdx.x >> 5];
     const Model &md = a.md;
@@ -295,7 +296,6 @@ __global__ void __launch_bounds__(SEARCH_WARPS * 32, SEARCH_BLOCKS) k_search(con
 // The anchors k_search left, a warp each: their candidates counted, then gathered and ranked
 // as k_nb<FILL> does.
 __global__ void __launch_bounds__(256) k_search_wide(const __grid_constant__ SearchArgs a) {
-    if (*a.err & ERR_NONFINITE) return;
     extern __shared__ __align__(16) unsigned char sw_smem[];
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;

@@ -2,8 +2,8 @@
 bucket in runs of at most item_size anchors, and k_search ends an item at its head's
 bucket, which it hashes from the head's pixel cell. A non-finite edge lies in bucket 0
 whatever its cell, so an item that it heads would take other buckets' anchors, each of them
-twice (and the wide ones past the end of their list), or none: the kernels that read items,
-rows and lists leave a run that holds one before they read any of them."""
+twice (and the wide ones past the end of their list), or none: no items are listed of a run
+that holds one, and the curvelet kernels leave it before they read its rows."""
 import os
 import re
 
@@ -63,14 +63,21 @@ def test_a_non_finite_head_breaks_the_items(item_size, cell):
     assert any(np.any(_processed(cells, finite, item_size, seed=s) != 1) for s in range(200))
 
 
-@pytest.mark.parametrize("file,kernel", [("cvl_search.cuh", "k_search"), ("cvl_search.cuh", "k_search_wide"),
-                                         ("cvl_curvelets.cuh", "k_curvelets"),
-                                         ("cvl_curvelets.cuh", "k_curvelets_exact")])
-def test_the_kernels_leave_such_a_run_first(file, kernel):
+def _kernel(file, name):
     with open(os.path.join(CSRC, file)) as f:
-        src = f.read()
-    body = re.search(r"__global__ void[^;{]*\b" + kernel + r"\([^{]*\)\s*\{(.*?)\n\}\n", src, re.S).group(1)
-    guard = re.search(r"if \(\*a\.err & ERR_NONFINITE\) return;", body)
-    assert guard, "no early return"
-    reads = re.search(r"a\.(items|item_cnt|wide_list|wide_cnt|over_list|over_cnt|row|at|e|F)\b", body)
-    assert guard.start() < reads.start()
+        return re.search(r"__global__ void[^;{]*\b" + name + r"\([^{]*\)\s*\{(.*?)\n\}\n", f.read(), re.S).group(1)
+
+
+def test_no_items_are_listed_of_such_a_run():
+    keys, scatter = _kernel("cvl_kernels.cuh", "k_bin_keys"), _kernel("cvl_kernels.cuh", "k_bin_scatter")
+    assert re.search(r"!isfinite\(x\)[^}]*atomicOr\(unfit, UNFIT_NONFINITE\)[^}]*continue;", keys)
+    assert "const bool list = items && *unfit == 0u;" in scatter
+    assert re.findall(r"if \((.*)\) items\[", scatter)[0].startswith("list && ")
+
+
+@pytest.mark.parametrize("kernel", ["k_curvelets", "k_curvelets_exact"])
+def test_the_curvelet_kernels_leave_such_a_run_first(kernel):
+    body = _kernel("cvl_curvelets.cuh", kernel)
+    guard = re.search(r"if \(\*a\.unfit\) (return;|\{[^}]*return;)", body)
+    reads = re.search(r"a\.(over_list|over_cnt|over_queue|row|csr_ids|F|B)\b", body)
+    assert guard and guard.start() < reads.start()
