@@ -57,8 +57,9 @@
 //   e1 >= (fN + max_k fE) / (e0 - 12u max_k),  |D| >= (eps + max_k fD) / (e0 - 12u max_k).
 // (2^-27 and 2^-30 for the default parameters and orientations within a turn.)
 // The FP64 path's own rounding (2^-50 of these magnitudes), the addition theorem on
-// its rounded angles (|theta| <= 2^10, checked when binning: 2^-41) and higher orders
-// of u are covered by 2% on Ethr, Dthr and S1.
+// its rounded angles (|theta| <= FAST_ANGLE = 2^20, checked when binning: 2^-31, against 4u
+// = 2^-22 in s and likewise in the others) and higher orders of u are covered by 2% on
+// Ethr, Dthr and S1.
 // Bounds are kept as (n, M): n the negated lower one, so that an intersection takes the
 // smaller of both, and a cell is open when M + n > 0. With h = 2.04 e0,
 //   min M + min n >  h       every bound considered, the cell is open;
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(FAST_WARPS * 32, FAST_BLOCKS) k_curvelets(cons
     const Model &md = a.md;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (*a.unfit) {  // no rows; the host runs the two-kernel path instead, or fails
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, ERR_CAPACITY);
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.err, ERR_ANGLE);
         return;
     }
     FastBlockSmem &T = *(FastBlockSmem *)cv_smem;

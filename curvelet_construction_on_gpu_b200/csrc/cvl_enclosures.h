@@ -10,6 +10,9 @@ namespace cvl {
 
 constexpr int FAST_P = 9;        // grid offsets of the column code (the default grid)
 constexpr int FAST_WIDE = 128;   // pairs of an anchor (max_candidates <= 128)
+// Orientations the enclosures hold for (rad): the reference's rounding of its angles is 2^-31
+// there, 0.2% and less of what single precision leaves of the quantities they enter.
+constexpr double FAST_ANGLE = 0x1p20;
 // e0 / max_k: larger leaves more comparisons undecided, smaller more columns to be made anew
 // (2^-13 to 2^-15 measured alike)
 constexpr double FAST_E0 = 0x1p-14;

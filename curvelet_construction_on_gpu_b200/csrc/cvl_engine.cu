@@ -547,6 +547,7 @@ struct RunOut {
     unsigned long long total_pairs = 0;
     unsigned long long total_curvelets = 0;
     unsigned max_deg = 0;
+    bool wide_angles = false;  // the fused path gave the run up for its orientations (ERR_ANGLE)
 };
 
 template <typename T, int CPL, int MINB>
@@ -800,10 +801,12 @@ int launch_finalize(cvl_engine *e, const FinalArgs &f, int n) {
     return check_launch("k_finalize_exact");
 }
 
-// A run's error bits: CVL_EAGAIN where the two-pass search, or the two-kernel path, is to run.
-int fast_status(unsigned h_err) {
+// A run's error bits: CVL_EAGAIN where the two-pass search, or (wide_angles) the two-kernel
+// path, is to run.
+int fast_status(unsigned h_err, RunOut &ro) {
     if (h_err & ERR_NONFINITE) return fail(CVL_EINVAL, "non-finite or out-of-range (|v| >= 1e9) edge coordinate");
-    if (h_err & ERR_CAPACITY) return CVL_EAGAIN;
+    ro.wide_angles = (h_err & ERR_ANGLE) != 0;
+    if (h_err & (ERR_CAPACITY | ERR_ANGLE)) return CVL_EAGAIN;
     if (h_err) return fail(CVL_EOVERFLOW, "kernel reported error bits " + std::to_string(h_err));
     return CVL_OK;
 }
@@ -900,7 +903,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
             CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
             e->mark("end");
             CVL_CUDA(cudaStreamSynchronize(s));
-            CVL_TRY(fast_status(h_err));
+            CVL_TRY(fast_status(h_err, ro));
             fast_totals(ro);
             return CVL_OK;
         }
@@ -917,7 +920,7 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
         CVL_CUDA(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaMemcpyAsync(&used, work, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
         CVL_CUDA(cudaStreamSynchronize(s));
-        if (!(h_err & ERR_ARENA) || (h_err & ~ERR_ARENA)) CVL_TRY(fast_status(h_err));
+        if (!(h_err & ERR_ARENA) || (h_err & ~ERR_ARENA)) CVL_TRY(fast_status(h_err, ro));
         if ((h_err & ERR_ARENA) && attempt == 0) {
             // the record arena was too small: size it to what this input needs and grow the
             // chains again (valid and close pairs are recounted from zero)
@@ -941,11 +944,13 @@ int run_fast_chunks(cvl_engine *e, const FastModel &fm, const FastBinned &F, con
 }
 
 // mode: 0 = full run, 1 = count valid pairs only, 2 = neighbour graph only
-// two_pass: count and fill the neighbour lists even where the one-pass search could serve.
+// route: TWO_PASS counts and fills the neighbour lists even where the one-pass search could
+// serve; TWO_KERNEL makes bundles and chains in two kernels, too.
+enum class Route { ANY, TWO_PASS, TWO_KERNEL };
 template <typename R>
 int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const int *d_map_off,
                  const std::vector<int32_t> &map_off_host, ModelT<R> md, int cpl, int mode, bool want_d2,
-                 RunOut &ro, bool two_pass = false) {
+                 RunOut &ro, Route route = Route::ANY) {
     const int M = (int)map_off_host.size() - 1;
     cudaStream_t s = e->stream;
     // one NVTX range per run on the host timeline, a mark at each stage's end
@@ -965,13 +970,13 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     const bool path = (mode != 2);
     FastModel fm{};
     if constexpr (std::is_same<R, double>::value) {
-        if (path && e->enclosures_on) fm = make_fast(md);
+        if (path && e->enclosures_on && route != Route::TWO_KERNEL) fm = make_fast(md);
     }
     // The one-pass search's pairs go to the buffers as they are, or to new ones of 32 per edge
     // (the workloads' mean is 7 to 22; 160 bytes per edge); a run they do not hold, or that
     // has no room for them, counts first.
     unsigned long long pair_cap = 0;
-    if (fm.ok && !two_pass && search_serves(md)) {
+    if (fm.ok && route == Route::ANY && search_serves(md)) {
         pair_cap = std::min<unsigned long long>(e->csr_ids.bytes / sizeof(int), e->pcls.bytes);
         if (pair_cap < 4ull * (unsigned long long)n) {
             pair_cap = 32ull * (unsigned long long)n;
@@ -1063,12 +1068,13 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
             ro.stats.assign(M, MapStats{});
             const int rc = run_fast_chunks(e, fm, F, FB, md, n, M, d_map_off, map_off_host, mode, tn, false, ro);
             if (rc != CVL_EAGAIN) return rc;
-            // the two passes, or once more with the pairs' own count of room
+            // the two kernels, the two passes, or once more with the pairs' own count of room
             unsigned long long need = 0;
             for (const MapStats &st : ro.stats) need += st.pairs;
+            Route next = ro.wide_angles ? Route::TWO_KERNEL : Route::TWO_PASS;
             if (need > pair_cap && e->alloc(e->csr_ids, sizeof(int) * need) == CVL_OK && e->alloc(e->pcls, need) == CVL_OK)
-                return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, false);
-            return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, true);
+                next = Route::ANY;
+            return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, next);
         }
     }
 
@@ -1420,7 +1426,7 @@ size_t graph_readback_bytes() {
 // CVL_OK with ro filled; CVL_EAGAIN when the run is not for a graph or did not fit
 // (the caller runs the direct path); another status on a real error.
 int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, const int *d_map_off,
-                       const std::vector<int32_t> &map_off_host, Model md, int cpl, RunOut &ro) {
+                       const std::vector<int32_t> &map_off_host, Model md, int cpl, Route route, RunOut &ro) {
     const int M = (int)map_off_host.size() - 1;
     const int b = bucket_of(n);
     if (!e->graphs_on || g_sync_check || b > 1) return CVL_EAGAIN;
@@ -1442,7 +1448,8 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     sh.edge_data_sz = sz;
     // (the input rows and map offsets are the caller's, already in place: they are
     // not reallocated here)
-    const FastModel fm = e->enclosures_on && search_serves(md) ? make_fast(md) : FastModel{};
+    const FastModel fm =
+        e->enclosures_on && route != Route::TWO_KERNEL && search_serves(md) ? make_fast(md) : FastModel{};
     if (fm.ok) md.sbits = SEARCH_SBITS;
     for (const WsItem &w : workspace_plan(e->tune, e->arena_hint, md, cpl, sh)) {
         if (w.buf == &cvl_engine::edges || w.buf == &cvl_engine::map_off) continue;
@@ -1733,7 +1740,8 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     const unsigned h_err = *err_h;
     if (h_err & ERR_NONFINITE) return fail(CVL_EINVAL, "non-finite or out-of-range (|v| >= 1e9) edge coordinate");
     const unsigned long long P = rb_h[0], C = rb_h[1];
-    if ((h_err & (ERR_CAPACITY | ERR_ARENA)) || C > C_cap) {
+    if ((h_err & (ERR_CAPACITY | ERR_ARENA | ERR_ANGLE)) || C > C_cap) {
+        ro.wide_angles = (h_err & ERR_ANGLE) != 0;
         ++e->graph_fallbacks;
         return CVL_EAGAIN;
     }
@@ -1777,18 +1785,25 @@ std::vector<WsItem> workspace_plan_with_graphs(const cvl_tuning *tune, unsigned 
     return v;
 }
 
-// The path: a bucket's graph where the run fits one, else the kernels launched one by one.
+// The path: a bucket's graph where the run fits one, else the kernels launched one by one. A run
+// whose orientations the enclosures do not hold for replays the two-kernel path's graph
+// then (517 edges: 203 us host to host, against 569 kernel by kernel).
 template <typename R>
 int run_pipeline(cvl_engine *e, const R *d_edges, int n, int sz, const int *d_map_off,
                  const std::vector<int32_t> &map_off_host, ModelT<R> md, int cpl, int mode, bool want_d2,
                  RunOut &ro) {
+    Route route = Route::ANY;
     if constexpr (std::is_same<R, double>::value) {
         if (mode == 0 && !want_d2) {
-            const int rc = run_pipeline_graph(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, ro);
+            int rc = run_pipeline_graph(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, route, ro);
+            if (rc == CVL_EAGAIN && ro.wide_angles) {
+                route = Route::TWO_KERNEL;
+                rc = run_pipeline_graph(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, route, ro);
+            }
             if (rc != CVL_EAGAIN) return rc;
         }
     }
-    return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro);
+    return run_pipeline_direct(e, d_edges, n, sz, d_map_off, map_off_host, md, cpl, mode, want_d2, ro, route);
 }
 
 template <typename T>

@@ -26,6 +26,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "cvl_enclosures.h"
+
 namespace cvl {
 
 constexpr unsigned FULL = 0xffffffffu;
@@ -39,11 +41,12 @@ constexpr unsigned ERR_NONFINITE = 1u;   // non-finite or out-of-range coordinat
 constexpr unsigned ERR_CAPACITY = 2u;    // a device capacity was exceeded
 constexpr unsigned ERR_INTERNAL = 4u;    // an internal invariant failed (bounds check)
 constexpr unsigned ERR_ARENA = 8u;       // the record arena was too small (the host resizes and reruns)
+constexpr unsigned ERR_ANGLE = 16u;      // UNFIT_ANGLE (the host runs the two-kernel path)
 
 // Why k_search and k_curvelets cannot take a run: k_bin_keys' verdict, before they start (a word
 // of its own: what sends a run to the two-kernel path does not change how that path
 // forms its quotients, which the certification flag decides).
-constexpr unsigned UNFIT_ANGLE = 1u;      // an orientation beyond +-1024 rad, where the enclosures do not hold
+constexpr unsigned UNFIT_ANGLE = 1u;      // an orientation beyond +-FAST_ANGLE, where the enclosures do not hold
 constexpr unsigned UNFIT_NONFINITE = 2u;  // ERR_NONFINITE
 
 // T is the path's scalar type: double (run_curvelet<double>) or float (the
@@ -313,7 +316,7 @@ __global__ void k_bin_keys(const T *__restrict__ edges, int sz, int N, const int
             continue;
         }
         if (uncertified && !(certify_coord(x) && certify_coord(y))) atomicOr(uncertified, 1u);
-        if (!(fabs(th) <= T(1024))) atomicOr(unfit, UNFIT_ANGLE);
+        if (!(fabs(th) <= T(FAST_ANGLE))) atomicOr(unfit, UNFIT_ANGLE);
         const int m = map_of(map_off, M, e);
         const int cx = lrint_dev(x);  // lrint, round half to even (preprocess.hpp:85-86)
         const int cy = lrint_dev(y);

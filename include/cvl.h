@@ -540,7 +540,8 @@ int cvl_engine_memory_get(cvl_engine *e, cvl_engine_memory *out);
  * one host synchronisation where the kernel-by-kernel path has three. A graph is
  * captured on a bucket's first run and again when the parameters, the tuning or
  * the buffers change (up to 6 kept per engine). A run beyond a capacity is
- * flagged on the device and run again kernel by kernel; the results are the same
+ * flagged on the device and run again kernel by kernel (one with an orientation beyond
+ * 2^20 rad by the graph of the two-kernel path); the results are the same
  * either way. CVL_NO_GRAPHS in the environment turns graphs off for new engines. */
 int cvl_engine_set_graphs(cvl_engine *e, int enable);
 typedef struct cvl_engine_graphs {
@@ -548,7 +549,7 @@ typedef struct cvl_engine_graphs {
     int32_t graphs;      /* captured graphs held */
     uint64_t captures;   /* graphs captured so far */
     uint64_t replays;    /* runs that replayed a graph */
-    uint64_t fallbacks;  /* of those, runs beyond a capacity, run again kernel by kernel */
+    uint64_t fallbacks;  /* of those, runs beyond a capacity or an angle, run again */
 } cvl_engine_graphs;
 int cvl_engine_graph_stats(cvl_engine *e, cvl_engine_graphs *out);
 

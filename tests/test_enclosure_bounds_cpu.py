@@ -141,12 +141,13 @@ SETS = [dict(), dict(max_k=3.0), dict(dx=0.36), dict(dx=0.8, sx=0.2, nrad=5.0, w
         dict(nrad=3.5, rad=8.0, w=2), dict(nrad=3.5, rad=8.0, w=8, max_k=0.05)]
 
 
+@pytest.mark.parametrize("turns", [0, 166_000])  # orientations up to 1.04e6 rad: FAST_ANGLE is 2^20
 @pytest.mark.parametrize("over", SETS, ids=lambda o: "-".join(f"{k}{v}" for k, v in o.items()) or "default")
-def test_columns(shim, over):
+def test_columns(shim, over, turns):
     m, f, R = _model(shim, **over)
     assert f.ok
     rng = np.random.default_rng(17)
-    DX, DY, T2, T0, i, j = _pairs(rng, m, R, 1_500_000, 0)
+    DX, DY, T2, T0, i, j = _pairs(rng, m, R, 1_500_000 if turns == 0 else 300_000, turns)
     sT, cT = (_r(x) for x in _trig(m, T2, j))
     d = _r(_offset(m.sx, i, m.P))
     X, Y = _r(DX), _r(DY)
@@ -169,7 +170,7 @@ def test_columns(shim, over):
     _check(m, _want(m, DX, DY, T2, T0, i, j), got, ok)
 
 
-@pytest.mark.parametrize("turns", [0, 1, 16, 160])
+@pytest.mark.parametrize("turns", [0, 1, 16, 160, 166_000])
 @pytest.mark.parametrize("over", SETS + [dict(max_k=0.002), dict(max_k=2.0 ** -10), dict(max_k=1000.0),
                                          dict(rad=1e6, w=64, max_k=0.002), dict(dx=0.36, max_k=2.0 ** -10),
                                          dict(dx=7.2, sx=2.0, max_k=0.002, nrad=30.0, w=30)],

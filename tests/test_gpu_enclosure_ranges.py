@@ -68,7 +68,7 @@ def _map(kind):
     return _scatter(20000, 220, 8)
 
 
-@pytest.mark.parametrize("turns", [0, 16, 159])  # orientations within 2 pi, about 100 and about 1000 rad
+@pytest.mark.parametrize("turns", [0, 16, 159, 166000])  # orientations within 2 pi, of about 100, 1000 and 1e6 rad
 @pytest.mark.parametrize("over", [dict(), dict(max_k=0.002), dict(max_k=2.0 ** -10), dict(max_k=900.0), dict(dx=0.36),
                                   dict(dx=0.36, max_k=2.0 ** -10), dict(nrad=60.0)],
                          ids=lambda o: "-".join(f"{k}{v:g}" for k, v in o.items()) or "default")
@@ -81,3 +81,29 @@ def test_angles_and_curvatures(engines, kind, over, turns):
     r = fused.run(e, p)
     _assert_fused(fused)
     _same(r, fp64.run(e, p))
+
+
+@pytest.mark.parametrize("edges", [517, None])  # both graphs' buckets
+def test_orientations_out_of_range(engines, edges):
+    """Beyond 2^20 rad the two-kernel path runs, by its own graph where graphs are on."""
+    direct, fp64 = engines
+    e = (synth.plain_small(3)[:edges] if edges else synth.plain_hd(1000)).copy()
+    e[len(e) // 2, 2] += 2 * np.pi * 400_000
+    want = fp64.run(e)
+    _same(direct.run(e), want)
+    assert "bundles" in _stages(direct)
+    g = direct.build_neighbor_graph(e)
+    assert direct.form_pairwise_bundles(g, cvl.CurveletParams()) == want.valid_pairs
+    with cvl.Engine() as eng:
+        for k in range(1, 4):
+            _same(eng.run(e), want)
+            assert _stages(eng) <= {"graph", "start"}, _stages(eng)
+            st = eng.graph_stats()
+            assert (st["replays"], st["fallbacks"]) == (2 * k, k)
+        assert st["captures"] == 3  # (the second graph's buffers make the first be captured again, once)
+        plain = e[: len(e) // 2]
+        _same(eng.run(plain), fp64.run(plain))  # the next run is not held back
+        assert eng.graph_stats()["replays"] == 7
+        a, b = eng.run_maps([plain, e])
+        _same(a, fp64.run(plain))
+        _same(b, want)
