@@ -179,6 +179,7 @@ struct cvl_engine {
     bool served = false;  // a server's engine: others run beside it (copy_result_to_host)
     // decisions on single-precision enclosures (CVL_NO_ENCLOSURES: every bundle in FP64)
     bool enclosures_on = std::getenv("CVL_NO_ENCLOSURES") == nullptr;
+    unsigned long long reserved_edges = 0;         // of the largest shape cvl_engine_reserve_workspace set aside
     uint64_t ws_epoch = 0;                         // workspace (re)allocations so far
     uint64_t graph_replays = 0, graph_fallbacks = 0, graph_captures = 0, graph_clock = 0;
     DBuf gdims, gchunks;
@@ -224,6 +225,32 @@ struct cvl_engine {
         held += want;
         ++ws_epoch;
         return CVL_OK;
+    }
+
+    void release(DBuf &b) {
+        if (b.p) cudaFreeAsync(b.p, stream);
+        held -= b.bytes;
+        b.p = nullptr;
+        b.bytes = 0;
+    }
+
+    // Room for the one-pass search's pairs of a run of n edges: the buffers as they are, or new
+    // ones of 32 pairs per edge (the workloads' mean is 7 to 22; 160 bytes per edge) where those
+    // hold fewer than 4 per edge. Runs within a reserved shape take what it set aside, and
+    // so do runs whose budget has no room for more: a run that does not fit is counted and run
+    // again. 0: no buffers.
+    unsigned long long pair_room(unsigned long long n) {
+        auto room = [&] { return std::min<unsigned long long>(csr_ids.bytes / sizeof(int), pcls.bytes); };
+        if (room() >= 4 * n || (room() && n <= reserved_edges)) return room();
+        const size_t ids = sizeof(int) * 32 * n, cls = 32 * n;
+        if (budget && held - csr_ids.bytes - pcls.bytes + std::max(ids, csr_ids.bytes) + std::max(cls, pcls.bytes) > budget)
+            return room();
+        if (alloc(csr_ids, ids) != CVL_OK) return 0;
+        if (alloc(pcls, cls) != CVL_OK) {
+            release(csr_ids);  // (the two passes need the memory)
+            return 0;
+        }
+        return room();
     }
 
     void mark(const char *name) {
@@ -972,18 +999,9 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
     if constexpr (std::is_same<R, double>::value) {
         if (path && e->enclosures_on && route != Route::TWO_KERNEL) fm = make_fast(md);
     }
-    // The one-pass search's pairs go to the buffers as they are, or to new ones of 32 per edge
-    // (the workloads' mean is 7 to 22; 160 bytes per edge); a run they do not hold, or that
-    // has no room for them, counts first.
+    // (a run whose pairs the one-pass search has no room for counts first)
     unsigned long long pair_cap = 0;
-    if (fm.ok && route == Route::ANY && search_serves(md)) {
-        pair_cap = std::min<unsigned long long>(e->csr_ids.bytes / sizeof(int), e->pcls.bytes);
-        if (pair_cap < 4ull * (unsigned long long)n) {
-            pair_cap = 32ull * (unsigned long long)n;
-            if (e->alloc(e->csr_ids, sizeof(int) * pair_cap) != CVL_OK || e->alloc(e->pcls, pair_cap) != CVL_OK)
-                pair_cap = 0;
-        }
-    }
+    if (fm.ok && route == Route::ANY && search_serves(md)) pair_cap = e->pair_room((unsigned long long)n);
     if (pair_cap) md.sbits = SEARCH_SBITS;
 
     // ---- workspace for N-sized arrays
@@ -2519,6 +2537,7 @@ int cvl_engine_reserve_workspace(cvl_engine *e, const cvl_workspace_shape *s, co
     e->arena_hint = std::max<unsigned long long>(e->arena_hint, (unsigned long long)s->num_curvelets);
     for (const WsItem &w : workspace_plan_with_graphs(e->tune, e->arena_hint, md, cpl, *s, e->graphs_on))
         CVL_TRY(e->alloc(e->*(w.buf), w.bytes));
+    e->reserved_edges = std::max(e->reserved_edges, (unsigned long long)s->num_edges);
     if (e->graphs_on && !e->gread_host) {  // the graphs' page-locked readback
         void *h = nullptr;
         if (cvl_alloc_fault_injected() || cudaMallocHost(&h, graph_readback_bytes() + sizeof(RunDims) + 64) != cudaSuccess) {
