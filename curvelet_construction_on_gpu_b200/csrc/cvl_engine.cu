@@ -1507,7 +1507,9 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
     const unsigned long long nums[] = {(unsigned long long)b, (unsigned long long)sz, (unsigned long long)cpl,
                                        e->ws_epoch, arena_cap, per_chunk, (unsigned long long)fm.ok};
     key.append((const char *)nums, sizeof(nums));
-    key.append((const char *)&tn, sizeof(tn));
+    const long long knobs[] = {tn.cell_size,     tn.bundle_blocks_per_sm, tn.growth_blocks_per_sm,
+                               tn.seeds_per_group, tn.anchors_per_warp,   (long long)tn.chunk_pairs};
+    key.append((const char *)knobs, sizeof(knobs));
     cvl_engine::GraphSlot *slot = nullptr;
     for (auto &g : e->graphs)
         if (g.key == key) slot = &g;

@@ -69,7 +69,9 @@ struct ModelT {
     unsigned hash_mask;          // table size - 1
     int shared_quot;             // FP64 transport: the k_dx quotients on one reciprocal
                                  // (QUOT_SHARED) unless a run's operands fail certify_*
+    int pad = 0;                 // no byte unset: graphs are kept by a model's bytes
 };
+static_assert(sizeof(ModelT<double>) == 9 * sizeof(double) + 10 * sizeof(int), "padding in a graph's key");
 
 // Operands whose ranges give every nonzero e1 and k_dx numerator of the FP64
 // transport a magnitude in [2^-500, 2^501), the range in which the transport's
