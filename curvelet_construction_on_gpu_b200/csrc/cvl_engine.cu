@@ -2704,6 +2704,17 @@ int cvl_engine_autotune(cvl_engine *e, const cvl_batch *b, const cvl_params *p, 
                         double *best_ms) {
     if (!e || !b || !p || !best || !best_ms || passes < 1) return fail(CVL_EINVAL, "invalid autotune arguments");
     const int bucket = bucket_of(b->n);
+    // The knobs that the batch's path reads: timing another would only choose by noise, and
+    // chunk_pairs sets a graph's pair capacity besides. k_curvelets' runs read
+    // anchors_per_warp where they are neither a graph nor persistent, and chunk_pairs where they
+    // yield to others.
+    Model md;
+    int cpl = 2;
+    CVL_TRY(make_model(e, p, p->nrad, 3u, p->max_candidates, md, cpl));
+    const bool fused = e->enclosures_on && search_serves(md) && make_fast(md).ok;
+    const bool graph = e->graphs_on && bucket <= 1;
+    const bool reads_apw = !fused || (!graph && !persistent_chunks(e, b->n));
+    const bool reads_chunks = !fused || (!graph && e->yield_fn);
     // one untimed run (workspace growth), then the median of three device times
     auto time_it = [&](const cvl_tuning &t, double &ms) -> int {
         e->tune[bucket] = t;
@@ -2739,28 +2750,28 @@ int cvl_engine_autotune(cvl_engine *e, const cvl_batch *b, const cvl_params *p, 
         for (int v : {3, 4}) {
             cvl_tuning t = cur;
             t.bundle_blocks_per_sm = v;
-            CVL_TRY(consider(t));
+            if (!fused) CVL_TRY(consider(t));
         }
         for (const auto &g : growth) {
             cvl_tuning t = cur;
             t.seeds_per_group = g[0];
             t.growth_blocks_per_sm = g[1];
-            CVL_TRY(consider(t));
+            if (!fused) CVL_TRY(consider(t));
         }
         for (int v : apws) {
             cvl_tuning t = cur;
             t.anchors_per_warp = v;
-            CVL_TRY(consider(t));
+            if (reads_apw) CVL_TRY(consider(t));
         }
         for (int v : cells) {
             cvl_tuning t = cur;
             t.cell_size = v;
-            CVL_TRY(consider(t));
+            if (!fused) CVL_TRY(consider(t));
         }
         for (int64_t v : chunks) {
             cvl_tuning t = cur;
             t.chunk_pairs = v;
-            CVL_TRY(consider(t));
+            if (reads_chunks) CVL_TRY(consider(t));
         }
     }
     e->tune[bucket] = cur;

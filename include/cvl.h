@@ -471,10 +471,12 @@ int cvl_write_edges_binary(const char *path, const double *edges, int64_t num_ed
 /* ---- tuning and the autotuner -------------------------------------------
  * No reference counterpart. An engine keeps one tuning per size bucket of the
  * batch (its total edges); every tuning gives the same results bit for bit,
- * only the time changes. Double runs on the default grid make bundles and chains in one
- * kernel with a hash block of 8: there only anchors_per_warp and chunk_pairs matter, and
- * those only where a run yields to others. The other knobs are float runs' and other grids'. cvl_engine_autotune searches them on a
- * device-resident batch by timing the whole path, and installs the best. */
+ * only the time changes. Double runs on the default grid make bundles and chains in
+ * one kernel with a hash block of 8: there only anchors_per_warp (of up to 64 Ki
+ * edges without a graph, and where a run yields to others) and chunk_pairs (where it
+ * yields) matter. The other knobs are float runs' and other grids'.
+ * cvl_engine_autotune searches them on a device-resident batch by timing the whole
+ * path, and installs the best. */
 #define CVL_TUNING_BUCKETS 4          /* batches of <= 64 Ki, <= 512 Ki, <= 4 Mi, and more edges */
 typedef struct cvl_tuning {
     int cell_size;                    /* spatial-hash block edge in pixel cells: 2, 4 or 8 (4; 8 above 512 Ki edges) */
@@ -491,9 +493,9 @@ int cvl_engine_get_tuning(cvl_engine *e, int bucket, cvl_tuning *t);
 /* bucket -1 sets every bucket. CVL_EINVAL for values outside the ranges above. */
 int cvl_engine_set_tuning(cvl_engine *e, int bucket, const cvl_tuning *t);
 /* Coordinate descent over the tuning of the batch's bucket. It runs `passes`
- * sweeps over the knobs, each candidate timed as the median of 3 runs of the
- * whole path (device time), and keeps a change only when it is faster by more
- * than 1%. The best tuning is installed for that bucket and written to *best,
+ * sweeps over the knobs that the batch's path reads, each candidate timed as the
+ * median of 3 runs of the whole path (device time), and keeps a change only when it
+ * is faster by more than 1%. The best tuning is installed for that bucket and written to *best,
  * and its time to *best_ms. The batch's results are not kept. */
 int cvl_engine_autotune(cvl_engine *e, const cvl_batch *b, const cvl_params *p, int passes, cvl_tuning *best,
                         double *best_ms);
