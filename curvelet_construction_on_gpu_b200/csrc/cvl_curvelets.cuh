@@ -84,7 +84,7 @@ constexpr int FAST_WARPS = 4;
 constexpr int FAST_BLOCKS = 5;
 constexpr int FAST_EXACT_BLOCKS = 3;
 // bundle slots of a k_curvelets_exact warp, as many as three blocks of an SM have room for (a
-// seed past them has its bundle made again at every visit: with 4 slots a 3.2M-edge run's
+// seed past them has its bundle made again at every visit: with 4 slots a 3.65M-edge run's
 // two kernels took 14.64 ms, with these 14.48; 16 or 24 in two blocks: 14.82)
 constexpr int FAST_WIDE_SLOTS = 14;
 constexpr int FAST_TILE = 4;     // consecutive anchors a queue-pulling warp takes at a time

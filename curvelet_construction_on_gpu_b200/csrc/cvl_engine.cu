@@ -727,7 +727,7 @@ BinnedT<R> binned_arrays(const cvl_engine *e) {
 // A run's UNFIT_* flags (beside the queues, cleared with the counters).
 inline unsigned *unfit_of(const cvl_engine *e) { return (unsigned *)((unsigned long long *)e->work.p + 4) + 1; }
 // The one-pass search: pairs into csr_ids / pcls (pair_cap of them), rows into fast_rows.
-SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &B, const FastBinned &F, int n, int M,
+SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &B, const FastBinned &F, int n,
                        unsigned long long pair_cap) {
     SearchArgs a{};
     unsigned long long *work = (unsigned long long *)e->work.p;
@@ -737,8 +737,6 @@ SearchArgs search_args(const cvl_engine *e, const Model &md, const EdgeRecords &
     a.cs2 = F.cs2;
     a.at = F.at;
     a.bstart = (const unsigned *)e->bstart.p;
-    a.N = n;
-    a.M = M;
     a.row = (unsigned long long *)e->pair_off.p;
     a.pair_ctr = work + 1;
     a.pair_cap = pair_cap;
@@ -817,15 +815,17 @@ FinalArgs final_args(const cvl_engine *e, const Model &md, const FastModel &fm, 
 // n: the most anchors the launch serves (a run's, or its graph's)
 int launch_finalize(cvl_engine *e, const FinalArgs &f, int n) {
     const int blocks = short_grid(n, 256), small = short_grid(n, FINAL_WARPS * FINAL_ANCHORS);
-    if (n > (64 << 10))
+    if (n > (64 << 10)) {
         k_finalize_exact<<<blocks, 256, 0, e->stream>>>(f);
-    else if (f.md.gms <= 4)
+        return check_launch("k_finalize_exact");
+    }
+    if (f.md.gms <= 4)
         k_finalize_small<4><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
     else if (f.md.gms <= 8)
         k_finalize_small<8><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
     else
         k_finalize_small<16><<<small, FINAL_WARPS * 32, 0, e->stream>>>(f);
-    return check_launch("k_finalize_exact");
+    return check_launch("k_finalize_small");
 }
 
 // A run's error bits: CVL_EAGAIN where the two-pass search, or (wide_angles) the two-kernel
@@ -1074,7 +1074,7 @@ int run_pipeline_direct(cvl_engine *e, const R *d_edges, int n, int sz, const in
         if (pair_cap) {
             const int sms = e->prop.multiProcessorCount;
             // a persistent grid; short blocks where others' work is to be let in
-            SearchArgs sa = search_args(e, md, FB, F, n, M, pair_cap);
+            SearchArgs sa = search_args(e, md, FB, F, n, pair_cap);
             const long long items = std::min<long long>(n, (long long)T + n / search_item(n));  // at most
             int blocks = std::min(short_grid(items, SEARCH_WARPS), sms * SEARCH_BLOCKS);
             if (e->yield_fn) {
@@ -1584,8 +1584,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
             na.pair_cap = (unsigned long long)sh.num_pairs;
             const int gn = std::min(short_grid(N, (long long)nb_wpb * 4), sms * 8);
             if (fm.ok) {
-                SearchArgs sa = search_args(e, md, FB, F, N, cap.M, (unsigned long long)sh.num_pairs);
-                sa.dims = dd;
+                const SearchArgs sa = search_args(e, md, FB, F, N, (unsigned long long)sh.num_pairs);
                 CVL_TRY(launch_search(e, sa, std::min(short_grid(N, SEARCH_WARPS), sms * SEARCH_BLOCKS), sms));
             } else {
                 k_nb<double, NB_COUNT><<<gn, nb_wpb * 32, 0, s>>>(na);  // no candidate staging
@@ -1594,14 +1593,12 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 CVL_TRY(check_launch("k_deg_from_ncand"));
                 CVL_TRY((scan<unsigned, unsigned long long>(e, (const unsigned *)e->deg.p, N,
                                                             (unsigned long long *)e->pair_off.p)));
-                {
-                    k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
-                                                     (int *)e->chunk_start.p, dd);
-                    CVL_TRY(check_launch("k_chunk_starts"));
-                    k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
-                                                  (const int *)e->chunk_start.p, per_chunk, cap.K, cdp, err);
-                    CVL_TRY(check_launch("k_chunk_dims"));
-                }
+                k_chunk_starts<<<gb, 256, 0, s>>>(N, (const unsigned long long *)e->pair_off.p + 1, per_chunk, cap.K,
+                                                 (int *)e->chunk_start.p, dd);
+                CVL_TRY(check_launch("k_chunk_starts"));
+                k_chunk_dims<<<1, 32, 0, s>>>(dd, (const unsigned long long *)e->pair_off.p,
+                                              (const int *)e->chunk_start.p, per_chunk, cap.K, cdp, err);
+                CVL_TRY(check_launch("k_chunk_dims"));
                 na.csr_ids = (int *)e->csr_ids.p;
                 na.csr_d2 = nullptr;
                 na.pcls = (unsigned char *)e->pcls.p;
@@ -1610,8 +1607,6 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 na.uncertified = uncertified;
                 k_nb<double, NB_FILL><<<gn, nb_wpb * 32, nb_smem, s>>>(na);
                 CVL_TRY(check_launch("k_nb<FILL>"));
-            }
-            if (!fm.ok) {
                 k_cell_ranks<double><<<1, 128, 0, s>>>(md, (unsigned short *)e->crank.p);
                 CVL_TRY(check_launch("k_cell_ranks"));
             }
@@ -1639,7 +1634,7 @@ int run_pipeline_graph(cvl_engine *e, const double *d_edges, int n, int sz, cons
                 fa.count = (unsigned *)e->count.p;
                 fa.stats = stats;
                 fa.err = err;
-                    fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
+                fa.arena_chunk = 1;  // one arena record per curvelet, no chunk tails
                 fa.dims = dd;
                 fa.tile = b == 1 ? FAST_TILE : 1;
                 // bucket 1 pulls anchors from the queue; bucket 0's runs are too small for

@@ -122,7 +122,7 @@ struct RecordField {
 // The edges as k_search, k_curvelets_exact and k_finalize_exact read them: those gather an
 // edge's fields at random, so they lie in one record of two whole sectors (in an array per
 // field, as k_nb and k_bundles read them, the scatter wrote ten places an edge and a gather
-// touched six sectors: binning of a 3.65M-edge map 0.80 -> 0.47 ms, its finalize 1.95 -> 1.81).
+// touched six sectors: binning of a 3.65M-edge map 0.80 -> 0.47 ms, its finalize 1.95 -> 1.85).
 constexpr int EDGE_RECORD = 8;
 struct EdgeRecords {
     RecordField<double, EDGE_RECORD> x, y, th, sp, cp, sm, cm;

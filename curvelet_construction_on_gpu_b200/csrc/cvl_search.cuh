@@ -3,12 +3,12 @@
 //
 // k_search: a warp per item, 32 or fewer anchors of a hash bucket, a lane per anchor. The
 // anchors of one 8-pixel hash block share their candidates: the edges of the 3 x 3 blocks
-// around it that lie within w pixels of it. The warp loads those once, keeps them in shared memory, and every lane tests
-// them with the reference's predicate (preprocess.hpp:129-167), reading each at the same time
-// as the others (a broadcast), and appends its neighbours to its column of a table. The rows
-// of the anchors are allocated together and back to back, so the warp writes them as one
-// coalesced run, a lane per pair, each with its rank by (distance, scan order) in its
-// anchor's column and its classes.
+// around it that lie within w pixels of it. The warp loads those once and keeps them in
+// shared memory. Every lane tests them with the reference's predicate
+// (preprocess.hpp:129-167), reading each at the same time as the others (a broadcast), and
+// appends its neighbours to its column of a table. The rows of the anchors are allocated
+// together and back to back, so the warp writes them as one coalesced run, a lane per pair,
+// each with its rank by (distance, scan order) in its anchor's column and its classes.
 //
 // A run with a non-finite edge fails (ERR_NONFINITE, final since k_bin_keys), and nothing from
 // here on may read what it left: k_bin_keys puts such an edge into bucket 0, whatever its
@@ -60,7 +60,6 @@ struct SearchArgs {
     const double2 *cs2;               // [N]
     const int4 *at;                   // [N] pixel cell, input index, map
     const unsigned *bstart;
-    int N, M;
     unsigned long long *row;          // [N] pack_row
     unsigned long long *pair_ctr;     // pairs allocated
     unsigned long long pair_cap;
@@ -77,7 +76,6 @@ struct SearchArgs {
     unsigned item_size;               // a power of two, at most 32
     unsigned *queue;                  // the next item (0 at start)
     unsigned pulls;                   // items a warp takes at most
-    const RunDims *dims;
 };
 
 struct SearchSmem {
