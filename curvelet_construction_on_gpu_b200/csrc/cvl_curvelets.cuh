@@ -336,7 +336,7 @@ __device__ __forceinline__ bool fine_column(const FastArgs &a, double2 cs, int i
                                             float &wmax) {
     const double2 c2 = a.F.cs2[i];
     const FastEdge ae = a.F.e[i];
-    const float ang = (float)(fabs(a.B.th[i]) + fabs(a.B.th[nn])) + a.fm.fa;
+    const float ang = fabsf((float)a.B.th[i]) + fabsf((float)a.B.th[nn]) + a.fm.fa;
     const float ethr = a.fm.fe * ang, dthr = a.fm.fd * ang;
     const double sT = fma(c2.y, cs.x, c2.x * cs.y), cT = fma(c2.x, cs.x, -(c2.y * cs.y));
     const double X = ae.x - a.F.e[nn].x, Y = ae.y - a.F.e[nn].y;

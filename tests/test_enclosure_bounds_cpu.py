@@ -186,7 +186,7 @@ def test_fine_columns(shim, over, turns):
     t2 = -2.0 * (sT * DX - cT * DY)
     N = t2 + 2.0 * d
     e1 = _r(d * (t2 + d) + (DX * DX + (DY * DY - m.dx2)))
-    ang = _r(_r(np.abs(T2) + np.abs(T0)) + f.fa)
+    ang = _r(_r(_r(np.abs(T2)) + _r(np.abs(T0))) + f.fa)
     ethr, dthr = _r(f.fe * ang), _r(f.fd * ang)
     re = _rcp(e1, rng)
     got, ok = [-_r(_r(N + 2.0 * m.dx) * re), _r(_r(2.0 * m.dx - N) * re)], e1 >= ethr
