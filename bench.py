@@ -51,12 +51,14 @@ sys.path.insert(0, ROOT)
 METRIC = "edges/s"
 # per computed (non-close) pair: 63 cells x 20 flops, divisions counted as 1
 FLOPS_PER_PAIR_CELL = 20
-# k_curvelets on the 242k-edge 1920x1080 map, one ncu capture (--set full,
-# profiles/k_curvelets_k_search_hd.md): warp instructions and DRAM bytes per edge. The
-# bundles stay on the chip, so the traffic is the pairs' ids and classes, the edges and the
-# records.
-CURVELETS_WARP_INSTR_PER_EDGE = 392_889_469 / 242_059
-CURVELETS_DRAM_BYTES_PER_EDGE = (30.807296e6 + 0.557312e6) / 242_059
+# k_curvelets and k_curvelets_exact, one ncu capture of each workload itself (1 pass;
+# profiles/launches_mixed64.md): warp instructions and DRAM bytes per edge. The bundles stay
+# on the chip, so the traffic is the pairs' ids and classes, the edges and the records.
+CURVELETS_NCU = {
+    "mixed64": ((80_496_266_982 + 1_935_806_308) / 33_710_534,
+                (11_575_324_672 + 3_604_541_440 + 542_437_120 + 37_102_848) / 33_710_534),
+    "plain_hd": ((386_806_586 + 3_275_757) / 242_059, (31_324_160 + 705_024 + 1_160_704) / 242_059),
+}
 # FP32 lanes and warp-instruction issue slots of one SM per cycle
 SM_FP32_LANES = 128
 SM_ISSUE_SLOTS = 4
@@ -738,11 +740,12 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
         return
     curv_ms = float(np.mean([k.get("curvelets", 0.0) for k in kern]))
     flops = FLOPS_PER_PAIR_CELL * 63 * nonclose
-    achieved = flops / (curv_ms / 1e3) / 1e12 if curv_ms > 0 else 0.0
+    achieved = flops / (curv_ms / 1e3) / 1e12 if curv_ms > 0 else None  # (a graph run has no stages)
     clocks = clk.summary()
     sms, hz = _sm_count(), 1e6 * float(clocks.get("sm_mhz") or 1965.0)
     fp32_peak = sms * SM_FP32_LANES * 2 * hz / 1e12
     issue_peak = sms * SM_ISSUE_SLOTS * hz
+    instr, dram = CURVELETS_NCU.get(args.workload, (None, None))
     stage_ms = {k: float(np.mean([d.get(k, 0.0) for d in kern])) for k in kern[0]} if kern else {}
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
@@ -754,19 +757,19 @@ def run_ours(args, maps, cfg, world, rank, local, pg):
         "curvelets_per_s": n_curv * world * args.steps / (sum_ms / 1e3),
         "stage_ms": stage_ms,
         "roofline": {"bound": "issue", "kernel": "k_curvelets (with k_curvelets_exact)", "achieved": achieved,
-                     "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
+                     "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak if achieved else None,
                      "peak_source": f"{sms} SMs x {SM_FP32_LANES} FP32 lanes x 2 x the sampled clock",
                      "work": f"{FLOPS_PER_PAIR_CELL} flops x 63 cells x {nonclose} non-close pairs, "
                              f"{max(1, int(curv_launches))} launch(es) per step; growth not counted",
-                     "traffic": CURVELETS_DRAM_BYTES_PER_EDGE * n_edges / max(1, int(curv_launches)),
+                     "traffic": dram * n_edges / max(1, int(curv_launches)) if dram else None,
                      "traffic_unit": "bytes per launch",
-                     "traffic_source": "ncu dram bytes of k_curvelets on the 242k-edge map, per edge",
+                     "traffic_source": "ncu dram bytes of both kernels on this workload, per edge",
                      "issue": {
-                         "warp_instr_per_edge": CURVELETS_WARP_INSTR_PER_EDGE,
-                         "frac": (CURVELETS_WARP_INSTR_PER_EDGE * n_edges / (curv_ms / 1e3) / issue_peak)
-                         if curv_ms > 0 else None,
-                         "note": "warp instructions per edge from ncu on the 242k-edge map, over this run's "
-                                 "curvelets stage, against 4 a cycle and SM; denser maps take more per edge"},
+                         "warp_instr_per_edge": instr,
+                         "frac": (instr * n_edges / (curv_ms / 1e3) / issue_peak)
+                         if instr and curv_ms > 0 else None,
+                         "note": "warp instructions per edge of both kernels from ncu on this workload, over this "
+                                 "run's curvelets stage, against 4 a cycle and SM"},
                      "fp64_peak_tflops": fp64_peak},
         "path_hbm": path_hbm(n_edges, n_curv, sum_ms / args.steps, _measured_peaks(),
                              edge_bytes=8 * int(maps[0].shape[1])),
