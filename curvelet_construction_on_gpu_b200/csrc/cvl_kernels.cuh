@@ -332,7 +332,8 @@ template <typename T>
 __global__ void k_bin_scatter(const T *__restrict__ edges, int sz, int N, const int *__restrict__ map_off,
                               int M, ModelT<T> md, const unsigned *__restrict__ ehash,
                               const unsigned *__restrict__ bstart, unsigned *__restrict__ bcount, BinnedT<T> B,
-                              double2 *__restrict__ rec, int *__restrict__ pos_of, FastEdge *__restrict__ fe, double2 *__restrict__ cs2,
+                              double2 *__restrict__ rec, int *__restrict__ pos_of, FastEdge *__restrict__ fe,
+                              double2 *__restrict__ cs2,
                               int4 *__restrict__ at, unsigned *__restrict__ items, unsigned *__restrict__ item_cnt,
                               unsigned item_size, const unsigned *__restrict__ unfit,
                               const RunDims *__restrict__ dims) {
