@@ -70,7 +70,8 @@ def _map(kind):
 
 @pytest.mark.parametrize("turns", [0, 16, 159, 166000])  # orientations within 2 pi, of about 100, 1000 and 1e6 rad
 @pytest.mark.parametrize("over", [dict(), dict(max_k=0.002), dict(max_k=2.0 ** -10), dict(max_k=900.0), dict(dx=0.36),
-                                  dict(dx=0.36, max_k=2.0 ** -10), dict(nrad=60.0)],
+                                  dict(dx=0.36, max_k=2.0 ** -10), dict(nrad=60.0), dict(nrad=1e3), dict(nrad=1e200),
+                                  dict(nrad=1e-3)],
                          ids=lambda o: "-".join(f"{k}{v:g}" for k, v in o.items()) or "default")
 @pytest.mark.parametrize("kind", ["small", "lines", "scatter"])
 def test_angles_and_curvatures(engines, kind, over, turns):
